@@ -204,6 +204,26 @@ int paro_plan_fill(const uint8_t* mask, int slices, int nbq, int nbk,
 int paro_plan_schedule(const int32_t* pair_ptr, const int32_t* pair_ent, int slices, int nbq, int nbk,
                        uint32_t* sched, int32_t* sched_cnt, paro_stream_t stream);
 
+/* The lists above in two calls, from a bit-packed copy of the mask, with the choice of the pairs on the device.
+ * overlap = 0: pair p is q-blocks 2p, 2p+1; the results equal paro_plan_count / _fill / _schedule.
+ * overlap = 1 (nbq < 65535): per slice, the first q-block not yet paired takes the free q-block it shares most k-blocks
+ * with (ties: the lowest id); a slice for which that does not need fewer tiles than adjacency keeps the adjacent pairs.
+ * pair_q [2 * slices*ceil(nbq/2)] receives the q-blocks of each pair (-1: none), and all lists are those of the mask
+ * with its rows in that order.
+ * paro_plan_offsets writes row_ptr, pair_ptr and totals[4] (device): kept blocks, merged entries, 1 if any slice was paired
+ * by overlap, 1 if a bounded device-side wait expired (the lists are then invalid).  The caller reads the totals back, allocates cols [kept] and pair_ent, sched [merged entries] (at
+ * least one element each), and paro_plan_lists fills them, sched_cnt, and (nullable, overlap only) sched_cnt_kernel: the
+ * step counts with (q-block id + 1) << 16, as paro_sparse_attn reads them.
+ * scratch: paro_plan_scratch_bytes(), 16-byte aligned, kept unchanged from the first call to the second. */
+size_t paro_plan_scratch_bytes(int slices, int nbq, int nbk, int overlap);
+int paro_plan_offsets(const uint8_t* mask, int slices, int nbq, int nbk, int overlap,
+                      int32_t* row_ptr, int32_t* pair_ptr, int32_t* pair_q, int32_t* totals,
+                      void* scratch, size_t scratch_bytes, paro_stream_t stream);
+int paro_plan_lists(int slices, int nbq, int nbk, int overlap,
+                    const int32_t* row_ptr, const int32_t* pair_ptr, const int32_t* pair_q,
+                    int32_t* cols, int32_t* pair_ent, uint32_t* sched, int32_t* sched_cnt, int32_t* sched_cnt_kernel,
+                    const void* scratch, size_t scratch_bytes, paro_stream_t stream);
+
 /* Checks walk lists that did not come from paro_plan_schedule in this process (read from a file, built
  * by other code) before paro_sparse_attn follows them: pair_ptr starts at 0, is monotone and stays within
  * sched_len entries; each q-block's step count fits its pair's slots (and is 0 for a q-block past the end);

@@ -103,11 +103,11 @@ def validate_plan(plan: "CompactPlan") -> None:
 
 
 def pair_rows_by_overlap(m: torch.Tensor) -> torch.Tensor:
-    """m: uint8/bool [slices, nbq, nbk] on the GPU.  Returns int64 [slices, nbq]: an order of the q-blocks
+    """m: uint8/bool [slices, nbq, nbk].  Returns int64 [slices, nbq]: an order of the q-blocks
     in which rows 2p and 2p+1 are good partners -- the kernel walks the UNION of a pair's two lists, a
     k-block both keep costs one tile instead of two.  Greedy: the first q-block not yet paired takes the
-    free q-block it shares most k-blocks with (ties: the lowest index).  Deterministic; nbq/2 rounds of a
-    few small kernels, vectorised over the slices."""
+    free q-block it shares most k-blocks with (ties: the lowest index).  This is the rule in plain torch;
+    compact_plan follows it on the device (csrc/plan_compact.cu)."""
     S, nbq, _ = m.shape
     mf = m.to(torch.float32)
     ov = torch.bmm(mf, mf.transpose(1, 2))                    # shared k-blocks of every two q-blocks
@@ -132,36 +132,11 @@ def compact_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: s
     validate: run validate_plan on the result (default: only when the environment variable
     PARO_DEBUG_PLANS is set to a non-empty value other than 0).
     pairing: "adjacent" -- work item p is q-blocks 2p and 2p+1; "overlap" -- q-blocks are paired by the
-    k-blocks they share (pair_rows_by_overlap), kept for the slices (heads) where that needs fewer tiles than adjacency."""
+    k-blocks they share (pair_rows_by_overlap), kept for the slices (heads) where that needs fewer tiles than adjacency.
+    The choice is made slice by slice, so that a head's plan -- and with it the order in which its rows
+    accumulate -- does not depend on which other heads are compacted with it."""
     if pairing not in ("adjacent", "overlap"):
         raise ValueError(f"unknown pairing {pairing!r}")
-    if pairing == "overlap":
-        _lib.require_cuda(mask)
-        nbq0, nbk0 = int(mask.shape[-2]), int(mask.shape[-1])
-        m0 = mask.reshape(-1, nbq0, nbk0)
-        m0 = (m0 if m0.dtype in (torch.uint8, torch.bool) else (m0 != 0)).contiguous().view(torch.uint8)
-        base = compact_plan(m0, validate=validate)
-        if nbq0 < 4 or nbq0 >= 0xFFFF:
-            return base
-        npairs0 = (nbq0 + 1) // 2
-        order = pair_rows_by_overlap(m0)
-        plan = compact_plan(torch.gather(m0, 1, order.unsqueeze(-1).expand(-1, -1, nbk0)), validate=validate)
-        # The choice is made slice by slice (head by head), so that a head's plan -- and with it the order
-        # in which its rows accumulate -- does not depend on which other heads are compacted with it.
-        ends = torch.arange(0, m0.shape[0] + 1, device=m0.device) * npairs0
-        per_slice = lambda pl: (pl.pair_ptr[ends[1:]] - pl.pair_ptr[ends[:-1]])
-        better = per_slice(plan) < per_slice(base)
-        if not bool(better.any()):
-            return base
-        if not bool(better.all()):
-            ident = torch.arange(nbq0, device=m0.device).expand_as(order)
-            order = torch.where(better.unsqueeze(1), order, ident)
-            plan = compact_plan(torch.gather(m0, 1, order.unsqueeze(-1).expand(-1, -1, nbk0)), validate=validate)
-        pq = torch.full((m0.shape[0], 2 * npairs0), -1, dtype=torch.int32, device=m0.device)
-        pq[:, :nbq0] = order.to(torch.int32)
-        plan.pair_q = pq.view(-1, 2).contiguous()
-        plan.sched_cnt_kernel = (plan.sched_cnt | ((plan.pair_q + 1) << 16)).contiguous()
-        return plan
     _lib.require_cuda(mask)
     if validate is None:
         import os
@@ -171,27 +146,37 @@ def compact_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: s
     nbq, nbk = int(mask.shape[-2]), int(mask.shape[-1])
     m = mask.reshape(-1, nbq, nbk)
     m = (m if m.dtype in (torch.uint8, torch.bool) else (m != 0)).contiguous().view(torch.uint8)
-    slices = m.shape[0]
+    slices, dev = m.shape[0], m.device
     npairs = (nbq + 1) // 2
+    overlap = int(pairing == "overlap" and 4 <= nbq < 0xFFFF)
     L = _lib.lib()
-    with torch.cuda.device(m.device):
-        row_ptr = torch.empty(slices * nbq + 1, dtype=torch.int32, device=m.device)
-        pair_ptr = torch.empty(slices * npairs + 1, dtype=torch.int32, device=m.device)
+    with torch.cuda.device(dev):
+        row_ptr = torch.empty(slices * nbq + 1, dtype=torch.int32, device=dev)
+        pair_ptr = torch.empty(slices * npairs + 1, dtype=torch.int32, device=dev)
+        pair_q = torch.empty(slices * npairs, 2, dtype=torch.int32, device=dev) if overlap else None
+        totals = torch.empty(4, dtype=torch.int32, device=dev)
+        need = L.paro_plan_scratch_bytes(slices, nbq, nbk, overlap)
+        scratch = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
         s = _lib.stream_ptr()
-        _lib.check(L.paro_plan_count(m.data_ptr(), slices, nbq, nbk, row_ptr.data_ptr(), pair_ptr.data_ptr(), s))
-        kept, tiles = int(row_ptr[-1].item()), int(pair_ptr[-1].item())
-        cols = torch.empty(max(kept, 1), dtype=torch.int32, device=m.device)
-        pair_ent = torch.empty(max(tiles, 1), dtype=torch.int32, device=m.device)
-        _lib.check(L.paro_plan_fill(m.data_ptr(), slices, nbq, nbk, row_ptr.data_ptr(), cols.data_ptr(), kept,
-                                    pair_ptr.data_ptr(), pair_ent.data_ptr(), tiles, s))
-        sched = torch.empty(max(tiles, 1), dtype=torch.int32, device=m.device)
-        sched_cnt = torch.empty(slices * npairs, 2, dtype=torch.int32, device=m.device)
-        _lib.check(L.paro_plan_schedule(pair_ptr.data_ptr(), pair_ent.data_ptr(), slices, nbq, nbk, sched.data_ptr(),
-                                        sched_cnt.data_ptr(), s))
+        _lib.check(L.paro_plan_offsets(m.data_ptr(), slices, nbq, nbk, overlap, row_ptr.data_ptr(), pair_ptr.data_ptr(),
+                                       _lib.ptr(pair_q), totals.data_ptr(), scratch.data_ptr(), scratch.numel(), s))
+        kept, tiles, paired, expired = totals.tolist()      # the lists' lengths: the one synchronisation of the call
+        if expired:
+            raise _lib.ParoError(_lib.PARO_ETIMEOUT, "a wait of the q-block pairing expired")
+        cols = torch.empty(max(kept, 1), dtype=torch.int32, device=dev)
+        pair_ent = torch.empty(max(tiles, 1), dtype=torch.int32, device=dev)
+        sched = torch.empty(max(tiles, 1), dtype=torch.int32, device=dev)
+        sched_cnt = torch.empty(slices * npairs, 2, dtype=torch.int32, device=dev)
+        cnt_kernel = torch.empty_like(sched_cnt) if paired else None
+        _lib.check(L.paro_plan_lists(slices, nbq, nbk, overlap, row_ptr.data_ptr(), pair_ptr.data_ptr(), _lib.ptr(pair_q),
+                                     cols.data_ptr(), pair_ent.data_ptr(), sched.data_ptr(), sched_cnt.data_ptr(),
+                                     _lib.ptr(cnt_kernel), scratch.data_ptr(), scratch.numel(), s))
     plan = CompactPlan(slices, nbq, nbk, row_ptr, cols[:kept], pair_ptr, pair_ent[:tiles], kept, tiles,
                        sched[:tiles], sched_cnt)
     if validate:
         validate_plan(plan)
+    if paired:
+        plan.pair_q, plan.sched_cnt_kernel = pair_q, cnt_kernel
     return plan
 
 
