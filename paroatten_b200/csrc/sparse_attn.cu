@@ -6,10 +6,17 @@
 // Work item (one CTA): a PAIR of adjacent 64-row q-blocks of one (batch, head), i.e. a 128-row
 // tile -- the native tcgen05.mma M.  The pair walks a schedule built with the plan: first the
 // k-blocks BOTH q-blocks keep (one K/V tile and one full-height MMA group serve all 128 rows), then
-// the remaining blocks of the upper half side by side with the remaining blocks of the lower half.
-// In a side-by-side step each MMA is issued with the query tile of all 128 rows but with a lane mask
-// that keeps it from writing the other half's accumulator rows, so both halves always have work (all
-// four SM sub-partitions run exponentials) and nothing is computed for blocks that are not kept.
+// the remaining blocks of the upper half side by side with the remaining blocks of the lower half, so both
+// halves always have work (all four SM sub-partitions run exponentials) and nothing is computed for blocks
+// that are not kept.
+// A side-by-side step is ONE group of tcgen05.mma.ws with M = 64: its two tiles lie back to back in shared
+// memory as one B operand of 2 x 64 keys (Q.K^T) or 2 x D channels (P.V), lanes 0-63 multiply by the first
+// and lanes 64-127 by the second.  Issued as two M = 128 instructions with half of the lanes masked, such a
+// step costs the tensor pipe twice the work that it needs: 356 + 512 clocks against 178 + 304 (one CTA per
+// SM, D = 128).  Masked instructions remain for the steps in which only one half still has blocks.
+// Measured, whole call, masked -> ws: 40 heads x 75600 tokens at density 0.2 23.5 -> 21.7 ms, 5 of those heads
+// 3.02 -> 2.81 ms, 2 x 12 x 32760 at 0.3 4.46 -> 4.26 ms, D = 64 2 x 48 x 17776 4.61 -> 4.54 ms; results are the
+// same bits.
 //
 //   warps 0-7   softmax + epilogue.  Row r of the tile belongs to two threads, one in each WARP SET:
 //               warp w (< 4, set 0) handles the even steps of its half, warp w+4 (set 1) the odd
@@ -19,7 +26,7 @@
 //               exact walk, the running row maximum passes from step to step through shared memory).
 //               P is written to TMEM as bf16; the epilogue stores O/l * v_scale + vm at the row's
 //               un-permuted position.  These warps take the registers the others give up.
-//   warp 8      one lane: TMA producer for the K ring (int8 tiles)
+//   warp 8      one lane: TMA producer for the K ring (int8 tiles; a slot holds one step's tiles)
 //   warp 9      one lane: TMA producer for the V^T ring (bf16 tiles)
 //   warp 10     owns TMEM; issues S = Q.K^T (kind::i8, A = Q from TMEM, int32 accumulators)
 //   warp 11     issues O += P.V (kind::f16 on bf16, A = P from TMEM, fp32 accumulators in TMEM)
@@ -27,9 +34,9 @@
 //               and addresses are formed in uniform registers; the tcgen05 instructions themselves
 //               are guarded by the elected lane's predicate.
 //
-// Hand-offs.  An issuer commits ONCE per tile, to the barrier of (half, step mod 4): "scores ready"
-// for Q.K^T, "P.V done" for P.V.  The softmax warps wait on it, and so does the ring's producer when it
-// wants that tile's stage back.  The softmax warps release S the moment the scores are in registers
+// Hand-offs.  An issuer commits once per step and half served, to the barrier of (half, step mod 4): "scores
+// ready" for Q.K^T, "P.V done" for P.V.  The softmax warps wait on it, and so does the ring's producer when it
+// wants that step's slot back.  The softmax warps release S the moment the scores are in registers
 // and write P after all of a step's arithmetic.
 //
 // TMEM (256 columns per CTA): S [0,64) int32 scores, P [64,96) bf16 probabilities, Q [96,128) the
@@ -65,19 +72,18 @@ constexpr float REF_OFFSET = 20.f;             // fixed reference: the first blo
 constexpr float ROWSUM_LIMIT = 1.2676506e30f;  // 2^100: a step's row sum beyond it gives the pair back
 
 template <int D> struct AttnCfg {
-  // Ring depths.  TMEM allows two CTAs per SM; the loads run far ahead of their use at any depth from 2
-  // to 6 (same time within noise), so the rings are kept short and the shared memory left over is
-  // requested back as L1 (carve-out attribute at launch) for the schedule entries and k-block scales.
-  static constexpr int K_STAGES = (D == 128) ? 3 : 4;
-  static constexpr int V_STAGES = (D == 128) ? 3 : 4;
-  // The commit barriers are indexed by step modulo STEP_BARS, and a ring stage is handed back to its
-  // producer through the commit barrier of the tile that used it: a producer can only tell that
+  // A ring slot holds the K (or V) tiles of one STEP: one tile, or the two halves' tiles back to back, so
+  // that they form one B operand.  Two slots at D = 128 are what two CTAs per SM leave room for.
+  static constexpr int K_SLOTS = (D == 128) ? 2 : 4;
+  static constexpr int V_SLOTS = (D == 128) ? 2 : 4;
+  // The commit barriers are indexed by step modulo STEP_BARS, and a ring slot is handed back to its
+  // producer through the commit barrier of the step that used it: a producer can only tell that
   // barrier's phases apart while the ring is no deeper than STEP_BARS.
   static constexpr int STEP_BARS = 4;
-  static_assert(K_STAGES <= STEP_BARS && V_STAGES <= STEP_BARS, "ring deeper than the commit barriers can tell apart");
-  static constexpr int K_BYTES = 64 * D;
+  static_assert(K_SLOTS <= STEP_BARS && V_SLOTS <= STEP_BARS, "ring deeper than the commit barriers can tell apart");
+  static constexpr int K_BYTES = 64 * D;    // one tile
   static constexpr int V_BYTES = D * 128;   // D rows of 64 bf16
-  static constexpr int TILE_BYTES = K_STAGES * K_BYTES + V_STAGES * V_BYTES;
+  static constexpr int TILE_BYTES = 2 * (K_SLOTS * K_BYTES + V_SLOTS * V_BYTES);
   static constexpr int AUX_BYTES = 4096;    // barriers, TMEM pointer, abort flag, v_scale, vm, row exchange
   static constexpr int SMEM_BYTES = TILE_BYTES + AUX_BYTES + 1024 /* alignment slack */;
 };
@@ -100,24 +106,24 @@ __global__ void __launch_bounds__(ATT_THREADS, 2)
 sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                          const AttnParams p) {
   using Cfg = AttnCfg<D>;
-  constexpr int KST = Cfg::K_STAGES, VST = Cfg::V_STAGES;
+  constexpr int KST = Cfg::K_SLOTS, VST = Cfg::V_SLOTS;
   // second launch of a call: only the work items the fixed-reference walk gave back
   if (p.from_list && (int)blockIdx.x >= *reinterpret_cast<volatile int32_t*>(p.redo)) return;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
-  uint8_t* sV = sK + KST * Cfg::K_BYTES;
+  uint8_t* sV = sK + KST * 2 * Cfg::K_BYTES;
   uint8_t* aux = smem + Cfg::TILE_BYTES;
   // mbarriers.  [h][par]: one per half of the pair and per parity of the step index, so that each
   // barrier is arrived on and waited for by the same parties in every phase.
   uint64_t* bar_q = reinterpret_cast<uint64_t*>(aux);   // [1]     Q tile stored in TMEM
-  uint64_t* bar_kfull = bar_q + 1;                      // [KST]   K tile landed
-  uint64_t* bar_vfull = bar_kfull + KST;                // [VST]   V tile landed
+  uint64_t* bar_kfull = bar_q + 1;                      // [KST]   K tiles of a step landed
+  uint64_t* bar_vfull = bar_kfull + KST;                // [VST]   V tiles of a step landed
   uint64_t* bar_sready = bar_vfull + VST;               // [2][4]  scores of (half, step mod 4) in TMEM: the Q.K^T
-                                                        //         finished, so its K stage is free as well
+                                                        //         finished, so its K slot is free as well
   uint64_t* bar_pvdone = bar_sready + 8;                // [2][4]  P.V of (half, step mod 4) finished: P may be
-                                                        //         rewritten, the V stage is free
+                                                        //         rewritten, the V slot is free
   uint64_t* bar_sfree = bar_pvdone + 8;                 // [2][2]  scores of (half, step parity) copied to registers
   uint64_t* bar_pready = bar_sfree + 4;                 // [2][2]  P of (half, step parity) written
   uint64_t* bar_drain = bar_pready + 4;                 // [2]     issuers' MMAs retired (abort path only)
@@ -153,22 +159,11 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const uint32_t cnt_a = (uint32_t)p.sched_cnt[2 * prow], cnt_b = (uint32_t)p.sched_cnt[2 * prow + 1];
   const int n_a = (int)(cnt_a & 0xFFFFu), n_b = (int)(cnt_b & 0xFFFFu);
   const int n_steps = max(n_a, n_b);
-  // A step has one MMA group of each kind per tile: group 0 serves the upper half, or both halves
-  // when the tile is shared (kbA == kbB); group 1 serves the lower half.  Sharing halves the tensor
-  // work of such a step but makes the two halves wait for each other in it.  (With single-lane
-  // issuers that wait cost more than it saved at D = 64; with the issuers running warp-wide sharing
-  // wins there too: 3.85 vs 3.96 ms on the CogVideoX shape.)
-  constexpr bool SHARE_TILES = true;
-  // Issuing a side-by-side step's two tiles in one burst (see `both` below) is slower at D = 128, where the
-  // tensor pipe is what the issuers wait for (21.5 vs 21.1 ms on the Wan-14B shape), and a little faster at
-  // D = 64.
-  constexpr bool FUSE_STEPS = (D == 64);
-#define PARO_STEP_GROUPS(e)                                                        \
-  const int ka_ = (int)((e) & 0xFFFFu), kb_ = (int)((e) >> 16);                    \
-  const bool shared_ = SHARE_TILES && ka_ == kb_;                                  \
-  const bool act_[2] = {ka_ != 0xFFFF, !shared_ && kb_ != 0xFFFF};                 \
-  [[maybe_unused]] const int kblk_[2] = {ka_, kb_};                                \
-  [[maybe_unused]] const int which_[2] = {shared_ ? 2 : 0, 1};
+  // A step is one group of MMAs of each kind: FORM_UPPER / FORM_LOWER when only one half still has blocks (128
+  // rows, the other half's accumulator rows masked), FORM_SHARED when both keep the same block (one tile, 128
+  // rows) and FORM_DUAL when each half has its own (two tiles, tcgen05.mma.ws: two 64-row products in one
+  // instruction).
+  enum { FORM_UPPER = 0, FORM_LOWER = 1, FORM_SHARED = 2, FORM_DUAL = 3 };
 
   if (threadIdx.x == 0) {
     mbar_init(bar_q, 4);
@@ -201,84 +196,62 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
-    if (warp == 8 && lane == 0) {
-      // ---------------------------------------------------------------- TMA producer: K ring
-      tma_prefetch_desc(&tm_k);
-      bool ok = true;
-      int t = 0;   // tiles so far = position in the ring
-      // a stage is free again when the Q.K^T of the tile that held it has finished: the scores-ready
-      // commit of that tile (no commit of its own for the ring)
-      const uint32_t a_done = smem_u32(bar_sready);
-      ReleaseFifo<KST> held;
-      // schedule entries are fetched two steps ahead of their use
-      uint32_t e_cur = n_steps > 0 ? sched[0] : 0u, e_nxt = n_steps > 1 ? sched[1] : 0u;
-      for (int i = 0; i < n_steps && ok; ++i) {
-        PARO_STEP_GROUPS(e_cur)
-        e_cur = e_nxt;
-        if (i + 2 < n_steps) e_nxt = ld_pinned_u32(sched + i + 2);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          if (!act_[j]) continue;
-          const int st = t % KST;
-          TR(0, i, 2 * j);
-          if (t >= KST && !mbar_wait_bounded_at(held.oldest() & 0x7fffffffu, held.oldest() >> 31, abort_flag, WAIT_LIMIT)) {
-            report_timeout(p, abort_flag, 1, i);
-            ok = false;
+    if (warp <= 9 && lane == 0) {
+      // ---------------------------------------------------------------- TMA producers: K ring (warp 8), V ring (warp 9)
+      auto produce = [&](auto ktag, const CUtensorMap* tm, uint8_t* ring, uint64_t* bar_full, uint64_t* bar_done) {
+        constexpr bool IS_K = decltype(ktag)::value;
+        constexpr int ST = IS_K ? KST : VST, BYTES = IS_K ? Cfg::K_BYTES : Cfg::V_BYTES;
+        [[maybe_unused]] constexpr int trole = IS_K ? 0 : 1;
+        tma_prefetch_desc(tm);
+        int t = 0;   // steps with tiles so far = position in the ring
+        // a slot is free again when the MMAs of the step that held it have finished: that step's scores-ready
+        // (K) or P.V-done (V) commit (no commit of its own for the ring)
+        const uint32_t a_done = smem_u32(bar_done);
+        ReleaseFifo<ST> held;
+        auto load = [&](uint8_t* dst, uint32_t kb, uint64_t* bar) {
+          if (IS_K) tma_load_3d(dst, tm, 0, (int)kb * 64, bh, bar);
+          else tma_load_3d(dst, tm, (int)kb * 64, 0, bh, bar);
+        };
+        // schedule entries are fetched two steps ahead of their use
+        uint32_t e_cur = n_steps > 0 ? sched[0] : 0u, e_nxt = n_steps > 1 ? sched[1] : 0u;
+        for (int i = 0; i < n_steps; ++i) {
+          const uint32_t ka = e_cur & 0xFFFFu, kb = e_cur >> 16;
+          e_cur = e_nxt;
+          if (i + 2 < n_steps) e_nxt = ld_pinned_u32(sched + i + 2);
+          const uint32_t first = ka != 0xFFFFu ? ka : kb;   // the tile at the front of the slot
+          if (first == 0xFFFFu) continue;
+          const bool two = ka != 0xFFFFu && kb != 0xFFFFu && ka != kb;
+          const int st = t % ST;
+          TR(trole, i, 0);
+          if (t >= ST && !mbar_wait_bounded_at(held.oldest() & 0x7fffffffu, held.oldest() >> 31, abort_flag, WAIT_LIMIT)) {
+            report_timeout(p, abort_flag, IS_K ? 1 : 9, i);
             break;
           }
-          held.push(commit_token(a_done, j, i));   // (a tile shared by both halves commits to both: j = 0 is watched)
+          held.push(commit_token(a_done, ka != 0xFFFFu ? 0 : 1, i));   // (a step of both halves commits to both)
           ++t;
-          TR(0, i, 2 * j + 1);
-          mbar_arrive_expect_tx(bar_kfull + st, Cfg::K_BYTES);
-          tma_load_3d(sK + st * Cfg::K_BYTES, &tm_k, 0, kblk_[j] * 64, bh, bar_kfull + st);
+          TR(trole, i, 1);
+          mbar_arrive_expect_tx(bar_full + st, two ? 2 * BYTES : BYTES);
+          load(ring + st * 2 * BYTES, first, bar_full + st);
+          if (two) load(ring + st * 2 * BYTES + BYTES, kb, bar_full + st);
         }
-      }
-      if (*abort_flag)   // leaving early: the copies this thread started must have landed first
-        for (int u = max(0, t - KST); u < t; ++u) mbar_wait_plain_bounded(bar_kfull + u % KST, (u / KST) & 1, WAIT_LIMIT);
-    } else if (warp == 9 && lane == 0) {
-      // ---------------------------------------------------------------- TMA producer: V ring
-      tma_prefetch_desc(&tm_v);
-      bool ok = true;
-      int t = 0;
-      const uint32_t a_done = smem_u32(bar_pvdone);   // the P.V commit of the tile that held the stage
-      ReleaseFifo<VST> held;
-      uint32_t e_cur = n_steps > 0 ? sched[0] : 0u, e_nxt = n_steps > 1 ? sched[1] : 0u;
-      for (int i = 0; i < n_steps && ok; ++i) {
-        PARO_STEP_GROUPS(e_cur)
-        e_cur = e_nxt;
-        if (i + 2 < n_steps) e_nxt = ld_pinned_u32(sched + i + 2);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          if (!act_[j]) continue;
-          const int st = t % VST;
-          TR(1, i, 2 * j);
-          if (t >= VST && !mbar_wait_bounded_at(held.oldest() & 0x7fffffffu, held.oldest() >> 31, abort_flag, WAIT_LIMIT)) {
-            report_timeout(p, abort_flag, 9, i);
-            ok = false;
-            break;
-          }
-          held.push(commit_token(a_done, j, i));
-          ++t;
-          TR(1, i, 2 * j + 1);
-          mbar_arrive_expect_tx(bar_vfull + st, Cfg::V_BYTES);
-          tma_load_3d(sV + st * Cfg::V_BYTES, &tm_v, kblk_[j] * 64, 0, bh, bar_vfull + st);
-        }
-      }
-      if (*abort_flag)
-        for (int u = max(0, t - VST); u < t; ++u) mbar_wait_plain_bounded(bar_vfull + u % VST, (u / VST) & 1, WAIT_LIMIT);
+        if (*abort_flag)   // leaving early: the copies this thread started must have landed first
+          for (int u = max(0, t - ST); u < t; ++u) mbar_wait_plain_bounded(bar_full + u % ST, (u / ST) & 1, WAIT_LIMIT);
+      };
+      if (warp == 8) produce(std::true_type{}, &tm_k, sK, bar_kfull, bar_sready);
+      else produce(std::false_type{}, &tm_v, sV, bar_vfull, bar_pvdone);
     } else if (warp == 10) {
       // ---------------------------------------------------------------- MMA issuer: S = Q.K^T
       // (the two issuers are separate warps so that a P.V group waiting for room in the tensor
       // queue does not hold back the next scores, and vice versa)
-      // Every tile of the walk passes through an issuer, so its instruction count per tile is on the
-      // kernel's critical path.  Hence: barrier addresses and the stage-0 descriptor are formed once,
-      // the polls of a tile's barriers are issued together, ring position and phase are counters, and
-      // the lane masks are compile-time constants of three instantiations of the tile code (W = 0
-      // upper half, 1 lower half, 2 both halves, unmasked form).
+      // Every step of the walk passes through an issuer, so its instruction count per step is on the
+      // kernel's critical path.  Hence: barrier addresses and the slot-0 descriptor are formed once,
+      // the polls of a step's barriers are issued together, ring position and phase are counters, and
+      // the lane masks are compile-time constants of the instantiations of the step code (W = FORM_*).
       // The whole warp runs this loop converged (values below are made warp-uniform with a shuffle from
       // lane 0, every decision is a vote), so that descriptors and addresses live in uniform registers;
       // the tcgen05 instructions themselves are guarded by the elected lane's predicate.
-      constexpr uint32_t IDESC_QK = instr_desc(2, 1, 1, 128, 64);  // s32 += s8 * s8
+      constexpr uint32_t IDESC_QK = instr_desc(2, 1, 1, 128, 64);        // s32 += s8 * s8
+      constexpr uint32_t IDESC_QK_DUAL = instr_desc(2, 1, 1, 64, 128);   // two tiles of 64 keys, one per half
       const uint32_t lead = elect_one();
       const int n_steps_u = __shfl_sync(0xffffffffu, n_steps, 0);
       const uint32_t tS_u = __shfl_sync(0xffffffffu, tS, 0), tQ_u = tS_u + 96u;
@@ -290,69 +263,48 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         const uint32_t a_sfree = smem_u32(bar_sfree), a_sready = smem_u32(bar_sready);
         const uint32_t a_kfull = smem_u32(bar_kfull);
         const uint64_t dK0 = smem_desc(smem_u32(sK), D);
-        uint32_t st = 0, kph = 0;   // ring stage of the next tile and the parity of its current use
-        // the MMAs of one tile and their commit
-        auto issue = [&](auto wtag, const int i, const uint32_t stage) {
+        uint32_t st = 0, kph = 0;   // ring slot of the next step and the parity of its current use
+        // the MMAs of one step and their commits
+        auto issue = [&](auto wtag, const int i, const uint32_t slot) {
           constexpr int W = decltype(wtag)::value;
-          const uint64_t dK = dK0 + (uint64_t)(stage * (uint32_t)(Cfg::K_BYTES >> 4));
+          const uint64_t dK = dK0 + (uint64_t)(slot * (uint32_t)(2 * Cfg::K_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < D / 32; ++k) {
-            if (W == 2) mma_i8_ts_p(lead, tS_u, tQ_u + 8 * k, desc_advance(dK, 32 * k), IDESC_QK, k > 0);
-            else if (W == 0)   // lanes NOT written: the rows of the half the tile does not serve
+            if (W == FORM_DUAL) mma_ws_i8_ts_p(lead, tS_u, tQ_u + 8 * k, desc_advance(dK, 32 * k), IDESC_QK_DUAL, k > 0);
+            else if (W == FORM_SHARED) mma_i8_ts_p(lead, tS_u, tQ_u + 8 * k, desc_advance(dK, 32 * k), IDESC_QK, k > 0);
+            else if (W == FORM_UPPER)   // lanes NOT written: the rows of the half the tile does not serve
               mma_i8_ts_masked_p(lead, tS_u, tQ_u + 8 * k, desc_advance(dK, 32 * k), IDESC_QK, k > 0, 0u, 0u, 0xffffffffu, 0xffffffffu);
             else
               mma_i8_ts_masked_p(lead, tS_u, tQ_u + 8 * k, desc_advance(dK, 32 * k), IDESC_QK, k > 0, 0xffffffffu, 0xffffffffu, 0u, 0u);
           }
           // one commit per half served: the softmax warps wait on it for the scores, the K producer for the stage
-          if (W != 1) mma_commit_at_p(lead, a_sready + 8u * (uint32_t)(i & 3));
-          if (W != 0) mma_commit_at_p(lead, a_sready + 32u + 8u * (uint32_t)(i & 3));
+          if (W != FORM_LOWER) mma_commit_at_p(lead, a_sready + 8u * (uint32_t)(i & 3));
+          if (W != FORM_UPPER) mma_commit_at_p(lead, a_sready + 32u + 8u * (uint32_t)(i & 3));
         };
-        auto tile = [&](auto wtag, const int i, const int ev) -> bool {
+        auto step = [&](auto wtag, const int i) -> bool {
           constexpr int W = decltype(wtag)::value;
           // the scores of step i-1 of the halves served are in registers: their rows of S may be
           // overwritten.  (i = 0 asks an unused barrier for parity 1, which passes at once.)
           const uint32_t par = (uint32_t)(i - 1) & 1u, ph = ((uint32_t)(i - 1) >> 1) & 1u;
-          TRL(2, i, ev + 0);
-          const bool r0 = W == 1 || mbar_poll(a_sfree + 8u * par, ph);
-          const bool r1 = W == 0 || mbar_poll(a_sfree + 16u + 8u * par, ph);
+          TRL(2, i, 0);
+          const bool r0 = W == FORM_LOWER || mbar_poll(a_sfree + 8u * par, ph);
+          const bool r1 = W == FORM_UPPER || mbar_poll(a_sfree + 16u + 8u * par, ph);
           const bool r2 = mbar_poll(a_kfull + 8u * st, kph);
           if (!__all_sync(0xffffffffu, r0 && r1 && r2)) {
             bool good = true;
-            if (W != 1) good = mbar_wait_bounded(bar_sfree + par, ph, abort_flag, WAIT_LIMIT);
-            if (W != 0) good = good && mbar_wait_bounded(bar_sfree + 2 + par, ph, abort_flag, WAIT_LIMIT);
+            if (W != FORM_LOWER) good = mbar_wait_bounded(bar_sfree + par, ph, abort_flag, WAIT_LIMIT);
+            if (W != FORM_UPPER) good = good && mbar_wait_bounded(bar_sfree + 2 + par, ph, abort_flag, WAIT_LIMIT);
             good = good && mbar_wait_bounded(bar_kfull + st, kph, abort_flag, WAIT_LIMIT);
             if (!__all_sync(0xffffffffu, good)) return false;
           }
-          TRL(2, i, ev + 1);
+          TRL(2, i, 1);
           tc_fence_after();
           issue(wtag, i, st);
           if (++st == KST) {
             st = 0;
             kph ^= 1u;
           }
-          TRL(2, i, ev + 3);
-          return true;
-        };
-        // A side-by-side step (one tile per half) whose four barriers are all complete -- the usual case
-        // while this thread is what the walk waits for -- is issued as straight-line code: one branch for
-        // the step instead of one per poll, tile and ring wrap (a taken branch costs a lone thread
-        // about as much as issuing an MMA).
-        auto both = [&](const int i) -> bool {
-          const uint32_t par = (uint32_t)(i - 1) & 1u, ph = ((uint32_t)(i - 1) >> 1) & 1u;
-          const uint32_t wrap1 = st + 1 == KST ? 1u : 0u, st1 = wrap1 ? 0u : st + 1, ph1 = kph ^ wrap1;
-          TRL(2, i, 0);
-          const bool r0 = mbar_poll(a_sfree + 8u * par, ph), r1 = mbar_poll(a_sfree + 16u + 8u * par, ph);
-          const bool r2 = mbar_poll(a_kfull + 8u * st, kph), r3 = mbar_poll(a_kfull + 8u * st1, ph1);
-          if (!__all_sync(0xffffffffu, r0 & r1 & r2 & r3)) return false;
-          TRL(2, i, 1);
-          tc_fence_after();
-          issue(std::integral_constant<int, 0>{}, i, st);
           TRL(2, i, 3);
-          issue(std::integral_constant<int, 1>{}, i, st1);
-          const uint32_t wrap2 = st1 + 1 == KST ? 1u : 0u;
-          st = wrap2 ? 0u : st1 + 1;
-          kph = ph1 ^ wrap2;
-          TRL(2, i, 7);
           return true;
         };
         uint32_t e_cur = n_steps_u > 0 ? sched[0] : 0u, e_nxt = n_steps_u > 1 ? sched[1] : 0u;
@@ -362,13 +314,11 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           e_cur = e_nxt;
           if (i + 2 < n_steps_u) e_nxt = ld_pinned_u32(sched + i + 2);
           bool good;
-          if (SHARE_TILES && ka == kb && ka != 0xFFFFu) {
-            good = tile(std::integral_constant<int, 2>{}, i, 0);
-          } else {
-            if (FUSE_STEPS && ka != 0xFFFFu && kb != 0xFFFFu && both(i)) continue;
-            good = ka == 0xFFFFu || tile(std::integral_constant<int, 0>{}, i, 0);
-            good = good && (kb == 0xFFFFu || tile(std::integral_constant<int, 1>{}, i, 4));
-          }
+          if (ka != 0xFFFFu && kb != 0xFFFFu)
+            good = ka == kb ? step(std::integral_constant<int, FORM_SHARED>{}, i) : step(std::integral_constant<int, FORM_DUAL>{}, i);
+          else
+            good = (ka == 0xFFFFu || step(std::integral_constant<int, FORM_UPPER>{}, i)) &&
+                   (kb == 0xFFFFu || step(std::integral_constant<int, FORM_LOWER>{}, i));
           if (!good) {
             report_timeout(p, abort_flag, 3, i);
             break;
@@ -381,7 +331,8 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
     } else if (warp == 11) {
       // ---------------------------------------------------------------- MMA issuer: O += P.V
-      constexpr uint32_t IDESC_PV = instr_desc(1, 1, 1, 128, D);   // f32 += bf16 * bf16
+      constexpr uint32_t IDESC_PV = instr_desc(1, 1, 1, 128, D);            // f32 += bf16 * bf16
+      constexpr uint32_t IDESC_PV_DUAL = instr_desc(1, 1, 1, 64, 2 * D);   // two tiles, one per half
       const uint32_t lead = elect_one();
       const int n_steps_u = __shfl_sync(0xffffffffu, n_steps, 0);
       const uint32_t tS_u = __shfl_sync(0xffffffffu, tS, 0), tP_u = tS_u + 64u, tO_u = tS_u + 128u;
@@ -389,64 +340,47 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       const uint32_t a_vfull = smem_u32(bar_vfull);
       const uint64_t dV0 = smem_desc(smem_u32(sV), 128);
       uint32_t st = 0, vph = 0;
-      auto issue = [&](auto wtag, const int i, const uint32_t stage) {
+      auto issue = [&](auto wtag, const int i, const uint32_t slot) {
         constexpr int W = decltype(wtag)::value;
-        const uint64_t dV = dV0 + (uint64_t)(stage * (uint32_t)(Cfg::V_BYTES >> 4));
+        const uint64_t dV = dV0 + (uint64_t)(slot * (uint32_t)(2 * Cfg::V_BYTES >> 4));
         // both halves start at step 0, so a tile that serves both never mixes a first with a later step
         const uint32_t acc0 = i > 0 ? 1u : 0u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t acc = k > 0 ? 1u : acc0;
-          if (W == 2) mma_f16_ts_p(lead, tO_u, tP_u + 8 * k, desc_advance(dV, 32 * k), IDESC_PV, acc);
-          else if (W == 0)
+          if (W == FORM_DUAL) mma_ws_f16_ts_p(lead, tO_u, tP_u + 8 * k, desc_advance(dV, 32 * k), IDESC_PV_DUAL, acc);
+          else if (W == FORM_SHARED) mma_f16_ts_p(lead, tO_u, tP_u + 8 * k, desc_advance(dV, 32 * k), IDESC_PV, acc);
+          else if (W == FORM_UPPER)
             mma_f16_ts_masked_p(lead, tO_u, tP_u + 8 * k, desc_advance(dV, 32 * k), IDESC_PV, acc, 0u, 0u, 0xffffffffu, 0xffffffffu);
           else
             mma_f16_ts_masked_p(lead, tO_u, tP_u + 8 * k, desc_advance(dV, 32 * k), IDESC_PV, acc, 0xffffffffu, 0xffffffffu, 0u, 0u);
         }
         // one commit per half served: P of that half may be rewritten, and the V producer takes it for the stage
-        if (W != 1) mma_commit_at_p(lead, a_pvdone + 8u * (uint32_t)(i & 3));
-        if (W != 0) mma_commit_at_p(lead, a_pvdone + 32u + 8u * (uint32_t)(i & 3));
+        if (W != FORM_LOWER) mma_commit_at_p(lead, a_pvdone + 8u * (uint32_t)(i & 3));
+        if (W != FORM_UPPER) mma_commit_at_p(lead, a_pvdone + 32u + 8u * (uint32_t)(i & 3));
       };
-      auto tile = [&](auto wtag, const int i, const int ev) -> bool {
+      auto step = [&](auto wtag, const int i) -> bool {
         constexpr int W = decltype(wtag)::value;
         const uint32_t par = (uint32_t)i & 1u, ph = ((uint32_t)i >> 1) & 1u;
-        TRL(3, i, ev + 0);
-        const bool r0 = W == 1 || mbar_poll(a_pready + 8u * par, ph);
-        const bool r1 = W == 0 || mbar_poll(a_pready + 16u + 8u * par, ph);
+        TRL(3, i, 0);
+        const bool r0 = W == FORM_LOWER || mbar_poll(a_pready + 8u * par, ph);
+        const bool r1 = W == FORM_UPPER || mbar_poll(a_pready + 16u + 8u * par, ph);
         const bool r2 = mbar_poll(a_vfull + 8u * st, vph);
         if (!__all_sync(0xffffffffu, r0 && r1 && r2)) {
           bool good = true;
-          if (W != 1) good = mbar_wait_bounded(bar_pready + par, ph, abort_flag, WAIT_LIMIT);
-          if (W != 0) good = good && mbar_wait_bounded(bar_pready + 2 + par, ph, abort_flag, WAIT_LIMIT);
+          if (W != FORM_LOWER) good = mbar_wait_bounded(bar_pready + par, ph, abort_flag, WAIT_LIMIT);
+          if (W != FORM_UPPER) good = good && mbar_wait_bounded(bar_pready + 2 + par, ph, abort_flag, WAIT_LIMIT);
           good = good && mbar_wait_bounded(bar_vfull + st, vph, abort_flag, WAIT_LIMIT);
           if (!__all_sync(0xffffffffu, good)) return false;
         }
-        TRL(3, i, ev + 1);
+        TRL(3, i, 1);
         tc_fence_after();
         issue(wtag, i, st);
         if (++st == VST) {
           st = 0;
           vph ^= 1u;
         }
-        TRL(3, i, ev + 3);
-        return true;
-      };
-      auto both = [&](const int i) -> bool {   // (as in the Q.K^T issuer)
-        const uint32_t par = (uint32_t)i & 1u, ph = ((uint32_t)i >> 1) & 1u;
-        const uint32_t wrap1 = st + 1 == VST ? 1u : 0u, st1 = wrap1 ? 0u : st + 1, ph1 = vph ^ wrap1;
-        TRL(3, i, 0);
-        const bool r0 = mbar_poll(a_pready + 8u * par, ph), r1 = mbar_poll(a_pready + 16u + 8u * par, ph);
-        const bool r2 = mbar_poll(a_vfull + 8u * st, vph), r3 = mbar_poll(a_vfull + 8u * st1, ph1);
-        if (!__all_sync(0xffffffffu, r0 & r1 & r2 & r3)) return false;
-        TRL(3, i, 1);
-        tc_fence_after();
-        issue(std::integral_constant<int, 0>{}, i, st);
         TRL(3, i, 3);
-        issue(std::integral_constant<int, 1>{}, i, st1);
-        const uint32_t wrap2 = st1 + 1 == VST ? 1u : 0u;
-        st = wrap2 ? 0u : st1 + 1;
-        vph = ph1 ^ wrap2;
-        TRL(3, i, 7);
         return true;
       };
       uint32_t e_cur = n_steps_u > 0 ? sched[0] : 0u, e_nxt = n_steps_u > 1 ? sched[1] : 0u;
@@ -456,13 +390,11 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         e_cur = e_nxt;
         if (i + 2 < n_steps_u) e_nxt = ld_pinned_u32(sched + i + 2);
         bool good;
-        if (SHARE_TILES && ka == kb && ka != 0xFFFFu) {
-          good = tile(std::integral_constant<int, 2>{}, i, 0);
-        } else {
-          if (FUSE_STEPS && ka != 0xFFFFu && kb != 0xFFFFu && both(i)) continue;
-          good = ka == 0xFFFFu || tile(std::integral_constant<int, 0>{}, i, 0);
-          good = good && (kb == 0xFFFFu || tile(std::integral_constant<int, 1>{}, i, 4));
-        }
+        if (ka != 0xFFFFu && kb != 0xFFFFu)
+          good = ka == kb ? step(std::integral_constant<int, FORM_SHARED>{}, i) : step(std::integral_constant<int, FORM_DUAL>{}, i);
+        else
+          good = (ka == 0xFFFFu || step(std::integral_constant<int, FORM_UPPER>{}, i)) &&
+                 (kb == 0xFFFFu || step(std::integral_constant<int, FORM_LOWER>{}, i));
         if (!good) {
           report_timeout(p, abort_flag, 5, i);
           break;

@@ -343,6 +343,30 @@ __device__ __forceinline__ void mma_f16_ts_masked_p(uint32_t lead, uint32_t d_tm
         "r"(lead)
       : "memory");
 }
+// The M = 64 forms of tcgen05.mma.ws with A in TMEM.  N is split over the two halves of the lanes: lanes 0-63
+// hold accumulator columns of B's rows 0..N/2-1, lanes 64-127 those of rows N/2..N-1, and each half of the
+// lanes multiplies by the A rows that lie in its own lanes.  With different A rows in the two halves ONE
+// instruction therefore computes two independent 64-row products, A_lo * B_lo^T and A_hi * B_hi^T.
+__device__ __forceinline__ void mma_ws_i8_ts_p(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                               uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.ws.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ws_f16_ts_p(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.ws.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ void mma_commit_at_p(uint32_t lead, uint32_t bar_saddr) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
