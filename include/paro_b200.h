@@ -275,6 +275,45 @@ int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16_t* v16,
                      int32_t* redo, size_t redo_bytes,
                      int32_t* status, paro_stream_t stream);
 
+/* One self-attention layer per call: what the entry points above do in sequence -- Q normalised, rotated,
+ * reordered and quantised per 32 rows, K per 64 rows (smooth_k: its mean over tokens taken out), V per channel,
+ * block-sparse attention, rows stored back in natural token order -- with the same results bit for bit, issued from one
+ * call on one work space of paro_layer_workspace_bytes(args) bytes (device memory, 16-byte aligned, contents irrelevant;
+ * calls that share one must be on one stream).  q, k, v, out: [B,H,N,D] through element strides {b, h, n}, all of `dtype`.
+ * Norm parameters as in paro_prep_qk_int8_norm (the RMS statistic is computed here).  host_status (nullable): four words
+ * of PINNED host memory that receive the status words when a wait expires.  ev_start / ev_stop (nullable): CUDA events
+ * recorded around the attention kernel.  Everything else as in paro_prep_qk_int8, paro_prep_v_fp8 and paro_sparse_attn. */
+typedef struct {
+  const void *q, *k, *v;
+  int64_t q_strides[3], k_strides[3], v_strides[3];
+  int dtype, B, H, N, D;
+  int n_text, F, Hh, W;
+  const int32_t* order_ids;
+  const void *cos_tab, *sin_tab;
+  int rope_mode, pairs_f, pairs_h;
+  int q_norm_mode, k_norm_mode;
+  float q_norm_eps, k_norm_eps;
+  const void *q_norm_weight, *q_norm_bias, *k_norm_weight, *k_norm_bias;
+  int smooth_k, smooth_v;
+  const int32_t* pair_ptr;
+  const uint32_t* sched;
+  const int32_t* sched_cnt;
+  int plan_slices, attn_mode;
+  const int32_t* inv_idx;
+  void* out;
+  int64_t out_strides[3];
+  float* lse;
+  float sm_scale;
+  int32_t* redo;
+  size_t redo_bytes;
+  int32_t *status, *host_status;
+  void* workspace;
+  size_t workspace_bytes;
+  void *ev_start, *ev_stop;
+} paro_layer_args;
+size_t paro_layer_workspace_bytes(const paro_layer_args* args);
+int paro_layer(const paro_layer_args* args, paro_stream_t stream);
+
 /* Merges two partial results of paro_sparse_attn computed over DISJOINT sets of key blocks (for
  * instance the two halves of a sequence held by two ranks) into the result over their union:
  * lse = log(exp(lse_a) + exp(lse_b)), out = o_a * exp(lse_a - lse) + o_b * exp(lse_b - lse), fp32 math,

@@ -14,7 +14,7 @@ import threading
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_PATH = os.path.join(HERE, "libparo_b200.so")
-SOURCES = ("common.cu", "perm_plan.cu", "plan_compact.cu", "rope_permute.cu", "quant.cu", "sparse_attn.cu", "attn_aux.cu")
+SOURCES = ("common.cu", "perm_plan.cu", "plan_compact.cu", "rope_permute.cu", "quant.cu", "sparse_attn.cu", "attn_aux.cu", "layer.cu")
 NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "-shared")
 
@@ -80,6 +80,23 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 _i32, _i64, _f32, _vp, _sz = ctypes.c_int, ctypes.c_int64, ctypes.c_float, ctypes.c_void_p, ctypes.c_size_t
 
+
+
+class LayerArgs(ctypes.Structure):
+    """paro_layer_args of include/paro_b200.h, field by field."""
+    _fields_ = [
+        ("q", _vp), ("k", _vp), ("v", _vp), ("q_strides", _i64 * 3), ("k_strides", _i64 * 3), ("v_strides", _i64 * 3),
+        ("dtype", _i32), ("B", _i32), ("H", _i32), ("N", _i32), ("D", _i32),
+        ("n_text", _i32), ("F", _i32), ("Hh", _i32), ("W", _i32), ("order_ids", _vp),
+        ("cos_tab", _vp), ("sin_tab", _vp), ("rope_mode", _i32), ("pairs_f", _i32), ("pairs_h", _i32),
+        ("q_norm_mode", _i32), ("k_norm_mode", _i32), ("q_norm_eps", _f32), ("k_norm_eps", _f32),
+        ("q_norm_weight", _vp), ("q_norm_bias", _vp), ("k_norm_weight", _vp), ("k_norm_bias", _vp),
+        ("smooth_k", _i32), ("smooth_v", _i32), ("pair_ptr", _vp), ("sched", _vp), ("sched_cnt", _vp),
+        ("plan_slices", _i32), ("attn_mode", _i32), ("inv_idx", _vp), ("out", _vp), ("out_strides", _i64 * 3),
+        ("lse", _vp), ("sm_scale", _f32), ("redo", _vp), ("redo_bytes", _sz), ("status", _vp), ("host_status", _vp),
+        ("workspace", _vp), ("workspace_bytes", _sz), ("ev_start", _vp), ("ev_stop", _vp)]
+
+
 SIGNATURES = {
     "paro_version": (ctypes.c_int, []),
     "paro_last_error": (ctypes.c_char_p, []),
@@ -111,6 +128,8 @@ SIGNATURES = {
     "paro_sparse_attn_redo_bytes": (_sz, [_i32, _i32, _i32]),
     "paro_sparse_attn": (_i32, [_vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _i32, _vp, _i32,
                                 _i64, _i64, _i64, _vp, _i32, _i32, _i32, _i32, _f32, _i32, _vp, _sz, _vp, _vp]),
+    "paro_layer_workspace_bytes": (_sz, [ctypes.POINTER(LayerArgs)]),
+    "paro_layer": (_i32, [ctypes.POINTER(LayerArgs), _vp]),
     "paro_status_poll": (_i32, [_vp, _vp, _vp]),
     "paro_plan_validate": (_i32, [_vp, _vp, _vp, _i32, _i32, _i32, _i64, _vp, _vp]),
     "paro_merge_attn_states": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i64, _i64, _i64, _vp]),

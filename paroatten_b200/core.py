@@ -1,6 +1,8 @@
 """Sparse-attention entry points (reference: paroattention/core.py)."""
 from __future__ import annotations
 
+import contextlib
+import ctypes
 from typing import Any, Optional, Sequence, Tuple, Union
 
 import torch
@@ -8,9 +10,8 @@ import torch.nn.functional as F
 
 from . import _lib
 from .plan import (CompactPlan, PermutePlan, PlanStore, SparsePlan, apply_empty_heads, compact_plan, perm_index)
-from .quant import (_hnd, _quant_int8, channel_mean, per_channel_fp8, per_warp_int8, per_block_int8, prep_qk_int8,
-                    prep_v_fp8)
-from .rope import RopeTables, rope_permute
+from .quant import _hnd, channel_mean, per_channel_fp8, per_warp_int8, per_block_int8
+from .rope import RopeTables, _norm_params
 
 _status = {}
 _status_mirror = {}   # device index -> pinned host copy of the status words, refreshed after every launch
@@ -76,12 +77,11 @@ def _mirror(device: torch.device) -> torch.Tensor:
 
 
 def _raise_if_earlier_launch_failed(device: torch.device) -> None:
-    """Every attention launch is followed by an asynchronous copy of the status words into pinned host
-    memory; each new call looks at that copy first (no synchronisation).  A launch that gave up a wait
+    """The status words also reach pinned host memory (copied after the launch, or written by the kernel itself
+    when a wait expires); each new call looks at that copy first (no synchronisation).  A launch that gave up a wait
     therefore stops the caller at the next attention call at the latest, instead of every later launch
     returning at once and leaving its output unwritten."""
-    m = _mirror(device)
-    if int(m[0]) != 0:
+    if ctypes.c_int32.from_address(_mirror(device).data_ptr()).value != 0:
         check_status(device)      # synchronises, clears the words and raises with the waiter's position
 
 
@@ -152,6 +152,65 @@ def sparse_attn_quantized(q_int8, q_scale, k_int8, k_scale, v16, v_scale, vm, pl
             sink.append(ev)
         _mirror(dev).copy_(_status_words(dev), non_blocking=True)
     return (out, lse) if return_lse else out
+
+
+def _on(device: torch.device):
+    """torch.cuda.device(device), or nothing to enter when it is the current device already."""
+    return contextlib.nullcontext() if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def _layer(q, k, v, orders, index, plan: CompactPlan, grid, n_text: int, rope: Optional[RopeTables], tensor_layout: str,
+           sm_scale: float, smooth_k: bool, smooth_v: bool, return_lse: bool, q_norm, k_norm, mode: str):
+    """paro_layer on tensors whose head dimension is 64 or 128: (out, lse or None)."""
+    if mode not in ("fast", "exact"):
+        raise ValueError(f"unknown mode {mode!r}")
+    dev = q.device
+    qv, kv, vv = _hnd(q, tensor_layout), _hnd(k, tensor_layout), _hnd(v, tensor_layout)
+    B, H, N, D = qv.shape
+    nb = (N + 63) // 64
+    if kv.shape != qv.shape or vv.shape != qv.shape:
+        raise ValueError("q, k and v must have the same shape")
+    if plan.nbq != nb or plan.nbk != nb:
+        raise ValueError(f"sparse plan is {plan.nbq}x{plan.nbk} blocks but the sequence has {nb}")
+    if plan.slices not in (H, B * H):
+        raise ValueError(f"sparse plan has {plan.slices} slices; expected H={H} or B*H={B * H}")
+    if orders.numel() != H:
+        raise ValueError("order_ids must hold one id per head")
+    if index.dtype != torch.int32 or tuple(index.shape) != (H, N - n_text) or not index.is_contiguous():
+        raise ValueError(f"inv_index must be contiguous int32 [H, N - n_text] = [{H}, {N - n_text}]")
+    _lib.require_cuda(orders, index, plan.pair_ptr, plan.sched)
+    L = _lib.lib()
+    _raise_if_earlier_launch_failed(dev)
+    out = torch.empty((B, H, N, D) if tensor_layout == "HND" else (B, N, H, D), dtype=q.dtype, device=dev)
+    ov = out if tensor_layout == "HND" else out.transpose(1, 2)
+    lse = torch.empty(B, H, N, dtype=torch.float32, device=dev) if return_lse else None
+    qn, qw, qb, qeps = _norm_params(q_norm, H, D, q)
+    kn, kw, kb, keps = _norm_params(k_norm, H, D, k)
+    redo = _redo_space(dev, B, H, N) if mode == "fast" else None
+    ev = None
+    if _timing_sink is not None:
+        ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+        for e in ev:
+            e.record()       # (creates the event; the call below records both again where they belong)
+    cnt = plan.sched_cnt_kernel if plan.sched_cnt_kernel is not None else plan.sched_cnt
+    three = ctypes.c_int64 * 3
+    a = _lib.LayerArgs(
+        qv.data_ptr(), kv.data_ptr(), vv.data_ptr(), three(*qv.stride()[:3]), three(*kv.stride()[:3]),
+        three(*vv.stride()[:3]), _lib.dtype_code(q.dtype), B, H, N, D, n_text, *grid, orders.data_ptr(),
+        None if rope is None else _lib.ptr(rope.cos), None if rope is None else _lib.ptr(rope.sin),
+        _lib.ROPE_NONE if rope is None else rope.mode, 0 if rope is None else rope.pairs_f,
+        0 if rope is None else rope.pairs_h, qn, kn, qeps, keps, _lib.ptr(qw), _lib.ptr(qb), _lib.ptr(kw), _lib.ptr(kb),
+        bool(smooth_k), bool(smooth_v), plan.pair_ptr.data_ptr(), plan.sched.data_ptr(), cnt.data_ptr(), plan.slices,
+        _lib.ATTN_FAST if mode == "fast" else _lib.ATTN_EXACT, index.data_ptr(), out.data_ptr(), three(*ov.stride()[:3]),
+        _lib.ptr(lse), sm_scale, _lib.ptr(redo), redo.numel() * 4 if redo is not None else 0,
+        _status_words(dev).data_ptr(), _mirror(dev).data_ptr(), None, 0,
+        None if ev is None else ev[0].cuda_event, None if ev is None else ev[1].cuda_event)
+    workspace = torch.empty(L.paro_layer_workspace_bytes(a), dtype=torch.uint8, device=dev)
+    a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
+    _lib.check(L.paro_layer(a, _lib.stream_ptr()))
+    if ev is not None:
+        _timing_sink.append(ev)
+    return out, lse
 
 
 def merge_attention_states(o_a: torch.Tensor, lse_a: torch.Tensor, o_b: torch.Tensor, lse_b: torch.Tensor,
@@ -294,7 +353,7 @@ def paro_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, permute_pl
     if sm_scale is None:
         sm_scale = head_dim_og ** -0.5
     dev = q.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         empty = None
         if isinstance(permute_plan, PermutePlan):
             orders, index = permute_plan.orders(i_block), permute_plan.index(i_block)
@@ -324,30 +383,18 @@ def paro_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, permute_pl
         # Q and V: the quantisers read the natural-order tensors through the RoPE + reordering front end
         # (no reordered 16-bit copy).  Smoothed K needs the mean of the rotated values first; rotating
         # twice costs more than writing the rotated copy once, so K keeps the two-step form.
-        q8, qs, _ = prep_qk_int8(q, orders, grid, n_text, rope, group=32, tensor_layout=tensor_layout, norm=q_norm)
-        if smooth_k:
-            kp = rope_permute(k, orders, grid, n_text, rope, tensor_layout=tensor_layout, norm=k_norm)
-            k8, ks = _quant_int8(kp, "HND", 64, km=channel_mean(kp))
-        else:
-            k8, ks, _ = prep_qk_int8(k, orders, grid, n_text, rope, group=64, tensor_layout=tensor_layout,
-                                     norm=k_norm)
-        v16, vs, vm, _ = prep_v_fp8(v, orders, grid, n_text, smooth_v=smooth_v, tensor_layout=tensor_layout)
-        res = sparse_attn_quantized(q8, qs, k8, ks, v16, vs, vm, plan, sm_scale, out_dtype=q.dtype, q_group=32,
-                                    inv_index=index, n_text=n_text, return_lse=return_lse, out_layout=tensor_layout,
-                                    mode=attn_mode)
+        o, lse = _layer(q, k, v, orders, index, plan, grid, int(n_text), rope, tensor_layout, float(sm_scale), smooth_k,
+                        smooth_v, return_lse, q_norm, k_norm, attn_mode)
         if empty is not None and empty_head_mode == "uniform":
-            # uniform attention over all N tokens: O = mean of V (the channel mean the V quantiser produced,
-            # or one reduction when smoothing is off); LSE of N equal scores of value 0
-            o_, _ = res if return_lse else (res, None)
-            mean_v = vm if vm is not None else channel_mean(v, tensor_layout, out_dtype=torch.float32)
+            # uniform attention over all N tokens: O = mean of V; LSE of N equal scores of value 0
+            mean_v = channel_mean(v, tensor_layout, out_dtype=torch.float32)
             hsel = empty.nonzero().flatten()
-            fill = mean_v[:, hsel].to(o_.dtype)                       # [B, n_empty, D]
+            fill = mean_v[:, hsel].to(o.dtype)                        # [B, n_empty, D]
             if tensor_layout == "HND":
-                o_[:, hsel] = fill.unsqueeze(2).expand(-1, -1, o_.shape[2], -1)
+                o[:, hsel] = fill.unsqueeze(2).expand(-1, -1, o.shape[2], -1)
             else:
-                o_[:, :, hsel] = fill.unsqueeze(1).expand(-1, o_.shape[1], -1, -1)
+                o[:, :, hsel] = fill.unsqueeze(1).expand(-1, o.shape[1], -1, -1)
             if return_lse:
-                res[1][:, hsel] = float(torch.log(torch.tensor(float(q.shape[2 if tensor_layout == "HND" else 1]))))
-    o, lse = res if return_lse else (res, None)
+                lse[:, hsel] = float(torch.log(torch.tensor(float(q.shape[2 if tensor_layout == "HND" else 1]))))
     o = o[..., :head_dim_og]
     return (o, lse) if return_lse else o

@@ -31,6 +31,7 @@ struct AttnParams {
   void* out;
   float* lse;
   int32_t* status;
+  int32_t* host_status; // nullable: pinned host copy of the status words, written when a wait expires
   int32_t* redo;        // work space described above
   int64_t osb, osh, osn;
   int plan_slices, q_group, n_text;
@@ -90,6 +91,14 @@ __device__ __forceinline__ void report_timeout(const AttnParams& p, volatile int
     p.status[1] = where;
     p.status[2] = (int)blockIdx.x;
     p.status[3] = iter;
+    if (p.host_status) {
+      volatile int32_t* h = p.host_status;
+      h[1] = where;
+      h[2] = (int)blockIdx.x;
+      h[3] = iter;
+      __threadfence_system();
+      h[0] = PARO_ETIMEOUT;
+    }
   }
   *abort_flag = 1;
 }
@@ -132,5 +141,13 @@ template <int S> struct ReleaseFifo {
 __device__ __forceinline__ uint32_t commit_token(uint32_t bars_saddr, int half, int step) {
   return (bars_saddr + 32u * (uint32_t)half + 8u * ((uint32_t)step & 3u)) | ((((uint32_t)step >> 2) & 1u) << 31);
 }
+
+// paro_sparse_attn with a pinned host copy of the status words (nullable).
+int sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t* v16, const float* q_scale, int q_group,
+                       const float* k_scale, const float* v_scale, const float* vm, const int32_t* pair_ptr,
+                       const uint32_t* sched, const int32_t* sched_cnt, int plan_slices, const int32_t* inv_idx, int n_text,
+                       void* out, int out_dtype, int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_n, float* lse,
+                       int B, int H, int N, int D, float sm_scale, int mode, int32_t* redo, size_t redo_bytes,
+                       int32_t* status, int32_t* host_status, cudaStream_t s);
 
 }  // namespace paro

@@ -1,0 +1,124 @@
+// One self-attention layer per call: the pre-attention passes and the attention kernel of
+// paro_attention, issued from one C entry point on one caller-provided work space.
+//
+// A layer is about ten launches.  Composed from Python (one ctypes call, its argument checks and two or three
+// tensor allocations per pass) they cost about 190 us of host time, which is what a call of a few thousand
+// tokens took; the device needs a fraction of that.  Here the host side is one call and the launches: 187 -> 74 us
+// for 2 heads x 1024 tokens, 194 -> 158 us for 6 x 5960 (where the device is what remains).
+#include "attn_common.cuh"
+#include "common.cuh"
+
+using namespace paro;
+
+namespace {
+
+// Sections of the work space, each on a 256-byte boundary.
+struct Sections {
+  size_t q8, k8, v16, qs, ks, vs, vm, km, kp, rms_q, rms_k, stats, total;
+};
+
+Sections sections(const paro_layer_args& a) {
+  const size_t BH = (size_t)a.B * a.H, rows = BH * a.N, D = a.D, nb = ((size_t)a.N + 63) / 64;
+  Sections s{};
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t here = at;
+    at += (bytes + 255) / 256 * 256;
+    return here;
+  };
+  s.q8 = take(rows * D);
+  s.k8 = take(rows * D);
+  s.v16 = take(BH * D * nb * 64 * 2);
+  s.qs = take(BH * nb * 2 * sizeof(float));
+  s.ks = take(BH * nb * sizeof(float));
+  s.vs = take(BH * D * sizeof(float));
+  s.vm = take(BH * D * sizeof(float));
+  s.km = take(BH * D * 2);
+  s.kp = take(a.smooth_k ? rows * D * 2 : 0);
+  s.rms_q = take(a.q_norm_mode == PARO_NORM_RMS_ALL ? (size_t)a.B * a.N * sizeof(float) : 0);
+  s.rms_k = take(a.k_norm_mode == PARO_NORM_RMS_ALL ? (size_t)a.B * a.N * sizeof(float) : 0);
+  s.stats = take(paro_channel_stats_scratch_bytes(a.B, a.H, a.N, a.D));
+  s.total = at;
+  return s;
+}
+
+}  // namespace
+
+extern "C" size_t paro_layer_workspace_bytes(const paro_layer_args* a) {
+  if (!a || a->B <= 0 || a->H <= 0 || a->N <= 0 || (a->D != 64 && a->D != 128)) return 0;
+  return sections(*a).total;
+}
+
+extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
+  PARO_REQUIRE(args, PARO_EINVAL, "paro_layer: null arguments");
+  const paro_layer_args& a = *args;
+  PARO_REQUIRE(a.B > 0 && a.H > 0 && a.N > 0 && (a.D == 64 || a.D == 128), PARO_ESHAPE, "paro_layer: bad sizes");
+  const Sections at = sections(a);
+  PARO_REQUIRE(a.workspace && aligned16(a.workspace) && a.workspace_bytes >= at.total, PARO_ECAP,
+               "paro_layer: work space too small or unaligned (%zu < %zu)", a.workspace_bytes, at.total);
+  cudaStream_t s = (cudaStream_t)stream;
+  uint8_t* w = static_cast<uint8_t*>(a.workspace);
+  int8_t* q8 = reinterpret_cast<int8_t*>(w + at.q8);
+  int8_t* k8 = reinterpret_cast<int8_t*>(w + at.k8);
+  uint16_t* v16 = reinterpret_cast<uint16_t*>(w + at.v16);
+  float *qs = reinterpret_cast<float*>(w + at.qs), *ks = reinterpret_cast<float*>(w + at.ks);
+  float *vs = reinterpret_cast<float*>(w + at.vs), *vm = reinterpret_cast<float*>(w + at.vm);
+  const size_t stats_bytes = at.total - at.stats;
+
+  // the per-token statistic of an RMS norm over all heads
+  auto inv_rms = [&](const void* x, const int64_t* st, int mode, float eps, size_t section, const float** out) -> int {
+    *out = nullptr;
+    if (mode != PARO_NORM_RMS_ALL) return PARO_OK;
+    float* buf = reinterpret_cast<float*>(w + section);
+    *out = buf;
+    return paro_row_inv_rms(x, a.dtype, a.B, a.H, a.N, a.D, st[0], st[1], st[2], eps, buf, stream);
+  };
+  // RoPE + reorder + INT8 of one tensor in one pass
+  auto prep = [&](const void* x, const int64_t* st, int group, int norm, const void* weight, const void* bias,
+                  const float* rms, float eps, int8_t* out, float* scale) -> int {
+    if (norm != PARO_NORM_NONE)
+      return paro_prep_qk_int8_norm(x, a.dtype, a.B, a.H, a.N, a.D, st[0], st[1], st[2], a.n_text, a.F, a.Hh, a.W,
+                                    a.order_ids, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, group, out, scale,
+                                    norm, weight, bias, rms, eps, stream);
+    return paro_prep_qk_int8(x, a.dtype, a.B, a.H, a.N, a.D, st[0], st[1], st[2], a.n_text, a.F, a.Hh, a.W, a.order_ids,
+                             a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, group, 0, nullptr, out, scale,
+                             nullptr, 0, stream);
+  };
+
+  const float* rms = nullptr;
+  if (int rc = inv_rms(a.q, a.q_strides, a.q_norm_mode, a.q_norm_eps, at.rms_q, &rms)) return rc;
+  if (int rc = prep(a.q, a.q_strides, 32, a.q_norm_mode, a.q_norm_weight, a.q_norm_bias, rms, a.q_norm_eps, q8, qs)) return rc;
+
+  if (int rc = inv_rms(a.k, a.k_strides, a.k_norm_mode, a.k_norm_eps, at.rms_k, &rms)) return rc;
+  if (!a.smooth_k) {
+    if (int rc = prep(a.k, a.k_strides, 64, a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, rms, a.k_norm_eps, k8, ks)) return rc;
+  } else {
+    // the mean to subtract is that of the rotated values, so the rotated copy is written once and read twice
+    void *kp = w + at.kp, *km = w + at.km;
+    const int64_t sn = a.D, sh = sn * a.N, sb = sh * a.H;
+    const int rc = a.k_norm_mode == PARO_NORM_NONE
+        ? paro_rope_permute(a.k, kp, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2], a.n_text,
+                            a.F, a.Hh, a.W, a.order_ids, 0, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, stream)
+        : paro_rope_permute_norm(a.k, kp, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2],
+                                 a.n_text, a.F, a.Hh, a.W, a.order_ids, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f,
+                                 a.pairs_h, a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, rms, a.k_norm_eps, stream);
+    if (rc) return rc;
+    if (int r = paro_channel_mean(kp, a.dtype, a.B, a.H, a.N, a.D, sb, sh, sn, km, nullptr, w + at.stats, stats_bytes, stream))
+      return r;
+    if (int r = paro_quant_int8(kp, a.dtype, a.B, a.H, a.N, a.D, sb, sh, sn, km, 0.f, 64, k8, ks, stream)) return r;
+  }
+
+  if (int rc = paro_prep_v_fp8(a.v, a.dtype, a.B, a.H, a.N, a.D, a.v_strides[0], a.v_strides[1], a.v_strides[2], a.n_text,
+                               a.F, a.Hh, a.W, a.order_ids, a.smooth_v, 448.0f, nullptr, v16, vs, a.smooth_v ? vm : nullptr,
+                               w + at.stats, stats_bytes, stream))
+    return rc;
+
+  if (a.ev_start) PARO_CUDA_OK(cudaEventRecord((cudaEvent_t)a.ev_start, s));
+  if (int rc = sparse_attn_launch(q8, k8, v16, qs, 32, ks, vs, a.smooth_v ? vm : nullptr, a.pair_ptr, a.sched, a.sched_cnt,
+                                  a.plan_slices, a.inv_idx, a.n_text, a.out, a.dtype, a.out_strides[0], a.out_strides[1],
+                                  a.out_strides[2], a.lse, a.B, a.H, a.N, a.D, a.sm_scale, a.attn_mode, a.redo, a.redo_bytes,
+                                  a.status, a.host_status, s))
+    return rc;
+  if (a.ev_stop) PARO_CUDA_OK(cudaEventRecord((cudaEvent_t)a.ev_stop, s));
+  return PARO_OK;
+}

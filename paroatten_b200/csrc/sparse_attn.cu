@@ -778,17 +778,12 @@ extern "C" size_t paro_sparse_attn_redo_bytes(int B, int H, int N) {
   return sizeof(int32_t) * (REDO_HEADER + (size_t)B * H * ((nb + 1) / 2));
 }
 
-extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16_t* v16,
-                                const float* q_scale, int q_group, const float* k_scale,
-                                const float* v_scale, const float* vm,
-                                const int32_t* pair_ptr, const uint32_t* sched, const int32_t* sched_cnt,
-                                int plan_slices,
-                                const int32_t* inv_idx, int n_text,
-                                void* out, int out_dtype,
-                                int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_n,
-                                float* lse, int B, int H, int N, int D, float sm_scale, int mode,
-                                int32_t* redo, size_t redo_bytes,
-                                int32_t* status, paro_stream_t stream) {
+int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t* v16, const float* q_scale, int q_group,
+                             const float* k_scale, const float* v_scale, const float* vm, const int32_t* pair_ptr,
+                             const uint32_t* sched, const int32_t* sched_cnt, int plan_slices, const int32_t* inv_idx,
+                             int n_text, void* out, int out_dtype, int64_t out_stride_b, int64_t out_stride_h,
+                             int64_t out_stride_n, float* lse, int B, int H, int N, int D, float sm_scale, int mode,
+                             int32_t* redo, size_t redo_bytes, int32_t* status, int32_t* host_status, cudaStream_t s) {
   PARO_REQUIRE(q8 && k8 && v16 && q_scale && k_scale && v_scale && pair_ptr && sched && sched_cnt && out && status, PARO_EINVAL,
                "paro_sparse_attn: null pointer");
   PARO_REQUIRE(B > 0 && H > 0 && N > 0, PARO_ESHAPE, "paro_sparse_attn: empty problem");
@@ -809,13 +804,12 @@ extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16
   AttnParams p;
   p.q8 = q8; p.q_scale = q_scale; p.k_scale = k_scale; p.v_scale = v_scale; p.vm = vm;
   p.pair_ptr = pair_ptr; p.sched = sched; p.sched_cnt = sched_cnt; p.inv_idx = inv_idx;
-  p.out = out; p.lse = lse; p.status = status; p.redo = redo;
+  p.out = out; p.lse = lse; p.status = status; p.host_status = host_status; p.redo = redo;
   p.osb = out_stride_b; p.osh = out_stride_h; p.osn = out_stride_n;
   p.plan_slices = plan_slices; p.q_group = q_group; p.n_text = n_text;
   p.B = B; p.H = H; p.N = N; p.nb = (N + 63) / 64; p.npairs = (p.nb + 1) / 2;
   p.from_list = 0;
   p.scale_log2 = sm_scale * 1.44269504f;
-  cudaStream_t s = (cudaStream_t)stream;
   const uint64_t ctas = (uint64_t)B * H * p.npairs;
   PARO_REQUIRE(ctas < (1ull << 31), PARO_ESHAPE, "paro_sparse_attn: too many work items");
   if (mode == PARO_ATTN_EXACT) return launch_attn_exact(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
@@ -825,6 +819,22 @@ extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16
   if (int rc = launch_attn_fixed(k8, v16, p, D, out_dtype, (unsigned)ctas, s)) return rc;
   p.from_list = 1;
   return launch_attn_exact(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
+}
+
+extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16_t* v16,
+                                const float* q_scale, int q_group, const float* k_scale,
+                                const float* v_scale, const float* vm,
+                                const int32_t* pair_ptr, const uint32_t* sched, const int32_t* sched_cnt,
+                                int plan_slices,
+                                const int32_t* inv_idx, int n_text,
+                                void* out, int out_dtype,
+                                int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_n,
+                                float* lse, int B, int H, int N, int D, float sm_scale, int mode,
+                                int32_t* redo, size_t redo_bytes,
+                                int32_t* status, paro_stream_t stream) {
+  return sparse_attn_launch(q8, k8, v16, q_scale, q_group, k_scale, v_scale, vm, pair_ptr, sched, sched_cnt, plan_slices,
+                            inv_idx, n_text, out, out_dtype, out_stride_b, out_stride_h, out_stride_n, lse, B, H, N, D,
+                            sm_scale, mode, redo, redo_bytes, status, nullptr, (cudaStream_t)stream);
 }
 
 

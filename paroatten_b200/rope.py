@@ -50,27 +50,35 @@ class QKNorm:
         return None
 
 
-def _norm_call_args(norm: Optional[QKNorm], xv: torch.Tensor):
-    """(mode, weight, bias, inv_rms, eps, keep-alive list) for an entry point that takes a norm;
-    xv is the [B,H,N,D] view of the activations.  For "rms" the per-token statistic is computed here."""
+def _norm_params(norm: Optional[QKNorm], H: int, D: int, like: torch.Tensor):
+    """(mode, weight, bias, eps) of a norm, the parameters cast to the activations' device and dtype."""
     if norm is None:
-        return _lib.NORM_NONE, None, None, None, 0.0, []
-    B, H, N, D = xv.shape
-    w = norm.weight.to(device=xv.device, dtype=xv.dtype).contiguous()
+        return _lib.NORM_NONE, None, None, 0.0
+    w = norm.weight.to(device=like.device, dtype=like.dtype).contiguous()
     if norm.kind == "layer":
         if w.numel() != D:
             raise ValueError("layer norm weight must have head_dim entries")
-        b = None if norm.bias is None else norm.bias.to(device=xv.device, dtype=xv.dtype).contiguous()
-        return _lib.NORM_LAYER_HEAD, w, b, None, float(norm.eps), [w, b]
+        b = None if norm.bias is None else norm.bias.to(device=like.device, dtype=like.dtype).contiguous()
+        return _lib.NORM_LAYER_HEAD, w, b, float(norm.eps)
     if norm.kind == "rms":
         if w.numel() != H * D:
             raise ValueError("rms norm weight must have heads*head_dim entries")
+        return _lib.NORM_RMS_ALL, w, None, float(norm.eps)
+    raise ValueError(f"unknown norm kind {norm.kind!r}")
+
+
+def _norm_call_args(norm: Optional[QKNorm], xv: torch.Tensor):
+    """(mode, weight, bias, inv_rms, eps, keep-alive list) for an entry point that takes a norm;
+    xv is the [B,H,N,D] view of the activations.  For "rms" the per-token statistic is computed here."""
+    B, H, N, D = xv.shape
+    mode, w, b, eps = _norm_params(norm, H, D, xv)
+    inv = None
+    if mode == _lib.NORM_RMS_ALL:
         inv = torch.empty(B, N, dtype=torch.float32, device=xv.device)
         _lib.check(_lib.lib().paro_row_inv_rms(
             xv.data_ptr(), _lib.dtype_code(xv.dtype), B, H, N, D, xv.stride(0), xv.stride(1), xv.stride(2),
-            float(norm.eps), inv.data_ptr(), _lib.stream_ptr()))
-        return _lib.NORM_RMS_ALL, w, None, inv, float(norm.eps), [w, inv]
-    raise ValueError(f"unknown norm kind {norm.kind!r}")
+            eps, inv.data_ptr(), _lib.stream_ptr()))
+    return mode, w, b, inv, eps, [w, b, inv]
 
 
 def axis_pairs(head_dim: int, family: str) -> Tuple[int, int, int]:

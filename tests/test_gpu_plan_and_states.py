@@ -304,3 +304,56 @@ def test_pairs_chosen_by_overlap(D, N, H, density, n_text):
         a, b = outs["adjacent", mode], outs["overlap", mode]
         assert po.cosine_per_head(b[0], a[0]).min().item() > 0.99999
         assert torch.allclose(b[1], a[1], atol=2e-3, rtol=0)
+
+
+def test_a_wait_that_runs_out_in_a_whole_layer_stops_the_next_call():
+    """The same malformed plan through paro_attention: the kernel itself leaves the status in pinned host memory (no copy
+    after the launch), so the next call raises, and the one after that is correct."""
+    H, grid, D = 2, (4, 16, 16), 128
+    N = grid[0] * grid[1] * grid[2]
+    q, k, v, orders = po.make_inputs(1, H, N, D, torch.bfloat16, seed=11)
+    mask = po.make_mask(H, N // 64, 0.5, seed=11)
+    plan = pb.compact_plan(mask.to(DEV))
+    cnt, ptr = plan.sched_cnt, plan.pair_ptr
+    r = int(((ptr[1:] - ptr[:-1]) - cnt[:, 0] > 0).nonzero()[0])
+    bad = cnt.clone()
+    bad[r, 0] += 1
+    args = (q.to(DEV), k.to(DEV), v.to(DEV), torch.tensor(orders))
+    pb.check_status()
+    pb.paro_attention(*args, _with(plan, sched_cnt=bad), grid_fhw=grid)
+    torch.cuda.synchronize()
+    with pytest.raises(_lib.ParoError, match="wait expired"):
+        pb.paro_attention(*args, plan, grid_fhw=grid)
+    got = pb.paro_attention(*args, plan, grid_fhw=grid)
+    pb.check_status()
+    assert_close(got, po.paro_attention(q, k, v, orders, mask, grid), "layer after the time-out")
+
+
+@pytest.mark.parametrize("layout,norm,smooth_k,n_text", [("HND", None, True, 0), ("NHD", "rms", True, 0),
+                                                         ("NHD", "layer", True, 77), ("HND", "layer", False, 5),
+                                                         ("HND", None, False, 0)])
+def test_one_layer_call_equals_its_passes(layout, norm, smooth_k, n_text):
+    """paro_attention (one C call on one work space) against the same passes called one by one, bit for bit."""
+    B, H, D, grid = 2, 3, 64, (3, 7, 9)
+    N = n_text + grid[0] * grid[1] * grid[2]
+    q, k, v, orders = po.make_inputs(B, H, N, D, torch.bfloat16, seed=5)
+    if layout == "NHD":
+        q, k, v = (t.transpose(1, 2).contiguous() for t in (q, k, v))
+    q, k, v = (t.to(DEV) for t in (q, k, v))
+    ids = torch.tensor(orders, dtype=torch.int32, device=DEV)
+    rope = pb.rope_tables(grid, D, "wan")
+    n = None
+    if norm == "layer":
+        n = pb.QKNorm("layer", torch.rand(D) + 0.5, torch.rand(D), 1e-6)
+    elif norm == "rms":
+        n = pb.QKNorm("rms", torch.rand(H * D) + 0.5, None, 1e-6)
+    plan = pb.compact_plan(po.make_mask(H, (N + 63) // 64, 0.5, seed=2).to(DEV), pairing="overlap")
+    got, lse = pb.paro_attention(q, k, v, ids, plan, grid_fhw=grid, n_text=n_text, rope=rope, tensor_layout=layout,
+                                 smooth_k=smooth_k, q_norm=n, k_norm=n, return_lse=True)
+    q8, qs, _ = pb.prep_qk_int8(q, ids, grid, n_text, rope, group=32, tensor_layout=layout, norm=n)
+    kp = pb.rope_permute(k, ids, grid, n_text, rope, tensor_layout=layout, norm=n)
+    _, _, k8, ks = pb.per_block_int8(kp, kp, pb.channel_mean(kp) if smooth_k else None, BLKQ=64, BLKK=64)
+    v16, vs, vm, _ = pb.prep_v_fp8(v, ids, grid, n_text, tensor_layout=layout)
+    want, wlse = pb.sparse_attn_quantized(q8, qs, k8, ks, v16, vs, vm, plan, D ** -0.5, inv_index=pb.perm_index(ids, grid),
+                                          n_text=n_text, return_lse=True, out_layout=layout)
+    assert torch.equal(got, want) and torch.equal(lse, wlse)
