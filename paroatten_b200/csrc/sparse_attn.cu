@@ -449,10 +449,15 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     float m_l = -INFINITY, l = 0.f, m_ref = 0.f;
     bool ok = true, redo = false;
     auto wait_bar = [&](uint32_t bar_saddr, int phase, int code, int i) {
-      const bool good = __all_sync(0xffffffffu, mbar_wait_bounded_at(bar_saddr, phase & 1, abort_flag, WAIT_LIMIT));
-      if (!good) report_timeout(p, abort_flag, code, i);
+      // (usually complete already: one poll and one vote, no divergent branch)
+      if (!__all_sync(0xffffffffu, mbar_poll(bar_saddr, phase & 1))) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded_at(bar_saddr, phase & 1, abort_flag, WAIT_LIMIT))) {
+          report_timeout(p, abort_flag, code, i);
+          return false;
+        }
+      }
       tc_fence_after();
-      return good;
+      return true;
     };
     uint64_t* const my_sfree = bar_sfree + 2 * half + set;
     uint64_t* const my_pready = bar_pready + 2 * half + set;
