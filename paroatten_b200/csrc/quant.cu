@@ -135,22 +135,39 @@ channel_stats_kernel(const T* __restrict__ x, int H, int N, int64_t sb, int64_t 
   }
 }
 
-// Pass 2: fold the chunk partials of one (b,h) in chunk order.
+// Pass 2: fold the chunk partials of one (b,h), in a fixed order.
 // mean = fp32(sum/N); amax = max(1e-7, max(|max-mean|, |min-mean|)) (equal to max|x-mean|, the
 // form of fused.cu:385-389); scale = amax/scale_max.
+// Latency: a thread that walks all chunks of its channel by itself needs 31 us for the 148 chunks of a 75600-token
+// head (5 heads, D = 128).  FIN_GROUPS threads share a channel, each with four loads in flight: 8 us; 15 -> 5 us for
+// 64 chunks.
+constexpr int FIN_GROUPS = 8;
 template <typename T>
-__global__ void channel_finalize_kernel(const ChannelPartial* __restrict__ part, int chunks, int D, int N,
+__global__ void __launch_bounds__(FIN_GROUPS * 128)
+channel_finalize_kernel(const ChannelPartial* __restrict__ part, int chunks, int D, int N,
                                         int smooth, float scale_max, T* __restrict__ mean_t,
                                         float* __restrict__ mean_f32, float* __restrict__ scale,
                                         float* __restrict__ inv_out, float* __restrict__ mean_used) {
-  const int bh = blockIdx.x, d = threadIdx.x;
+  __shared__ double s_sum[FIN_GROUPS * 128];
+  __shared__ float s_mx[FIN_GROUPS * 128], s_mn[FIN_GROUPS * 128];
+  const int bh = blockIdx.x, d = threadIdx.x % D, g = threadIdx.x / D;
   double s = 0.0;
   float a = -INFINITY, i = INFINITY;
-  for (int c = 0; c < chunks; ++c) {
+#pragma unroll 4
+  for (int c = g; c < chunks; c += FIN_GROUPS) {
     const ChannelPartial p = part[((size_t)bh * chunks + c) * D + d];
     s += p.sum;
     a = fmaxf(a, p.mx);
     i = fminf(i, p.mn);
+  }
+  s_sum[threadIdx.x] = s; s_mx[threadIdx.x] = a; s_mn[threadIdx.x] = i;
+  __syncthreads();
+  if (g) return;
+#pragma unroll
+  for (int k = 1; k < FIN_GROUPS; ++k) {
+    s += s_sum[k * D + d];
+    a = fmaxf(a, s_mx[k * D + d]);
+    i = fminf(i, s_mn[k * D + d]);
   }
   const float mean = smooth ? __double2float_rn(s / (double)N) : 0.0f;
   if (mean_t) mean_t[(size_t)bh * D + d] = F16Traits<T>::from_float(__double2float_rn(s / (double)N));
@@ -275,65 +292,95 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
 }
 
 // ---------------------------------------------------------------------------------------------
-// FP8 cast + transpose: CTA = 256 threads = one 64-token block of one (b,h).
-// Phase 1 stages the raw tile in shared memory with coalesced 16-byte loads; phase 2 lets
-// consecutive lanes take consecutive channels (conflict-free column reads) and each thread emit a
-// run of tokens of its channel as whole 32-byte sectors.
+// FP8 cast + transpose: CTA = 256 threads = one 64-token block of one (b,h).  HBM-bound: 2 bytes in and 2 (3
+// with the fp8 copy) bytes out per element.
+// Rows are quantised in the layout they are read in (16 bytes = 8 channels of a token), go to shared memory as
+// bf16 and come back transposed through ldmatrix.trans.  The eight rows of an 8x8 matrix are chosen so that the
+// four matrices of one ldmatrix leave a thread with EIGHT consecutive tokens of its channel: tokens
+// 8*(row/2) + 2*matrix + row%2 of a 32-token group.  A thread then stores 16 bytes and four lanes together
+// 64, whole sectors.  16-byte chunks are XOR-swizzled by (token & 1) | (token/8 & 3) * 2, which takes the
+// eight rows of every matrix to different banks.  2 x 12 x 32760 x 128: 126 -> 80 us, 2 x 48 x 17776 x 64: 121 us (read
+// column by column, two bytes at a time, and stored 16 bytes per channel: half sectors).
 template <typename T, int D, int GM>
 __global__ void __launch_bounds__(256)
 quant_v_fp8_kernel(const T* __restrict__ v, int H, int N, int npad, int64_t sb, int64_t sh, int64_t sn,
                    const float* __restrict__ inv_tab, const float* __restrict__ mean_tab,
                    uint8_t* __restrict__ v8, __nv_bfloat16* __restrict__ v16, const Gather gather) {
-  constexpr int TPR = D / 8;
+  constexpr int TPR = D / 8;                // 16-byte chunks (= threads) per row
   constexpr int ROWS = 256 / TPR;
-  constexpr int LD = D + 8;                 // padded row, keeps 16-byte alignment
-  constexpr int RUN = 64 / (256 / D);       // tokens per thread in phase 2 (32 for D=128, 16 for D=64)
-  __shared__ __align__(16) T tile[64 * LD];
+  constexpr int LOADS = 64 / ROWS;
+  __shared__ __align__(16) uint4 tile[64 * TPR];
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
   const int t0 = blockIdx.x * 64;
   const T* base = v + b * sb + h * sh;
+  auto slot = [](int token, int chunk) { return token * TPR + (chunk ^ ((token & 1) | ((token >> 3) & 3) << 1)); };
   {
     const GatherCtx<GM> gc(gather, h);
-    const int c8 = (threadIdx.x % TPR) * 8;
-#pragma unroll
-    for (int r = threadIdx.x / TPR; r < 64; r += ROWS) {
-      uint4 val = make_uint4(0, 0, 0, 0);
+    const int c = threadIdx.x % TPR, r0 = threadIdx.x / TPR;
+    constexpr int RPW = 32 / TPR;           // rows a warp covers with one load
+    const int lane = threadIdx.x & 31;
+    Pack8<T> row[LOADS];
+    // each of the warp's eight rows is decoded once, by lane (load, row of the load), and handed to its threads
+    int d_src = 0;
+    if constexpr (GM != GM_PLAIN) {
       int gf, gy, gx;
-      if (t0 + r < N) val = *reinterpret_cast<const uint4*>(base + (size_t)gc.source(t0 + r, gf, gy, gx) * sn + c8);
-      *reinterpret_cast<uint4*>(&tile[r * LD + c8]) = val;
+      const int t = t0 + (threadIdx.x >> 5) * RPW + lane % RPW + (lane / RPW) % LOADS * ROWS;
+      if (t < N) d_src = gc.source(t, gf, gy, gx);
+    }
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+      const int tok = t0 + r0 + i * ROWS;
+      int src = tok;
+      if constexpr (GM != GM_PLAIN) src = __shfl_sync(0xffffffffu, d_src, i * RPW + lane / TPR);
+      row[i].v = make_uint4(0, 0, 0, 0);
+      if (tok < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn + c * 8);
+    }
+    float mean[8], inv[8];                  // inv = scale_max / amax, from the finalize pass
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(mean + j) = *reinterpret_cast<const float4*>(mean_tab + (size_t)bh * D + c * 8 + j);
+      *reinterpret_cast<float4*>(inv + j) = *reinterpret_cast<const float4*>(inv_tab + (size_t)bh * D + c * 8 + j);
+    }
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+      const int r = r0 + i * ROWS;
+      uint32_t w[4] = {0u, 0u, 0u, 0u};     // tokens past the end are zero
+      if (t0 + r < N) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float y0 = __fmul_rn(__fsub_rn(F16Traits<T>::to_float(row[i].e[2 * j]), mean[2 * j]), inv[2 * j]);
+          const float y1 = __fmul_rn(__fsub_rn(F16Traits<T>::to_float(row[i].e[2 * j + 1]), mean[2 * j + 1]), inv[2 * j + 1]);
+          const __nv_fp8x2_storage_t p = __nv_cvt_float2_to_fp8x2(make_float2(y0, y1), __NV_SATFINITE, __NV_E4M3);
+          // e4m3 -> fp16 -> bf16: both steps exact (3 mantissa bits, exponents inside either range)
+          const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(p, __NV_E4M3);
+          const __nv_bfloat162 b2 = __floats2bfloat162_rn(__half2float(__half(__half_raw{h2.x})), __half2float(__half(__half_raw{h2.y})));
+          w[j] = *reinterpret_cast<const uint32_t*>(&b2);
+        }
+      }
+      tile[slot(r, c)] = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
   __syncthreads();
-  const int d = threadIdx.x % D, run = threadIdx.x / D;
-  const float mean = mean_tab[(size_t)bh * D + d];
-  const float inv = inv_tab[(size_t)bh * D + d];  // scale_max / amax, from the finalize pass
-  uint32_t w8[RUN / 4];
-  uint32_t w16[RUN / 2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int i = 0; i < RUN; i += 2) {
-    float y[2];
+  for (int u = warp; u < 2 * TPR; u += 8) {   // unit = 8 channels x 32 tokens
+    const int chunk = u >> 1, tg = (u & 1) * 32;
+    const int tok = tg + 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);   // the row this lane points ldmatrix at
+    const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(tile + slot(tok, chunk)));
+    uint32_t w[4];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+    const int d = chunk * 8 + (lane >> 2), first = t0 + tg + (lane & 3) * 8;
+    const size_t o = ((size_t)bh * D + d) * npad + first;
+    if (v16) *reinterpret_cast<uint4*>(v16 + o) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (v8) {   // the bf16 values are e4m3 values: the conversion back is exact
+      uint32_t q[4];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int r = run * RUN + i + k;
-      float f = 0.f;
-      if (t0 + r < N) f = __fmul_rn(__fsub_rn(F16Traits<T>::to_float(tile[r * LD + d]), mean), inv);
-      y[k] = f;
+      for (int j = 0; j < 4; ++j)
+        q[j] = __nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u)),
+                                        __NV_SATFINITE, __NV_E4M3);
+      *reinterpret_cast<uint2*>(v8 + o) = make_uint2(q[0] | q[1] << 16, q[2] | q[3] << 16);
     }
-    const __nv_fp8x2_storage_t p = __nv_cvt_float2_to_fp8x2(make_float2(y[0], y[1]), __NV_SATFINITE, __NV_E4M3);
-    if ((i & 3) == 0) w8[i / 4] = (uint32_t)p; else w8[i / 4] |= (uint32_t)p << 16;
-    // e4m3 -> fp16 -> bf16: both steps exact (3 mantissa bits, exponents inside either range)
-    const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(p, __NV_E4M3);
-    const __nv_bfloat162 b2 = __floats2bfloat162_rn(__half2float(__half(__half_raw{h2.x})), __half2float(__half(__half_raw{h2.y})));
-    w16[i / 2] = *reinterpret_cast<const uint32_t*>(&b2);
-  }
-  const size_t o = ((size_t)bh * D + d) * npad + t0 + run * RUN;
-#pragma unroll
-  for (int i = 0; i < RUN / 16; ++i)
-    if (v8) *reinterpret_cast<uint4*>(v8 + o + i * 16) = make_uint4(w8[4 * i], w8[4 * i + 1], w8[4 * i + 2], w8[4 * i + 3]);
-  if (v16) {
-#pragma unroll
-    for (int i = 0; i < RUN / 8; ++i)
-      *reinterpret_cast<uint4*>(v16 + o + i * 8) = make_uint4(w16[4 * i], w16[4 * i + 1], w16[4 * i + 2], w16[4 * i + 3]);
   }
 }
 
@@ -384,11 +431,11 @@ extern "C" int paro_channel_mean(const void* x, int dtype, int B, int H, int N, 
   ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
   if (dtype == PARO_F16) {
     launch_stats<__half>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__half><<<B * H, D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (__half*)mean_out,
+    channel_finalize_kernel<__half><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (__half*)mean_out,
                                                         mean_f32, nullptr, nullptr, nullptr);
   } else {
     launch_stats<__nv_bfloat16>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__nv_bfloat16><<<B * H, D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f,
+    channel_finalize_kernel<__nv_bfloat16><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f,
                                                                (__nv_bfloat16*)mean_out, mean_f32, nullptr, nullptr,
                                                                nullptr);
   }
@@ -453,7 +500,7 @@ int run_v_fp8(const void* v, int B, int H, int N, int D, int64_t sb, int64_t sh,
   float* inv_tab = reinterpret_cast<float*>(part + bh * chunks * D);
   float* mean_tab = inv_tab + bh * D;
   launch_stats<T>(v, B, H, N, D, sb, sh, sn, part, s);   // statistics do not depend on the token order
-  channel_finalize_kernel<T><<<B * H, D, 0, s>>>(part, chunks, D, N, smooth, scale_max, (T*)nullptr,
+  channel_finalize_kernel<T><<<B * H, FIN_GROUPS * D, 0, s>>>(part, chunks, D, N, smooth, scale_max, (T*)nullptr,
                                                  smooth ? vm : nullptr, v_scale, inv_tab, mean_tab);
   const int npad = (N + 63) / 64 * 64;
   dim3 grid(npad / 64, B * H);
@@ -546,11 +593,11 @@ extern "C" int paro_channel_mean_noalloc(const void* x, int dtype, int B, int H,
   // left behind by an earlier call has to be cleared
   if (dtype == PARO_F16) {
     launch_stats<__half>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__half><<<B * H, D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (__half*)mean_out,
+    channel_finalize_kernel<__half><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (__half*)mean_out,
                                                         mean_f32, nullptr, nullptr, nullptr);
   } else {
     launch_stats<__nv_bfloat16>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__nv_bfloat16><<<B * H, D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f,
+    channel_finalize_kernel<__nv_bfloat16><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f,
                                                                (__nv_bfloat16*)mean_out, mean_f32, nullptr, nullptr,
                                                                nullptr);
   }
@@ -592,7 +639,7 @@ int run_prep_int8(const void* x, int B, int H, int N, int D, int64_t sb, int64_t
     gs.order_ids = nullptr;
     ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
     launch_stats<T>(x, B, H, N, D, sb, sh, sn, part, s, gs);
-    channel_finalize_kernel<T><<<B * H, D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (T*)km_out, nullptr, nullptr,
+    channel_finalize_kernel<T><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (T*)km_out, nullptr, nullptr,
                                                    nullptr, nullptr);
     km = static_cast<const T*>(km_out);
     launches = 3;
