@@ -36,7 +36,7 @@ enum {
 };
 
 enum { PARO_F16 = 0, PARO_BF16 = 1 };
-enum { PARO_ROPE_NONE = 0, PARO_ROPE_REAL_F32 = 1, PARO_ROPE_COMPLEX_F64 = 2 };
+enum { PARO_ROPE_NONE = 0, PARO_ROPE_REAL_F32 = 1, PARO_ROPE_COMPLEX_F64 = 2, PARO_ROPE_COMPLEX_F64_APPROX = 3 };
 enum { PARO_NORM_NONE = 0, PARO_NORM_LAYER_HEAD = 1, PARO_NORM_RMS_ALL = 2 };
 enum { PARO_ATTN_FAST = 0, PARO_ATTN_EXACT = 1 };
 
@@ -63,6 +63,8 @@ int paro_build_perm_index(const int32_t* order_ids, int H, int F, int Hh, int W,
  * pairs_f/pairs_h: how many leading channel pairs follow the f / h coordinate (rest: w).
  * sin_tab == NULL (all entry points that take the two tables): cos_tab is then ONE table
  * [F+Hh+W, D/2, 2] with cos and sin of a pair side by side, fetched by a single load.
+ * PARO_ROPE_COMPLEX_F64_APPROX: the same results as PARO_ROPE_COMPLEX_F64, faster; cos_tab is the interleaved fp64 table
+ * and sin_tab (16-byte aligned) the same table rounded to fp32.
  * Replaces csrc/rope/rope.cu:14-48 (rope_permutation) and permute_qk / permute_attn_out
  * (cogvideox.py:22-110). */
 int paro_rope_permute(const void* in, void* out, int dtype, int B, int H, int N, int D,

@@ -20,7 +20,7 @@ NVCC_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17",
 
 PARO_OK, PARO_EINVAL, PARO_ESHAPE, PARO_EALIGN, PARO_ETIMEOUT, PARO_ECUDA, PARO_ECAP = 0, -1, -2, -3, -4, -5, -6
 F16, BF16 = 0, 1
-ROPE_NONE, ROPE_REAL_F32, ROPE_COMPLEX_F64 = 0, 1, 2
+ROPE_NONE, ROPE_REAL_F32, ROPE_COMPLEX_F64, ROPE_COMPLEX_F64_APPROX = 0, 1, 2, 3
 NORM_NONE, NORM_LAYER_HEAD, NORM_RMS_ALL = 0, 1, 2
 ATTN_FAST, ATTN_EXACT = 0, 1
 

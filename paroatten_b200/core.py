@@ -11,7 +11,7 @@ import torch.nn.functional as F
 from . import _lib
 from .plan import (CompactPlan, PermutePlan, PlanStore, SparsePlan, apply_empty_heads, compact_plan, perm_index)
 from .quant import _hnd, channel_mean, per_channel_fp8, per_warp_int8, per_block_int8
-from .rope import RopeTables, _norm_params
+from .rope import RopeTables, _norm_params, _rope_args
 
 _status = {}
 _status_mirror = {}   # device index -> pinned host copy of the status words, refreshed after every launch
@@ -193,13 +193,12 @@ def _layer(q, k, v, orders, index, plan: CompactPlan, grid, n_text: int, rope: O
         for e in ev:
             e.record()       # (creates the event; the call below records both again where they belong)
     cnt = plan.sched_cnt_kernel if plan.sched_cnt_kernel is not None else plan.sched_cnt
+    rope_mode, cos, sin, pairs_f, pairs_h = _rope_args(rope)
     three = ctypes.c_int64 * 3
     a = _lib.LayerArgs(
         qv.data_ptr(), kv.data_ptr(), vv.data_ptr(), three(*qv.stride()[:3]), three(*kv.stride()[:3]),
         three(*vv.stride()[:3]), _lib.dtype_code(q.dtype), B, H, N, D, n_text, *grid, orders.data_ptr(),
-        None if rope is None else _lib.ptr(rope.cos), None if rope is None else _lib.ptr(rope.sin),
-        _lib.ROPE_NONE if rope is None else rope.mode, 0 if rope is None else rope.pairs_f,
-        0 if rope is None else rope.pairs_h, qn, kn, qeps, keps, _lib.ptr(qw), _lib.ptr(qb), _lib.ptr(kw), _lib.ptr(kb),
+        cos, sin, rope_mode, pairs_f, pairs_h, qn, kn, qeps, keps, _lib.ptr(qw), _lib.ptr(qb), _lib.ptr(kw), _lib.ptr(kb),
         bool(smooth_k), bool(smooth_v), plan.pair_ptr.data_ptr(), plan.sched.data_ptr(), cnt.data_ptr(), plan.slices,
         _lib.ATTN_FAST if mode == "fast" else _lib.ATTN_EXACT, index.data_ptr(), out.data_ptr(), three(*ov.stride()[:3]),
         _lib.ptr(lse), sm_scale, _lib.ptr(redo), redo.numel() * 4 if redo is not None else 0,

@@ -54,6 +54,11 @@ template <> struct F16Traits<__nv_bfloat16> {
   static __device__ __forceinline__ __nv_bfloat16 from_float(float v) { return __float2bfloat16_rn(v); }
 };
 
+// Passes of a layer over V and over K's rotated copy (quant.cu), issued by paro_layer.
+size_t layer_kv_scratch_bytes(int B, int H, int N, int D);
+int layer_kv_passes(const paro_layer_args& a, const void* kp, void* km, int8_t* k8, float* ks, uint16_t* v16, float* vs,
+                    float* vm, void* scratch, int32_t* zero_word, cudaStream_t s);
+
 // Eight 16-bit values moved as one 16-byte vector.
 template <typename T> union Pack8 {
   uint4 v;

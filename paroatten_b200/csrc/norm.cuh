@@ -34,7 +34,8 @@ __device__ __forceinline__ void normalize8(Pack8<T>& x, int c8, int D, int b, in
     }
 #pragma unroll
     for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const float mean = __double2float_rn(s / (double)D);
+    const double inv_d = 1.0 / (8 * TPR);   // (a power of two: the product is the quotient)
+    const float mean = __double2float_rn(s * inv_d);
     double q = 0.0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -43,7 +44,7 @@ __device__ __forceinline__ void normalize8(Pack8<T>& x, int c8, int D, int b, in
     }
 #pragma unroll
     for (int o = TPR / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    const float var = __double2float_rn(q / (double)D);
+    const float var = __double2float_rn(q * inv_d);
     const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, a.eps)));
     Pack8<T> w, bb;
     w.v = *reinterpret_cast<const uint4*>(static_cast<const T*>(a.weight) + c8);

@@ -40,20 +40,22 @@ struct GatherCtx {
   PermDecoder dec;
   __device__ GatherCtx(const Gather& g_, int h)
       : g(g_), dec(GM != GM_PLAIN && g_.order_ids ? g_.order_ids[h] : 0, g_.F, g_.Hh, g_.W) {}
-  // source token of row `tok`; f < 0 for rows that are not rotated (text tokens, or no gather)
-  __device__ __forceinline__ int source(int tok, int& f, int& y, int& x) const {
-    f = y = x = -1;
+  // source token of row `tok`
+  __device__ __forceinline__ int source(int tok) const {
+    int f, y, x;
     if constexpr (GM == GM_PLAIN) return tok;
     if (tok < g.n_text) return tok;
-    const int src = g.n_text + dec.source(tok - g.n_text, f, y, x);
-    return src;
+    return g.n_text + dec.source(tok - g.n_text, f, y, x);
   }
-  template <typename T> __device__ __forceinline__ void rotate(Pack8<T>& v, int c8, int D, int f, int y, int x) const {
-    if constexpr (GM == GM_ROPE_F32) {
-      if (f >= 0) rotate8<T, PARO_ROPE_REAL_F32>(v, c8, D, f, y, x, g.F, g.Hh, g.rope);
-    } else if constexpr (GM == GM_ROPE_F64) {
-      if (f >= 0) rotate8<T, PARO_ROPE_COMPLEX_F64>(v, c8, D, f, y, x, g.F, g.Hh, g.rope);
-    }
+  // Entry r of the table: row tok0 + r of the sequence (rows past the end: not rotated).
+  template <int ROWS> __device__ __forceinline__ void fill(RowTable<ROWS>& t, int rows, int tok0, int N, int D) const {
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) fill_row(t, r, tok0 + r, N, D >> 2, dec, g.n_text, g.F, g.Hh);
+  }
+  // rows r, r + step, ... of the table
+  template <int NR, typename T, int ROWS>
+  __device__ __forceinline__ void rotate(Pack8<T>* v, const PairAxes& pa, const RowTable<ROWS>& rows, int r, int step) const {
+    if constexpr (GM == GM_ROPE_F32) rotate8<NR, T, PARO_ROPE_REAL_F32>(v, pa, rows, r, step, g.rope);
+    else if constexpr (GM == GM_ROPE_F64) rotate8<NR, T, PARO_ROPE_COMPLEX_F64>(v, pa, rows, r, step, g.rope);
   }
 };
 
@@ -75,23 +77,38 @@ struct ChannelPartial {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Pass 1 of the per-channel reductions: per (b,h, chunk of tokens) the fp64 sum, max and min of
+// Pass 1 of the per-channel reductions: per (b,h, chunk of tokens) the fp64 sum and (EXTREMES) max and min of
 // every channel.  Thread = one 8-channel slice of a token row; rows of the chunk are walked in a
 // fixed order and the cross-thread reduction is sequential, so results do not depend on timing.
-template <typename T, int D, int GM>
-__global__ void __launch_bounds__(256)
-channel_stats_kernel(const T* __restrict__ x, int H, int N, int64_t sb, int64_t sh, int64_t sn,
-                     ChannelPartial* __restrict__ part, int chunks, const Gather gather) {
+// blockIdx.z: which of (up to) two tensors of the same shape -- K and V of a layer are reduced by one launch.
+struct StatsSrc {
+  const void* x;
+  int64_t sb, sh, sn;
+  ChannelPartial* part;
+};
+template <typename T, int D, int GM, bool EXTREMES>
+__global__ void __launch_bounds__(256, GM >= GM_ROPE_F32 ? 2 : 3)
+channel_stats_kernel(const StatsSrc src0, const StatsSrc src1, int H, int N, int chunks, const Gather gather) {
+  const bool second = blockIdx.z != 0;
+  const T* x = static_cast<const T*>(second ? src1.x : src0.x);
+  ChannelPartial* part = second ? src1.part : src0.part;
+  const int64_t sb = second ? src1.sb : src0.sb, sh = second ? src1.sh : src0.sh, sn = second ? src1.sn : src0.sn;
   constexpr int TPR = D / 8;
   constexpr int ROWS = 256 / TPR;
   __shared__ double s_sum[ROWS][D + 1];
-  __shared__ float s_mx[ROWS][D + 1];
-  __shared__ float s_mn[ROWS][D + 1];
+  __shared__ float s_mx[EXTREMES ? ROWS : 1][D + 1];
+  __shared__ float s_mn[EXTREMES ? ROWS : 1][D + 1];
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
   const int c8 = (threadIdx.x % TPR) * 8, r = threadIdx.x / TPR;
   const int t0 = blockIdx.x * STATS_CHUNK, t1 = min(N, t0 + STATS_CHUNK);
   const T* base = x + b * sb + h * sh;
   const GatherCtx<GM> gc(gather, h);
+  const PairAxes pa(c8, gather.rope);
+  __shared__ RowTable<GM == GM_PLAIN ? 1 : STATS_CHUNK> rows;
+  if constexpr (GM != GM_PLAIN) {
+    gc.fill(rows, STATS_CHUNK, t0, N, D);
+    __syncthreads();
+  }
   double sum[8];
   float mx[8], mn[8];
 #pragma unroll
@@ -99,36 +116,45 @@ channel_stats_kernel(const T* __restrict__ x, int H, int N, int64_t sb, int64_t 
   // four rows are in flight per thread; they are accumulated in the order of a plain loop
   for (int t = t0 + r; t < t1; t += 4 * ROWS) {
     Pack8<T> v[4];
-    int gf[4], gy[4], gx[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int tu = t + u * ROWS;
-      gf[u] = gy[u] = gx[u] = -1;
-      if (tu < t1) v[u].v = *reinterpret_cast<const uint4*>(base + (size_t)gc.source(tu, gf[u], gy[u], gx[u]) * sn + c8);
+      if (tu < t1) v[u].v = *reinterpret_cast<const uint4*>(base + (size_t)(GM == GM_PLAIN ? tu : rows.src[tu - t0]) * sn + c8);
+    }
+    if constexpr (GM == GM_ROPE_F32 || GM == GM_ROPE_F64) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t + u * ROWS < t1) gc.template rotate<1>(v + u, pa, rows, t + u * ROWS - t0, 0);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (t + u * ROWS >= t1) break;
-      gc.rotate(v[u], c8, D, gf[u], gy[u], gx[u]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float f = F16Traits<T>::to_float(v[u].e[j]);
         sum[j] += (double)f;
-        mx[j] = fmaxf(mx[j], f);
-        mn[j] = fminf(mn[j], f);
+        if (EXTREMES) {
+          mx[j] = fmaxf(mx[j], f);
+          mn[j] = fminf(mn[j], f);
+        }
       }
     }
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) { s_sum[r][c8 + j] = sum[j]; s_mx[r][c8 + j] = mx[j]; s_mn[r][c8 + j] = mn[j]; }
+  for (int j = 0; j < 8; ++j) {
+    s_sum[r][c8 + j] = sum[j];
+    if (EXTREMES) { s_mx[r][c8 + j] = mx[j]; s_mn[r][c8 + j] = mn[j]; }
+  }
   __syncthreads();
   if (threadIdx.x < D) {
     double s = 0.0;
     float a = -INFINITY, i = INFINITY;
     for (int k = 0; k < ROWS; ++k) {
       s += s_sum[k][threadIdx.x];
-      a = fmaxf(a, s_mx[k][threadIdx.x]);
-      i = fminf(i, s_mn[k][threadIdx.x]);
+      if (EXTREMES) {
+        a = fmaxf(a, s_mx[k][threadIdx.x]);
+        i = fminf(i, s_mn[k][threadIdx.x]);
+      }
     }
     ChannelPartial p{s, a, i};
     part[((size_t)bh * chunks + blockIdx.x) * D + threadIdx.x] = p;
@@ -139,15 +165,23 @@ channel_stats_kernel(const T* __restrict__ x, int H, int N, int64_t sb, int64_t 
 // mean = fp32(sum/N); amax = max(1e-7, max(|max-mean|, |min-mean|)) (equal to max|x-mean|, the
 // form of fused.cu:385-389); scale = amax/scale_max.
 // Latency: a thread that walks all chunks of its channel by itself needs 31 us for the 148 chunks of a 75600-token
-// head (5 heads, D = 128).  FIN_GROUPS threads share a channel, each with four loads in flight: 8 us; 15 -> 5 us for
-// 64 chunks.
+// head.  FIN_GROUPS threads share a channel, each with four loads in flight.
 constexpr int FIN_GROUPS = 8;
+template <typename T> struct FinalizeDst {
+  const ChannelPartial* part;
+  int smooth;
+  float scale_max;
+  T* mean_t;
+  float *mean_f32, *scale, *inv_out, *mean_used;
+};
+// blockIdx.y: which of (up to) two tensors; zero_word (nullable): a word of device memory to clear on the way (the
+// attention call's redo counter, which otherwise takes a memset of its own).
 template <typename T>
 __global__ void __launch_bounds__(FIN_GROUPS * 128)
-channel_finalize_kernel(const ChannelPartial* __restrict__ part, int chunks, int D, int N,
-                                        int smooth, float scale_max, T* __restrict__ mean_t,
-                                        float* __restrict__ mean_f32, float* __restrict__ scale,
-                                        float* __restrict__ inv_out, float* __restrict__ mean_used) {
+channel_finalize_kernel(const FinalizeDst<T> dst0, const FinalizeDst<T> dst1, int chunks, int D, int N, int32_t* zero_word) {
+  const FinalizeDst<T>& dst = blockIdx.y ? dst1 : dst0;
+  const ChannelPartial* __restrict__ part = dst.part;
+  if (zero_word && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *zero_word = 0;
   __shared__ double s_sum[FIN_GROUPS * 128];
   __shared__ float s_mx[FIN_GROUPS * 128], s_mn[FIN_GROUPS * 128];
   const int bh = blockIdx.x, d = threadIdx.x % D, g = threadIdx.x / D;
@@ -169,34 +203,66 @@ channel_finalize_kernel(const ChannelPartial* __restrict__ part, int chunks, int
     a = fmaxf(a, s_mx[k * D + d]);
     i = fminf(i, s_mn[k * D + d]);
   }
-  const float mean = smooth ? __double2float_rn(s / (double)N) : 0.0f;
-  if (mean_t) mean_t[(size_t)bh * D + d] = F16Traits<T>::from_float(__double2float_rn(s / (double)N));
-  if (mean_f32) mean_f32[(size_t)bh * D + d] = __double2float_rn(s / (double)N);
-  if (scale) {
+  const size_t o = (size_t)bh * D + d;
+  const float mean = dst.smooth ? __double2float_rn(s / (double)N) : 0.0f;
+  if (dst.mean_t) dst.mean_t[o] = F16Traits<T>::from_float(__double2float_rn(s / (double)N));
+  if (dst.mean_f32) dst.mean_f32[o] = __double2float_rn(s / (double)N);
+  if (dst.scale) {
     const float amax = fmaxf(1e-7f, fmaxf(fabsf(__fsub_rn(a, mean)), fabsf(__fsub_rn(i, mean))));
-    scale[(size_t)bh * D + d] = __fdiv_rn(amax, scale_max);
-    inv_out[(size_t)bh * D + d] = __fdiv_rn(scale_max, amax);
-    mean_used[(size_t)bh * D + d] = mean;
+    dst.scale[o] = __fdiv_rn(amax, dst.scale_max);
+    dst.inv_out[o] = __fdiv_rn(dst.scale_max, amax);
+    dst.mean_used[o] = mean;
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-// INT8: CTA = 128 threads = one 64-token block; warp w owns tokens 16w..16w+15.
+// INT8: one CTA = `blocks` consecutive 64-token blocks of one (b,h); warp w owns 64/WARPS tokens of each.
+// 2 bytes in, 1 byte out per element.
+// Passes that rotate (INT8_TABLE): 256 threads; source tokens and table rows of all the CTA's blocks are worked out once
+// into shared memory.  Four blocks per CTA against one: 190 -> 140 us for 2 x 48 x 17776 x 64 with the fp32 rotation,
+// 257 -> 204 us for 2 x 12 x 32760 x 128 with RMS norm and the fp64 rotation.  (Loading the next block's rows ahead
+// costs the registers of a third CTA per SM: 148, 239 us.)
+// Passes that do not: 128 threads with twice the rows in flight each, one block per CTA, source tokens by shuffle (the
+// form above takes 90 us instead of 72 for 2 x 48 x 17776 x 64 in plain order, 29 instead of 22 for 40 x 4680 x 128
+// reordered).
+constexpr int INT8_BLOCKS = 4;               // most blocks per CTA
+template <int GM> struct Int8Cfg {
+  static constexpr bool TABLE = GM == GM_ROPE_F32 || GM == GM_ROPE_F64;
+  static constexpr int WARPS = TABLE ? 8 : 4;
+};
 template <typename T, int D, int GROUP, int GM, int NM>
-__global__ void __launch_bounds__(128, GM == GM_ROPE_F64 ? 4 : (GM == GM_ROPE_F32 || NM != PARO_NORM_NONE ? 5 : 6))
+__global__ void __launch_bounds__(32 * Int8Cfg<GM>::WARPS, !Int8Cfg<GM>::TABLE ? (NM != PARO_NORM_NONE ? 5 : 6)
+                                                           : (GM == GM_ROPE_F64 || NM != PARO_NORM_NONE ? 3 : 4))
 quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __restrict__ out,
                   float* __restrict__ scale, int H, int N, int64_t sb, int64_t sh, int64_t sn,
-                  float fold, int n_scale_per_bh, const Gather gather, const NormArgs norm) {
+                  float fold, int n_scale_per_bh, int blocks, const Gather gather, const NormArgs norm) {
+  constexpr bool TABLE = Int8Cfg<GM>::TABLE;
+  constexpr int WARPS = Int8Cfg<GM>::WARPS, ROWS = 64 / WARPS;   // ROWS: tokens per warp and block
   constexpr int TPR = D / 8;          // threads per token row
   constexpr int RPL = 32 / TPR;       // rows covered by one warp-wide load
-  constexpr int LOADS = 16 / RPL;     // loads per thread
-  __shared__ float s_amax[4];
+  constexpr int LOADS = ROWS / RPL;   // loads per thread and block
+  __shared__ float s_amax[2][WARPS];
+  __shared__ RowTable<TABLE ? 64 * INT8_BLOCKS : 1> rows;
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c8 = (lane % TPR) * 8;
-  const int tok0 = blockIdx.x * 64 + warp * 16 + lane / TPR;
-  const T* base = x + b * sb + h * sh;
+  const int first = blockIdx.x * (TABLE ? blocks : 1) * 64, r0 = warp * ROWS + lane / TPR;
+  const int n_blocks = TABLE ? min(blocks, (N - first + 63) / 64) : 1;
+  const T* base = x + b * sb + h * sh + c8;
   const GatherCtx<GM> gc(gather, h);
+  [[maybe_unused]] const PairAxes pa(c8, gather.rope);
+  if constexpr (TABLE) {
+    gc.fill(rows, 64 * n_blocks, first, N, D);
+    __syncthreads();
+  }
+  // source token of the thread's row of load i in block blk (all lanes: a shuffle in the reordering form, where lane l
+  // holds the source of the warp's row l % ROWS in d_src)
+  int d_src = 0;
+  auto source = [&](int blk, int i) {
+    if constexpr (TABLE) return rows.src[blk * 64 + r0 + i * RPL];
+    else if constexpr (GM == GM_REORDER) return __shfl_sync(0xffffffffu, d_src, i * RPL + lane / TPR);
+    else return first + blk * 64 + r0 + i * RPL;
+  };
 
   float mean[8];
 #pragma unroll
@@ -207,86 +273,77 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
 #pragma unroll
     for (int j = 0; j < 8; ++j) mean[j] = F16Traits<T>::to_float(m.e[j]);
   }
-
   // the (rotated) rows stay packed in registers; they are widened once for the maximum and once more
   // for the rounding, which costs a shift per element and halves the registers held across the barrier
-  Pack8<T> row[LOADS];
-  float amax = 0.f;
   auto widen = [&](const Pack8<T>& p, int j) {
     float f = F16Traits<T>::to_float(p.e[j]);
     if (km) f = __fsub_rn(f, mean[j]);
     if (fold != 0.f) f = __fmul_rn(f, fold);
     return f;
   };
-  // Each of the warp's 16 tokens is decoded once (source token and grid position) by lane t and
-  // lane t+16, and handed to the threads that load it.
-  int d_src = 0, d_f = -1, d_y = -1, d_x = -1;
-  if constexpr (GM != GM_PLAIN) {
-    const int t = blockIdx.x * 64 + warp * 16 + (lane & 15);
-    if (t < N) d_src = gc.source(t, d_f, d_y, d_x);
-  }
-#pragma unroll
-  for (int i = 0; i < LOADS; ++i) {   // all loads first, so that every row of the thread is in flight at once
-    const int tok = tok0 + i * RPL;
-    row[i].v = make_uint4(0, 0, 0, 0);
-    int src = tok;
-    if constexpr (GM != GM_PLAIN) src = __shfl_sync(0xffffffffu, d_src, i * RPL + lane / TPR);
-    if (tok < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn + c8);
-  }
-#pragma unroll
-  for (int i = 0; i < LOADS; ++i) {
-    const int tok = tok0 + i * RPL;
-    if constexpr (NM != PARO_NORM_NONE) {   // all lanes: the row statistics are reduced with full-warp shuffles
-      int src = tok < N ? tok : 0;
-      if constexpr (GM != GM_PLAIN) src = __shfl_sync(0xffffffffu, d_src, i * RPL + lane / TPR);
-      normalize8<T, NM, TPR>(row[i], c8, D, b, h, N, src, norm);
+#pragma unroll 1
+  for (int blk = 0; blk < n_blocks; ++blk) {
+    Pack8<T> row[LOADS];
+    if constexpr (GM == GM_REORDER) {
+      const int t = first + blk * 64 + warp * ROWS + lane % ROWS;
+      if (t < N) d_src = gc.source(t);
     }
-    if constexpr (GM == GM_ROPE_F32 || GM == GM_ROPE_F64) {
-      const int from = i * RPL + lane / TPR;
-      const int gf = __shfl_sync(0xffffffffu, d_f, from);
-      const int gy = __shfl_sync(0xffffffffu, d_y, from);
-      const int gx = __shfl_sync(0xffffffffu, d_x, from);
-      if (tok < N) gc.rotate(row[i], c8, D, gf, gy, gx);
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {   // all loads first, so that every row of the thread is in flight at once
+      const int src = source(blk, i);
+      row[i].v = make_uint4(0, 0, 0, 0);
+      if (first + blk * 64 + r0 + i * RPL < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn);
     }
-    if (tok < N) {
+    float amax = 0.f;
+    if constexpr (NM != PARO_NORM_NONE) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(widen(row[i], j)));
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if (lane == 0) s_amax[warp] = amax;
-  __syncthreads();
-  if (GROUP == 64) {
-    amax = fmaxf(fmaxf(s_amax[0], s_amax[1]), fmaxf(s_amax[2], s_amax[3]));
-  } else {
-    amax = fmaxf(s_amax[warp & ~1], s_amax[warp | 1]);
-  }
-  amax = fmaxf(amax, 1e-7f);
-  if (GROUP == 64) {
-    if (threadIdx.x == 0) scale[(size_t)bh * n_scale_per_bh + blockIdx.x] = __fdiv_rn(amax, 127.0f);
-  } else {
-    if (lane == 0 && (warp & 1) == 0)
-      scale[(size_t)bh * n_scale_per_bh + blockIdx.x * 2 + (warp >> 1)] = __fdiv_rn(amax, 127.0f);
-  }
-  const float inv = __fdiv_rn(127.0f, amax);
-#pragma unroll
-  for (int i = 0; i < LOADS; ++i) {
-    const int tok = tok0 + i * RPL;
-    if (tok < N) {
-      // round to nearest even (NaN -> 0), then saturate and pack two values per instruction
-      int qi[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) qi[j] = __float2int_rn(__fmul_rn(widen(row[i], j), inv));
-      uint32_t w[2];
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t hi16, word;
-        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(hi16) : "r"(qi[half * 4 + 3]), "r"(qi[half * 4 + 2]), "r"(0));
-        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(word) : "r"(qi[half * 4 + 1]), "r"(qi[half * 4 + 0]), "r"(hi16));
-        w[half] = word;
+      for (int i = 0; i < LOADS; ++i) {   // all lanes: the row statistics are reduced with full-warp shuffles
+        const int src = source(blk, i);
+        normalize8<T, NM, TPR>(row[i], c8, D, b, h, N, first + blk * 64 + r0 + i * RPL < N ? src : 0, norm);
       }
-      *reinterpret_cast<uint2*>(out + ((size_t)bh * N + tok) * D + c8) = make_uint2(w[0], w[1]);
+    }
+    if constexpr (TABLE) {
+      constexpr int NR = GM == GM_ROPE_F32 ? ROTATE_ROWS_F32 : ROTATE_ROWS_F64;
+#pragma unroll
+      for (int i = 0; i < LOADS; i += NR) gc.template rotate<NR>(row + i, pa, rows, blk * 64 + r0 + i * RPL, RPL);
+    }
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+      if (first + blk * 64 + r0 + i * RPL < N) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(widen(row[i], j)));
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) s_amax[blk & 1][warp] = amax;   // (two buffers: one barrier per block)
+    __syncthreads();
+    constexpr int GW = WARPS * GROUP / 64;   // warps per scale group
+    const int g0 = warp / GW * GW;
+    amax = 1e-7f;
+#pragma unroll
+    for (int i = 0; i < GW; ++i) amax = fmaxf(amax, s_amax[blk & 1][g0 + i]);
+    if (lane == 0 && warp == g0)
+      scale[(size_t)bh * n_scale_per_bh + (first / 64 + blk) * (64 / GROUP) + warp / GW] = __fdiv_rn(amax, 127.0f);
+    const float inv = __fdiv_rn(127.0f, amax);
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) {
+      const int tok = first + blk * 64 + r0 + i * RPL;
+      if (tok < N) {
+        // round to nearest even (NaN -> 0), then saturate and pack two values per instruction
+        int qi[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) qi[j] = __float2int_rn(__fmul_rn(widen(row[i], j), inv));
+        uint32_t w[2];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t hi16, word;
+          asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(hi16) : "r"(qi[half * 4 + 3]), "r"(qi[half * 4 + 2]), "r"(0));
+          asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(word) : "r"(qi[half * 4 + 1]), "r"(qi[half * 4 + 0]), "r"(hi16));
+          w[half] = word;
+        }
+        *reinterpret_cast<uint2*>(out + ((size_t)bh * N + tok) * D + c8) = make_uint2(w[0], w[1]);
+      }
     }
   }
 }
@@ -299,8 +356,7 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
 // four matrices of one ldmatrix leave a thread with EIGHT consecutive tokens of its channel: tokens
 // 8*(row/2) + 2*matrix + row%2 of a 32-token group.  A thread then stores 16 bytes and four lanes together
 // 64, whole sectors.  16-byte chunks are XOR-swizzled by (token & 1) | (token/8 & 3) * 2, which takes the
-// eight rows of every matrix to different banks.  2 x 12 x 32760 x 128: 126 -> 80 us, 2 x 48 x 17776 x 64: 121 us (read
-// column by column, two bytes at a time, and stored 16 bytes per channel: half sectors).
+// eight rows of every matrix to different banks.
 template <typename T, int D, int GM>
 __global__ void __launch_bounds__(256)
 quant_v_fp8_kernel(const T* __restrict__ v, int H, int N, int npad, int64_t sb, int64_t sh, int64_t sn,
@@ -323,9 +379,8 @@ quant_v_fp8_kernel(const T* __restrict__ v, int H, int N, int npad, int64_t sb, 
     // each of the warp's eight rows is decoded once, by lane (load, row of the load), and handed to its threads
     int d_src = 0;
     if constexpr (GM != GM_PLAIN) {
-      int gf, gy, gx;
       const int t = t0 + (threadIdx.x >> 5) * RPW + lane % RPW + (lane / RPW) % LOADS * ROWS;
-      if (t < N) d_src = gc.source(t, gf, gy, gx);
+      if (t < N) d_src = gc.source(t);
     }
 #pragma unroll
     for (int i = 0; i < LOADS; ++i) {
@@ -398,17 +453,27 @@ size_t stats_bytes(int B, int H, int N, int D) {
   return bh * stats_chunks(N) * D * sizeof(ChannelPartial) + 2 * bh * D * sizeof(float);
 }
 
-template <typename T>
-void launch_stats(const void* x, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn,
-                  ChannelPartial* part, cudaStream_t s, const Gather& g = Gather{}) {
-  dim3 grid(stats_chunks(N), B * H);
+// The statistics of n = 1 or 2 tensors (gather: the first one only, n = 1) and their fold.
+template <typename T, bool EXTREMES>
+void launch_stats(const StatsSrc* src, const FinalizeDst<T>* dst, int n, int B, int H, int N, int D, cudaStream_t s,
+                  const Gather& g = Gather{}, int32_t* zero_word = nullptr) {
+  const int chunks = stats_chunks(N);
+  const dim3 grid(chunks, B * H, n);
   dispatch_gather(g, [&](auto gm) {
-    constexpr int GM = decltype(gm)::value;
-    if (D == 128)
-      channel_stats_kernel<T, 128, GM><<<grid, 256, 0, s>>>((const T*)x, H, N, sb, sh, sn, part, stats_chunks(N), g);
-    else
-      channel_stats_kernel<T, 64, GM><<<grid, 256, 0, s>>>((const T*)x, H, N, sb, sh, sn, part, stats_chunks(N), g);
+    constexpr int GM = EXTREMES ? GM_PLAIN : decltype(gm)::value;   // (the extremes of V do not depend on the order)
+    if (D == 128) channel_stats_kernel<T, 128, GM, EXTREMES><<<grid, 256, 0, s>>>(src[0], src[n - 1], H, N, chunks, g);
+    else channel_stats_kernel<T, 64, GM, EXTREMES><<<grid, 256, 0, s>>>(src[0], src[n - 1], H, N, chunks, g);
   });
+  channel_finalize_kernel<T><<<dim3(B * H, n), FIN_GROUPS * D, 0, s>>>(dst[0], dst[n - 1], chunks, D, N, zero_word);
+}
+
+// Mean over tokens of one tensor.
+template <typename T>
+void launch_mean(const void* x, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn, ChannelPartial* part,
+                 void* mean_t, float* mean_f32, cudaStream_t s, const Gather& g = Gather{}) {
+  const StatsSrc src{x, sb, sh, sn, part};
+  const FinalizeDst<T> dst{part, 1, 1.f, static_cast<T*>(mean_t), mean_f32, nullptr, nullptr, nullptr};
+  launch_stats<T, false>(&src, &dst, 1, B, H, N, D, s, g);
 }
 
 }  // namespace
@@ -429,16 +494,8 @@ extern "C" int paro_channel_mean(const void* x, int dtype, int B, int H, int N, 
   PARO_REQUIRE(aligned16(scratch), PARO_EALIGN, "paro_channel_mean: scratch not 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
   ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
-  if (dtype == PARO_F16) {
-    launch_stats<__half>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__half><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (__half*)mean_out,
-                                                        mean_f32, nullptr, nullptr, nullptr);
-  } else {
-    launch_stats<__nv_bfloat16>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__nv_bfloat16><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f,
-                                                               (__nv_bfloat16*)mean_out, mean_f32, nullptr, nullptr,
-                                                               nullptr);
-  }
+  if (dtype == PARO_F16) launch_mean<__half>(x, B, H, N, D, stride_b, stride_h, stride_n, part, mean_out, mean_f32, s);
+  else launch_mean<__nv_bfloat16>(x, B, H, N, D, stride_b, stride_h, stride_n, part, mean_out, mean_f32, s);
   return check_launch("channel_mean", 2);
 }
 
@@ -447,15 +504,18 @@ template <typename T, int D, int NM>
 void launch_int8_norm(const void* x, const void* km, int8_t* out, float* scale, int B, int H, int N, int64_t sb,
                       int64_t sh, int64_t sn, float fold, int group, cudaStream_t s, const Gather& g, const NormArgs& nm) {
   const int nb = (N + 63) / 64;
-  dim3 grid(nb, B * H);
   dispatch_gather(g, [&](auto gm) {
     constexpr int GM = decltype(gm)::value;
+    // several blocks per CTA where that leaves every SM a few CTAs; below that one each, for the latency
+    const int64_t total = (int64_t)nb * B * H;
+    const int blocks = !Int8Cfg<GM>::TABLE ? 1 : total >= 148 * 16 ? INT8_BLOCKS : total >= 148 * 8 ? 2 : 1;
+    const dim3 grid((nb + blocks - 1) / blocks, B * H);
     if (group == 64)
-      quant_int8_kernel<T, D, 64, GM, NM><<<grid, 128, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N, sb, sh, sn,
-                                                               fold, nb, g, nm);
+      quant_int8_kernel<T, D, 64, GM, NM><<<grid, 32 * Int8Cfg<GM>::WARPS, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N,
+                                                                                   sb, sh, sn, fold, nb, blocks, g, nm);
     else
-      quant_int8_kernel<T, D, 32, GM, NM><<<grid, 128, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N, sb, sh, sn,
-                                                               fold, nb * 2, g, nm);
+      quant_int8_kernel<T, D, 32, GM, NM><<<grid, 32 * Int8Cfg<GM>::WARPS, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N,
+                                                                                   sb, sh, sn, fold, nb * 2, blocks, g, nm);
   });
 }
 
@@ -490,18 +550,10 @@ extern "C" int paro_quant_int8(const void* x, int dtype, int B, int H, int N, in
 }
 
 namespace {
+// The quantisation pass of V; inv_tab / mean_tab from the statistics.
 template <typename T>
-int run_v_fp8(const void* v, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn, int smooth,
-              float scale_max, uint8_t* v8, uint16_t* v16, float* v_scale, float* vm, void* scratch,
-              cudaStream_t s, const Gather& g = Gather{}) {
-  const int chunks = stats_chunks(N);
-  const size_t bh = (size_t)B * H;
-  ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
-  float* inv_tab = reinterpret_cast<float*>(part + bh * chunks * D);
-  float* mean_tab = inv_tab + bh * D;
-  launch_stats<T>(v, B, H, N, D, sb, sh, sn, part, s);   // statistics do not depend on the token order
-  channel_finalize_kernel<T><<<B * H, FIN_GROUPS * D, 0, s>>>(part, chunks, D, N, smooth, scale_max, (T*)nullptr,
-                                                 smooth ? vm : nullptr, v_scale, inv_tab, mean_tab);
+void launch_v_fp8(const void* v, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn, const float* inv_tab,
+                  const float* mean_tab, uint8_t* v8, uint16_t* v16, cudaStream_t s, const Gather& g) {
   const int npad = (N + 63) / 64 * 64;
   dim3 grid(npad / 64, B * H);
   dispatch_gather(g, [&](auto gm) {
@@ -514,6 +566,20 @@ int run_v_fp8(const void* v, int B, int H, int N, int D, int64_t sb, int64_t sh,
       quant_v_fp8_kernel<T, 64, GM><<<grid, 256, 0, s>>>((const T*)v, H, N, npad, sb, sh, sn, inv_tab, mean_tab, v8,
                                                          (__nv_bfloat16*)v16, g);
   });
+}
+
+template <typename T>
+int run_v_fp8(const void* v, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn, int smooth,
+              float scale_max, uint8_t* v8, uint16_t* v16, float* v_scale, float* vm, void* scratch,
+              cudaStream_t s, const Gather& g = Gather{}) {
+  const size_t bh = (size_t)B * H;
+  ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
+  float* inv_tab = reinterpret_cast<float*>(part + bh * stats_chunks(N) * D);
+  float* mean_tab = inv_tab + bh * D;
+  const StatsSrc src{v, sb, sh, sn, part};                // statistics do not depend on the token order
+  const FinalizeDst<T> dst{part, smooth, scale_max, nullptr, smooth ? vm : nullptr, v_scale, inv_tab, mean_tab};
+  launch_stats<T, true>(&src, &dst, 1, B, H, N, D, s);
+  launch_v_fp8<T>(v, B, H, N, D, sb, sh, sn, inv_tab, mean_tab, v8, v16, s, g);
   return check_launch("quant_v_fp8", 3);
 }
 }  // namespace
@@ -591,16 +657,8 @@ extern "C" int paro_channel_mean_noalloc(const void* x, int dtype, int B, int H,
   ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
   // every partial the second pass reads is written by the first pass of the same call, so nothing
   // left behind by an earlier call has to be cleared
-  if (dtype == PARO_F16) {
-    launch_stats<__half>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__half><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (__half*)mean_out,
-                                                        mean_f32, nullptr, nullptr, nullptr);
-  } else {
-    launch_stats<__nv_bfloat16>(x, B, H, N, D, stride_b, stride_h, stride_n, part, s);
-    channel_finalize_kernel<__nv_bfloat16><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f,
-                                                               (__nv_bfloat16*)mean_out, mean_f32, nullptr, nullptr,
-                                                               nullptr);
-  }
+  if (dtype == PARO_F16) launch_mean<__half>(x, B, H, N, D, stride_b, stride_h, stride_n, part, mean_out, mean_f32, s);
+  else launch_mean<__nv_bfloat16>(x, B, H, N, D, stride_b, stride_h, stride_n, part, mean_out, mean_f32, s);
   return check_launch("channel_mean_noalloc", 2);
 }
 
@@ -613,17 +671,11 @@ int make_gather(Gather* g, const char* who, int N, int D, int n_text, int F, int
                 int rope_mode, const void* cos_tab, const void* sin_tab, int pairs_f, int pairs_h) {
   PARO_REQUIRE(F > 0 && Hh > 0 && W > 0 && n_text >= 0 && (int64_t)n_text + (int64_t)F * Hh * W == N, PARO_ESHAPE,
                "%s: n_text + F*H*W = %lld != N = %d", who, (long long)n_text + (long long)F * Hh * W, N);
-  PARO_REQUIRE(rope_mode >= PARO_ROPE_NONE && rope_mode <= PARO_ROPE_COMPLEX_F64, PARO_EINVAL,
-               "%s: unknown rope_mode %d", who, rope_mode);
-  if (rope_mode != PARO_ROPE_NONE) {
-    PARO_REQUIRE(cos_tab, PARO_EINVAL, "%s: rope tables missing", who);   // sin_tab NULL = interleaved (cos, sin) table
-    PARO_REQUIRE(pairs_f >= 0 && pairs_h >= 0 && pairs_f + pairs_h <= D / 2, PARO_ESHAPE,
-                 "%s: pairs_f + pairs_h exceeds D/2", who);
-  }
+  if (int rc = check_rope(who, rope_mode, cos_tab, sin_tab, pairs_f, pairs_h, D)) return rc;
   g->enabled = 1;
   g->n_text = n_text; g->F = F; g->Hh = Hh; g->W = W;
   g->order_ids = order_ids;
-  g->rope = RopeArgs{rope_mode, cos_tab, sin_tab, pairs_f, pairs_h};
+  g->rope = make_rope(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h);
   return PARO_OK;
 }
 
@@ -637,10 +689,7 @@ int run_prep_int8(const void* x, int B, int H, int N, int D, int64_t sb, int64_t
     // reads the input in natural order (rotation only)
     Gather gs = g;
     gs.order_ids = nullptr;
-    ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
-    launch_stats<T>(x, B, H, N, D, sb, sh, sn, part, s, gs);
-    channel_finalize_kernel<T><<<B * H, FIN_GROUPS * D, 0, s>>>(part, stats_chunks(N), D, N, 1, 1.f, (T*)km_out, nullptr, nullptr,
-                                                   nullptr, nullptr);
+    launch_mean<T>(x, B, H, N, D, sb, sh, sn, static_cast<ChannelPartial*>(scratch), km_out, nullptr, s, gs);
     km = static_cast<const T*>(km_out);
     launches = 3;
   }
@@ -720,4 +769,46 @@ extern "C" int paro_prep_v_fp8(const void* v, int dtype, int B, int H, int N, in
   return dtype == PARO_F16
              ? run_v_fp8<__half>(v, B, H, N, D, stride_b, stride_h, stride_n, smooth, scale_max, v8, v16, v_scale, vm, scratch, s, g)
              : run_v_fp8<__nv_bfloat16>(v, B, H, N, D, stride_b, stride_h, stride_n, smooth, scale_max, v8, v16, v_scale, vm, scratch, s, g);
+}
+
+// What a layer does with V, and with K's rotated copy `kp` (contiguous; NULL: K is not smoothed): the statistics of
+// both in one launch, their fold in another, then both quantisation passes.
+namespace {
+template <typename T>
+int layer_kv(const void* kp, const void* v, const int64_t* vst, int B, int H, int N, int D, const Gather& g, int smooth_v,
+             void* km, int8_t* k8, float* ks, uint16_t* v16, float* vs, float* vm, void* scratch, int32_t* zero_word,
+             cudaStream_t s) {
+  const size_t bh = (size_t)B * H, n_part = bh * stats_chunks(N) * D;
+  ChannelPartial* part = static_cast<ChannelPartial*>(scratch);
+  float* inv_tab = reinterpret_cast<float*>(part + 2 * n_part);
+  float* mean_tab = inv_tab + bh * D;
+  const int64_t ksn = D, ksh = ksn * N, ksb = ksh * H;
+  const StatsSrc src[2] = {{v, vst[0], vst[1], vst[2], part}, {kp, ksb, ksh, ksn, part + n_part}};
+  const FinalizeDst<T> dst[2] = {{part, smooth_v, 448.0f, nullptr, smooth_v ? vm : nullptr, vs, inv_tab, mean_tab},
+                                 {part + n_part, 1, 1.f, static_cast<T*>(km), nullptr, nullptr, nullptr, nullptr}};
+  launch_stats<T, true>(src, dst, kp ? 2 : 1, B, H, N, D, s, Gather{}, zero_word);
+  launch_v_fp8<T>(v, B, H, N, D, vst[0], vst[1], vst[2], inv_tab, mean_tab, nullptr, v16, s, g);
+  if (int rc = check_launch("layer_kv", 3)) return rc;
+  if (!kp) return PARO_OK;
+  return D == 128 ? launch_int8<T, 128>(kp, km, k8, ks, B, H, N, ksb, ksh, ksn, 0.f, 64, s)
+                  : launch_int8<T, 64>(kp, km, k8, ks, B, H, N, ksb, ksh, ksn, 0.f, 64, s);
+}
+}  // namespace
+
+size_t paro::layer_kv_scratch_bytes(int B, int H, int N, int D) {
+  return 2 * stats_bytes(B, H, N, D);
+}
+
+int paro::layer_kv_passes(const paro_layer_args& a, const void* kp, void* km, int8_t* k8, float* ks, uint16_t* v16, float* vs,
+                          float* vm, void* scratch, int32_t* zero_word, cudaStream_t s) {
+  if (int rc = check_tensor("paro_layer(v)", a.v, a.dtype, a.B, a.H, a.N, a.D, a.v_strides[0], a.v_strides[1], a.v_strides[2]))
+    return rc;
+  Gather g{};
+  if (int rc = make_gather(&g, "paro_layer", a.N, a.D, a.n_text, a.F, a.Hh, a.W, a.order_ids, PARO_ROPE_NONE, nullptr, nullptr,
+                           0, 0))
+    return rc;
+  return a.dtype == PARO_F16
+             ? layer_kv<__half>(kp, a.v, a.v_strides, a.B, a.H, a.N, a.D, g, a.smooth_v, km, k8, ks, v16, vs, vm, scratch, zero_word, s)
+             : layer_kv<__nv_bfloat16>(kp, a.v, a.v_strides, a.B, a.H, a.N, a.D, g, a.smooth_v, km, k8, ks, v16, vs, vm, scratch,
+                                       zero_word, s);
 }

@@ -3,6 +3,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "perm.cuh"
 
 namespace paro {
 
@@ -11,101 +12,182 @@ struct RopeArgs {
   const void* cos_tab; // [F+Hh+W, D/2]; or, when sin_tab is NULL, [F+Hh+W, D/2, 2] holding (cos, sin) side by side
   const void* sin_tab; // [F+Hh+W, D/2] or NULL (one 8- or 16-byte load then fetches both values of a pair)
   int pairs_f, pairs_h;
+  const float4* tab32; // the table as fp32, cos and sin side by side, 16-byte aligned: two pairs per load; or NULL
 };
 
-// Angles of the thread's four channel pairs, kept from one row to the next: consecutive rows of the
-// reordered sequence differ in the fastest grid coordinate only, so the pairs driven by the other two
-// coordinates find their (cos, sin) already in registers and skip the table load.
-template <int MODE> struct RotCache {
-  using F = typename std::conditional<MODE == PARO_ROPE_REAL_F32, float, double>::type;
-  F c[4], s[4];
-  int row[4];
-  __device__ __forceinline__ RotCache() {
+// tab32 of a call: REAL_F32 with an interleaved table is that table; COMPLEX_F64_APPROX brings one next to its fp64
+// table (which the values that fp32 cannot settle are computed from).
+inline RopeArgs make_rope(int mode, const void* cos_tab, const void* sin_tab, int pairs_f, int pairs_h) {
+  RopeArgs r{mode, cos_tab, sin_tab, pairs_f, pairs_h, nullptr};
+  if (mode == PARO_ROPE_COMPLEX_F64_APPROX) {
+    r.mode = PARO_ROPE_COMPLEX_F64;
+    r.sin_tab = nullptr;
+    r.tab32 = static_cast<const float4*>(sin_tab);
+  } else if (mode == PARO_ROPE_REAL_F32 && !sin_tab && aligned16(cos_tab)) {
+    r.tab32 = static_cast<const float4*>(cos_tab);
+  }
+  return r;
+}
+
+// Arguments common to the entry points that rotate.
+inline int check_rope(const char* who, int mode, const void* cos_tab, const void* sin_tab, int pairs_f, int pairs_h, int D) {
+  PARO_REQUIRE(mode >= PARO_ROPE_NONE && mode <= PARO_ROPE_COMPLEX_F64_APPROX, PARO_EINVAL, "%s: unknown rope_mode %d", who, mode);
+  if (mode == PARO_ROPE_NONE) return PARO_OK;
+  PARO_REQUIRE(cos_tab, PARO_EINVAL, "%s: rope tables missing", who);   // sin_tab NULL = interleaved (cos, sin) table
+  PARO_REQUIRE(pairs_f >= 0 && pairs_h >= 0 && pairs_f + pairs_h <= D / 2, PARO_ESHAPE, "%s: pairs_f + pairs_h exceeds D/2", who);
+  PARO_REQUIRE(mode != PARO_ROPE_COMPLEX_F64_APPROX || (sin_tab && aligned16(sin_tab)), PARO_EALIGN,
+               "%s: the fp32 table is missing or not 16-byte aligned", who);
+  return PARO_OK;
+}
+
+template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Where the rows of a block of the (reordered) sequence come from and which table rows turn them, worked out once
+// per row by one thread (two integer divisions by run-time extents) instead of by each of the row's D/8 threads.
+// off[a][r]: table row of axis a times D/4, i.e. the offset of its first two pairs; -1: the row is not rotated.
+template <int ROWS> struct RowTable {
+  int src[ROWS];
+  int off[3][ROWS];
+};
+
+template <int ROWS>
+__device__ __forceinline__ void fill_row(RowTable<ROWS>& t, int r, int tok, int N, int quarter, const PermDecoder& dec,
+                                         int n_text, int F, int Hh) {
+  int src = tok, f = -1, y = 0, x = 0;
+  if (tok >= n_text && tok < N) src = n_text + dec.source(tok - n_text, f, y, x);
+  t.src[r] = src;
+  t.off[0][r] = f < 0 ? -1 : f * quarter;
+  t.off[1][r] = f < 0 ? -1 : (F + y) * quarter;
+  t.off[2][r] = f < 0 ? -1 : (F + Hh + x) * quarter;
+}
+
+// What a thread that owns channels c8..c8+7 needs to find its four pairs' angles: the axis that drives each.
+struct PairAxes {
+  int pair0, ax[4];
+  __device__ __forceinline__ PairAxes(int c8, const RopeArgs& r) : pair0(c8 >> 1) {
 #pragma unroll
-    for (int p = 0; p < 4; ++p) row[p] = -1;
+    for (int p = 0; p < 4; ++p)
+      ax[p] = pair0 + p < r.pairs_f ? 0 : (pair0 + p < r.pairs_f + r.pairs_h ? 1 : 2);
   }
 };
 
-// Rotates the four channel pairs held in `x` (channels c8..c8+7 of a token at grid
-// coordinate f,y,x).  Products and sums are rounded separately (no fused multiply-add) so that
-// results equal a plain elementwise evaluation.
-// MODE: PARO_ROPE_REAL_F32 or PARO_ROPE_COMPLEX_F64 (compile time, so that a kernel only carries the
-// registers of the arithmetic it uses).
-template <typename T, int MODE>
-__device__ __forceinline__ void rotate8(Pack8<T>& x, int c8, int D, int f, int y, int xw,
-                                        int F, int Hh, const RopeArgs& r, RotCache<MODE>& cache) {
-  using FT = typename RotCache<MODE>::F;
+// fp64 rotation of a channel pair, rounded to fp32 and then to the 16-bit type.  Products and sums are rounded
+// separately (no fused multiply-add) so that results equal a plain elementwise evaluation.
+template <typename T>
+__device__ __forceinline__ uint32_t rotate_pair_f64(float x0, float x1, double c, double s) {
+  const double a = (double)x0, b = (double)x1;
+  const double re = __dsub_rn(__dmul_rn(a, c), __dmul_rn(b, s));
+  const double im = __dadd_rn(__dmul_rn(a, s), __dmul_rn(b, c));
+  return pack_pair<T>(__double2float_rn(re), __double2float_rn(im));
+}
+template <typename T>
+__device__ __forceinline__ uint32_t rotate_pair_f32(float x0, float x1, float c, float s) {
+  return pack_pair<T>(__fadd_rn(__fmul_rn(x0, c), __fmul_rn(-x1, s)), __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s)));
+}
+
+// The fp64 result's bits from fp32 arithmetic, or a non-zero return where these are not certain.  fp32 is off by at
+// most 3 * 2^-24 * (|x0|+|x1|) * (|c|+|s|); e is twice that (the rounding of r-e, r+e itself included), 2^-100 and
+// 2^-140 cover table entries and products below the normal range.  Rounding is monotonic: where r-e and r+e round to
+// the same 16-bit value the fp64 result between them does too.  Uncertain are about one value in 2^13 for bf16 and
+// 2^10 for fp16, and zeros, Inf and NaN.
+template <typename T>
+__device__ __forceinline__ uint32_t rotate_pair_checked(float x0, float x1, float c, float s, uint32_t& out) {
+  const float re = fmaf(x0, c, -__fmul_rn(x1, s)), im = fmaf(x0, s, __fmul_rn(x1, c));
+  const float e = fmaf(__fmul_rn(fabsf(x0) + fabsf(x1), fabsf(c) + fabsf(s) + 0x1p-100f), 0x3p-23f, 0x1p-140f);
+  out = pack_pair<T>(re - e, im - e);
+  return out ^ pack_pair<T>(re + e, im + e);
+}
+
+template <int MODE>
+__device__ __forceinline__ void load_angles(const RopeArgs& r, size_t t,
+                                            typename std::conditional<MODE == PARO_ROPE_REAL_F32, float, double>::type& c,
+                                            typename std::conditional<MODE == PARO_ROPE_REAL_F32, float, double>::type& s) {
+  using FT = typename std::conditional<MODE == PARO_ROPE_REAL_F32, float, double>::type;
   using FT2 = typename std::conditional<MODE == PARO_ROPE_REAL_F32, float2, double2>::type;
-  const int half = D >> 1;
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int pair = (c8 >> 1) + p;
-    const int row = pair < r.pairs_f ? f : (pair < r.pairs_f + r.pairs_h ? F + y : F + Hh + xw);
-    if (row != cache.row[p]) {
-      const size_t t = (size_t)row * half + pair;
-      if (r.sin_tab == nullptr) {
-        const FT2 cs = static_cast<const FT2*>(r.cos_tab)[t];
-        cache.c[p] = cs.x; cache.s[p] = cs.y;
-      } else {
-        cache.c[p] = static_cast<const FT*>(r.cos_tab)[t];
-        cache.s[p] = static_cast<const FT*>(r.sin_tab)[t];
-      }
-      cache.row[p] = row;
-    }
-    const FT c = cache.c[p], s = cache.s[p];
-    if constexpr (MODE == PARO_ROPE_REAL_F32) {
-      const float x0 = F16Traits<T>::to_float(x.e[2 * p]);
-      const float x1 = F16Traits<T>::to_float(x.e[2 * p + 1]);
-      const float o0 = __fadd_rn(__fmul_rn(x0, c), __fmul_rn(-x1, s));
-      const float o1 = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
-      x.e[2 * p] = F16Traits<T>::from_float(o0);
-      x.e[2 * p + 1] = F16Traits<T>::from_float(o1);
-    } else {
-      const double x0 = (double)F16Traits<T>::to_float(x.e[2 * p]);
-      const double x1 = (double)F16Traits<T>::to_float(x.e[2 * p + 1]);
-      const double re = __dsub_rn(__dmul_rn(x0, c), __dmul_rn(x1, s));
-      const double im = __dadd_rn(__dmul_rn(x0, s), __dmul_rn(x1, c));
-      x.e[2 * p] = F16Traits<T>::from_float(__double2float_rn(re));
-      x.e[2 * p + 1] = F16Traits<T>::from_float(__double2float_rn(im));
-    }
+  if (r.sin_tab == nullptr) {
+    const FT2 cs = static_cast<const FT2*>(r.cos_tab)[t];
+    c = cs.x; s = cs.y;
+  } else {
+    c = static_cast<const FT*>(r.cos_tab)[t];
+    s = static_cast<const FT*>(r.sin_tab)[t];
   }
 }
 
-// Without a cache: straight-line code, every pair's angles are loaded (what the quantiser front ends use;
-// there the compare-and-skip of the cached form costs more than the loads it saves).
-template <typename T, int MODE>
-__device__ __forceinline__ void rotate8(Pack8<T>& x, int c8, int D, int f, int y, int xw,
-                                        int F, int Hh, const RopeArgs& r) {
-  using FT = typename RotCache<MODE>::F;
-  using FT2 = typename std::conditional<MODE == PARO_ROPE_REAL_F32, float2, double2>::type;
-  const int half = D >> 1;
+// Rows rotated at a time.  Two hide more of the table's latency (LayerNorm + rotation + reorder of 2 x 48 x 17776 x 64:
+// 187 -> 168 us), but with the fp64 fallback the second row's registers cost more than that (RMS norm, 2 x 12 x 32760 x
+// 128: 167 us one at a time, 217 two).
+constexpr int ROTATE_ROWS_F32 = 2, ROTATE_ROWS_F64 = 1;
+
+// Rotates the four channel pairs held in each of x[0..NR), rows r, r + step, ... of the table.  The angles of all NR
+// rows are requested before the first is used, and the rows meet in one branch (for values that fp32 does not settle),
+// so that their latencies overlap.  MODE: PARO_ROPE_REAL_F32 or PARO_ROPE_COMPLEX_F64 (compile time, so that a
+// kernel only carries the registers of the arithmetic it uses).
+template <int NR, typename T, int MODE, int ROWS>
+__device__ __forceinline__ void rotate8(Pack8<T>* x, const PairAxes& pa, const RowTable<ROWS>& rows, int r, int step,
+                                        const RopeArgs& rope) {
+  uint32_t bad = 1;
+  if (rope.tab32) {
+    // Two pairs per 16-byte load.  Where an axis ends between the two, the second one's angles are loaded by
+    // themselves.
+    float4 cs[NR][2];
+    int o0[NR];
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int pair = (c8 >> 1) + p;
-    const int row = pair < r.pairs_f ? f : (pair < r.pairs_f + r.pairs_h ? F + y : F + Hh + xw);
-    const size_t t = (size_t)row * half + pair;
-    FT c, s;
-    if (r.sin_tab == nullptr) {
-      const FT2 cs = static_cast<const FT2*>(r.cos_tab)[t];
-      c = cs.x; s = cs.y;
-    } else {
-      c = static_cast<const FT*>(r.cos_tab)[t];
-      s = static_cast<const FT*>(r.sin_tab)[t];
+    for (int u = 0; u < NR; ++u) {
+      o0[u] = rows.off[pa.ax[0]][r + u * step];
+      const int o2 = rows.off[pa.ax[2]][r + u * step];
+      cs[u][0] = rope.tab32[max(o0[u], 0) + (pa.pair0 >> 1)];
+      cs[u][1] = rope.tab32[max(o2, 0) + (pa.pair0 >> 1) + 1];
     }
-    if constexpr (MODE == PARO_ROPE_REAL_F32) {
-      const float x0 = F16Traits<T>::to_float(x.e[2 * p]);
-      const float x1 = F16Traits<T>::to_float(x.e[2 * p + 1]);
-      const float o0 = __fadd_rn(__fmul_rn(x0, c), __fmul_rn(-x1, s));
-      const float o1 = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
-      x.e[2 * p] = F16Traits<T>::from_float(o0);
-      x.e[2 * p + 1] = F16Traits<T>::from_float(o1);
-    } else {
-      const double x0 = (double)F16Traits<T>::to_float(x.e[2 * p]);
-      const double x1 = (double)F16Traits<T>::to_float(x.e[2 * p + 1]);
-      const double re = __dsub_rn(__dmul_rn(x0, c), __dmul_rn(x1, s));
-      const double im = __dadd_rn(__dmul_rn(x0, s), __dmul_rn(x1, c));
-      x.e[2 * p] = F16Traits<T>::from_float(__double2float_rn(re));
-      x.e[2 * p + 1] = F16Traits<T>::from_float(__double2float_rn(im));
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (pa.ax[2 * h + 1] != pa.ax[2 * h]) {
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+          const int o = max(rows.off[pa.ax[2 * h + 1]][r + u * step], 0);
+          const float2 second = reinterpret_cast<const float2*>(rope.tab32)[2 * o + pa.pair0 + 2 * h + 1];
+          cs[u][h].z = second.x; cs[u][h].w = second.y;
+        }
+      }
+    uint32_t out[NR][4];
+    bad = 0;
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+      uint32_t b = 0;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const float c = p & 1 ? cs[u][p >> 1].z : cs[u][p >> 1].x, s = p & 1 ? cs[u][p >> 1].w : cs[u][p >> 1].y;
+        const float x0 = F16Traits<T>::to_float(x[u].e[2 * p]), x1 = F16Traits<T>::to_float(x[u].e[2 * p + 1]);
+        if constexpr (MODE == PARO_ROPE_REAL_F32) out[u][p] = rotate_pair_f32<T>(x0, x1, c, s);
+        else b |= rotate_pair_checked<T>(x0, x1, c, s, out[u][p]);
+      }
+      if (o0[u] >= 0) bad |= b;
+    }
+    if (MODE == PARO_ROPE_REAL_F32 || !bad) {
+#pragma unroll
+      for (int u = 0; u < NR; ++u)
+        if (o0[u] >= 0) x[u].v = make_uint4(out[u][0], out[u][1], out[u][2], out[u][3]);
+      return;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < NR; ++u) {
+    if (rows.off[0][r + u * step] < 0) continue;
+    uint32_t* w = reinterpret_cast<uint32_t*>(&x[u].v);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      typename std::conditional<MODE == PARO_ROPE_REAL_F32, float, double>::type c, s;
+      load_angles<MODE>(rope, (size_t)(2 * rows.off[pa.ax[p]][r + u * step] + pa.pair0 + p), c, s);
+      const float x0 = F16Traits<T>::to_float(x[u].e[2 * p]), x1 = F16Traits<T>::to_float(x[u].e[2 * p + 1]);
+      if constexpr (MODE == PARO_ROPE_REAL_F32) w[p] = rotate_pair_f32<T>(x0, x1, c, s);
+      else w[p] = rotate_pair_f64<T>(x0, x1, c, s);
     }
   }
 }

@@ -8,8 +8,7 @@
 
 namespace paro {
 
-// Block = 256 threads; a thread owns one 16-byte slice of PASSES consecutive rows (consecutive rows share
-// the slow grid coordinates, so most of their rotation angles are reused from registers).
+// Block = 256 threads = 64 (D = 128) or 128 rows; a thread owns one 16-byte slice of PASSES consecutive rows.
 // blockIdx.x: group of rows, blockIdx.y: b*H + h.
 template <typename T, int D, int MODE, int NM>
 __global__ void __launch_bounds__(256)
@@ -17,55 +16,42 @@ rope_permute_kernel(const T* __restrict__ in, T* __restrict__ out, int H, int N,
                     int64_t sb, int64_t sh, int64_t sn, int n_text, int F, int Hh, int W,
                     const int32_t* __restrict__ order_ids, int inverse, RopeArgs rope, NormArgs norm) {
   constexpr int TPR = D / 8;            // threads per row
-  constexpr int ROWS = 256 / TPR;       // rows per pass
   constexpr int PASSES = 4;
+  constexpr int BLOCK_ROWS = 256 / TPR * PASSES;
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
   const int c8 = (threadIdx.x % TPR) * 8;
-  const int r0 = blockIdx.x * (ROWS * PASSES) + (threadIdx.x / TPR) * PASSES;
-  const PermDecoder dec(order_ids ? order_ids[h] : 0, F, Hh, W);
-  const T* src_base = in + b * sb + h * sh;
-  T* dst_base = out + (size_t)bh * N * D;
+  const int tok0 = blockIdx.x * BLOCK_ROWS, r0 = (threadIdx.x / TPR) * PASSES;
+  const T* src_base = in + b * sb + h * sh + c8;
+  T* dst_base = out + (size_t)bh * N * D + c8;
+  // (without order ids the rows keep their places: order 0)
+  __shared__ RowTable<BLOCK_ROWS> rows;
+  if (threadIdx.x < BLOCK_ROWS)
+    fill_row(rows, threadIdx.x, tok0 + threadIdx.x, N, D / 4, PermDecoder(order_ids ? order_ids[h] : 0, F, Hh, W), n_text, F, Hh);
+  __syncthreads();
 
   Pack8<T> val[PASSES];
-  int dst_row[PASSES], src_row[PASSES], fy[PASSES], yy[PASSES], xx[PASSES];
 #pragma unroll
   for (int i = 0; i < PASSES; ++i) {
-    const int row = r0 + i;
-    dst_row[i] = -1;
-    src_row[i] = 0;
+    const int r = r0 + i;
     val[i].v = make_uint4(0, 0, 0, 0);
-    if (row >= N) continue;
-    int src = row, dst = row;
-    fy[i] = yy[i] = xx[i] = -1;
-    if (row >= n_text) {
-      const int j = row - n_text;
-      int f, y, x;
-      const int other = n_text + dec.source(j, f, y, x);
-      if (order_ids == nullptr) {
-        // natural order: the coordinate of j itself
-        const PermDecoder ident(0, F, Hh, W);
-        ident.source(j, f, y, x);
-      } else if (inverse) {
-        dst = other;
-      } else {
-        src = other;
-      }
-      fy[i] = f; yy[i] = y; xx[i] = x;
-    }
-    dst_row[i] = dst;
-    src_row[i] = src;
-    val[i].v = *reinterpret_cast<const uint4*>(src_base + (size_t)src * sn + c8);
+    if (tok0 + r < N) val[i].v = *reinterpret_cast<const uint4*>(src_base + (size_t)(inverse ? tok0 + r : rows.src[r]) * sn);
   }
-  [[maybe_unused]] RotCache<MODE == PARO_ROPE_REAL_F32 ? PARO_ROPE_REAL_F32 : PARO_ROPE_COMPLEX_F64> rot;
+  [[maybe_unused]] const PairAxes pa(c8, rope);
+  // every lane takes part in the normalisation's shuffles, also those whose row is past the end
+  if constexpr (NM != PARO_NORM_NONE) {
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i)
+      normalize8<T, NM, TPR>(val[i], c8, D, b, h, N, tok0 + r0 + i < N ? rows.src[r0 + i] : 0, norm);
+  }
+  if constexpr (MODE != PARO_ROPE_NONE) {
+    constexpr int NR = MODE == PARO_ROPE_REAL_F32 ? ROTATE_ROWS_F32 : ROTATE_ROWS_F64;
+#pragma unroll
+    for (int i = 0; i < PASSES; i += NR) rotate8<NR, T, MODE>(val + i, pa, rows, r0 + i, 1, rope);
+  }
 #pragma unroll
   for (int i = 0; i < PASSES; ++i) {
-    // every lane takes part in the normalisation's shuffles, also those whose row is past the end
-    if constexpr (NM != PARO_NORM_NONE) normalize8<T, NM, TPR>(val[i], c8, D, b, h, N, src_row[i], norm);
-    if (dst_row[i] < 0) continue;
-    if constexpr (MODE != PARO_ROPE_NONE) {
-      if (fy[i] >= 0) rotate8<T, MODE>(val[i], c8, D, fy[i], yy[i], xx[i], F, Hh, rope, rot);
-    }
-    *reinterpret_cast<uint4*>(dst_base + (size_t)dst_row[i] * D + c8) = val[i].v;
+    const int r = r0 + i;
+    if (tok0 + r < N) *reinterpret_cast<uint4*>(dst_base + (size_t)(inverse ? rows.src[r] : tok0 + r) * D) = val[i].v;
   }
 }
 
@@ -144,16 +130,10 @@ extern "C" int paro_rope_permute(const void* in, void* out, int dtype, int B, in
   PARO_REQUIRE(in != out, PARO_EINVAL, "paro_rope_permute: in-place operation is not supported");
   PARO_REQUIRE(F > 0 && Hh > 0 && W > 0 && n_text >= 0 && (int64_t)n_text + (int64_t)F * Hh * W == N, PARO_ESHAPE,
                "paro_rope_permute: n_text + F*H*W = %lld != N = %d", (long long)n_text + (long long)F * Hh * W, N);
-  PARO_REQUIRE(rope_mode >= PARO_ROPE_NONE && rope_mode <= PARO_ROPE_COMPLEX_F64, PARO_EINVAL,
-               "paro_rope_permute: unknown rope_mode %d", rope_mode);
+  if (int rc = check_rope("paro_rope_permute", rope_mode, cos_tab, sin_tab, pairs_f, pairs_h, D)) return rc;
   PARO_REQUIRE(!(inverse && rope_mode != PARO_ROPE_NONE), PARO_EINVAL,
                "paro_rope_permute: the inverse permutation does not rotate");
-  if (rope_mode != PARO_ROPE_NONE) {
-    PARO_REQUIRE(cos_tab, PARO_EINVAL, "paro_rope_permute: rope tables missing");   // sin_tab NULL = interleaved (cos, sin) table
-    PARO_REQUIRE(pairs_f >= 0 && pairs_h >= 0 && pairs_f + pairs_h <= D / 2, PARO_ESHAPE,
-                 "paro_rope_permute: pairs_f + pairs_h exceeds D/2");
-  }
-  RopeArgs r{rope_mode, cos_tab, sin_tab, pairs_f, pairs_h};
+  const RopeArgs r = make_rope(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h);
   NormArgs nm{};
   cudaStream_t s = (cudaStream_t)stream;
   return dtype == PARO_F16
@@ -173,15 +153,9 @@ extern "C" int paro_rope_permute_norm(const void* in, void* out, int dtype, int 
   PARO_REQUIRE(in != out, PARO_EINVAL, "paro_rope_permute_norm: in-place operation is not supported");
   PARO_REQUIRE(F > 0 && Hh > 0 && W > 0 && n_text >= 0 && (int64_t)n_text + (int64_t)F * Hh * W == N, PARO_ESHAPE,
                "paro_rope_permute_norm: n_text + F*H*W = %lld != N = %d", (long long)n_text + (long long)F * Hh * W, N);
-  PARO_REQUIRE(rope_mode >= PARO_ROPE_NONE && rope_mode <= PARO_ROPE_COMPLEX_F64, PARO_EINVAL,
-               "paro_rope_permute_norm: unknown rope_mode %d", rope_mode);
-  if (rope_mode != PARO_ROPE_NONE) {
-    PARO_REQUIRE(cos_tab, PARO_EINVAL, "paro_rope_permute_norm: rope tables missing");
-    PARO_REQUIRE(pairs_f >= 0 && pairs_h >= 0 && pairs_f + pairs_h <= D / 2, PARO_ESHAPE,
-                 "paro_rope_permute_norm: pairs_f + pairs_h exceeds D/2");
-  }
+  if (int rc = check_rope("paro_rope_permute_norm", rope_mode, cos_tab, sin_tab, pairs_f, pairs_h, D)) return rc;
   if (int rc = check_norm("paro_rope_permute_norm", norm_mode, norm_weight, norm_bias, inv_rms, eps)) return rc;
-  RopeArgs r{rope_mode, cos_tab, sin_tab, pairs_f, pairs_h};
+  const RopeArgs r = make_rope(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h);
   NormArgs nm{norm_mode, norm_weight, norm_bias, inv_rms, eps};
   cudaStream_t s = (cudaStream_t)stream;
   return dtype == PARO_F16

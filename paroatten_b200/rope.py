@@ -21,6 +21,26 @@ class RopeTables:
         self.cos = torch.stack([cos, sin], dim=-1).contiguous()
         self.sin = None
         self.pairs_f, self.pairs_h = pairs_f, pairs_h
+        self.call_args()            # (the fp32 copy belongs to the stream that makes the table, not to its first user's)
+
+    def call_args(self):
+        """(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h) of an entry point.  An fp64 table goes with its fp32 copy
+        (PARO_ROPE_COMPLEX_F64_APPROX); the copy is made again when the table has been written to or replaced."""
+        cos, sin = self.cos, self.sin
+        if self.mode != _lib.ROPE_COMPLEX_F64 or sin is not None or cos.dtype != torch.float64:
+            return self.mode, cos.data_ptr(), _lib.ptr(sin), self.pairs_f, self.pairs_h
+        version = 0 if cos.is_inference() else cos._version
+        copy = getattr(self, "_fp32", None)
+        if copy is None or copy[0] is not cos or copy[1] != version:
+            copy = self._fp32 = (cos, version, cos.to(torch.float32))
+        return _lib.ROPE_COMPLEX_F64_APPROX, cos.data_ptr(), copy[2].data_ptr(), self.pairs_f, self.pairs_h
+
+
+_NO_ROPE = (_lib.ROPE_NONE, 0, 0, 0, 0)
+
+
+def _rope_args(rope: Optional[RopeTables]):
+    return _NO_ROPE if rope is None else rope.call_args()
 
 
 @dataclass
@@ -180,22 +200,18 @@ def rope_permute(x: torch.Tensor, order_ids: Optional[torch.Tensor], grid, n_tex
             raise ValueError("order_ids must hold one id per head")
     with torch.cuda.device(x.device):
         out = torch.empty(B, H, N, D, dtype=x.dtype, device=x.device)
-        r = rope
         if norm is not None:
             if inverse:
                 raise ValueError("the inverse permutation does not normalise")
             mode, w, b, inv, eps, _keep = _norm_call_args(norm, x)
             _lib.check(_lib.lib().paro_rope_permute_norm(
                 x.data_ptr(), out.data_ptr(), _lib.dtype_code(x.dtype), B, H, N, D, x.stride(0), x.stride(1), x.stride(2),
-                int(n_text), F, Hh, W, _lib.ptr(order_ids), r.mode if r is not None else _lib.ROPE_NONE,
-                _lib.ptr(r.cos if r else None), _lib.ptr(r.sin if r else None), r.pairs_f if r else 0,
-                r.pairs_h if r else 0, mode, _lib.ptr(w), _lib.ptr(b), _lib.ptr(inv), eps, _lib.stream_ptr()))
+                int(n_text), F, Hh, W, _lib.ptr(order_ids), *_rope_args(rope), mode, _lib.ptr(w), _lib.ptr(b), _lib.ptr(inv), eps, _lib.stream_ptr()))
             return out
         _lib.check(_lib.lib().paro_rope_permute(
             x.data_ptr(), out.data_ptr(), _lib.dtype_code(x.dtype), B, H, N, D, x.stride(0), x.stride(1), x.stride(2),
             int(n_text), F, Hh, W, _lib.ptr(order_ids), int(bool(inverse)),
-            r.mode if r is not None else _lib.ROPE_NONE, _lib.ptr(r.cos if r else None),
-            _lib.ptr(r.sin if r else None), r.pairs_f if r else 0, r.pairs_h if r else 0, _lib.stream_ptr()))
+            *_rope_args(rope), _lib.stream_ptr()))
     return out
 
 

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import paroatten_b200 as pb
+from paroatten_b200 import _lib
 from oracle import paro_oracle as po
 
 pytestmark = pytest.mark.gpu
@@ -278,3 +279,57 @@ def test_reference_default_block_sizes(N, D, dtype):
     assert qsb.shape == wsb.shape == (B, H, (N + 127) // 128)
     assert torch.equal(q8b.cpu(), w8b) and torch.equal(qsb.cpu(), wsb)
     assert torch.equal(k8b.cpu(), po.quant_int8(k, 64)[0]) and torch.equal(ksb.cpu(), po.quant_int8(k, 64)[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,pairs_f,pairs_h,scale", [(128, 22, 21, 1.0), (128, 5, 30, 300.0), (64, 0, 17, 1e-3), (64, 32, 0, 1.0)])
+def test_fp64_rotation_settled_in_fp32_has_the_fp64_bits(dtype, D, pairs_f, pairs_h, scale):
+    """The fp64 rotation is evaluated in fp32 where that settles the 16-bit result: the same bits as the fp64-only path
+    (separate tables) for axes that end inside a group of pairs, tables that are no unit rotations, and zeros, denormals,
+    Inf and NaN among the inputs; and the oracle's values."""
+    B, H, grid, n_text = 2, 6, (3, 7, 11), 13
+    N, half = n_text + grid[0] * grid[1] * grid[2], D // 2
+    g = torch.Generator().manual_seed(D + pairs_f)
+    x = (torch.randn(B, H, N, D, generator=g) * torch.randn(B, H, N, D, generator=g).mul(3).exp2()).to(dtype)
+    special = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), torch.finfo(dtype).max,
+                            torch.finfo(dtype).tiny / 8, -torch.finfo(dtype).tiny / 4]).to(dtype)
+    at = torch.rand(x.shape, generator=g) < 0.02
+    x[at] = special[torch.randint(0, len(special), (int(at.sum()),), generator=g)]
+    ang = torch.rand(sum(grid), half, dtype=torch.float64, generator=g) * 7
+    cos, sin = ang.cos() * scale, ang.sin() * scale
+    cos[0], sin[0] = 1.0, 0.0
+    ids = torch.tensor([0, 1, 2, 3, 4, 5], dtype=torch.int32, device=DEV)
+    tabs = pb.RopeTables(_lib.ROPE_COMPLEX_F64, cos.to(DEV), sin.to(DEV), pairs_f, pairs_h)
+    plain = pb.RopeTables(_lib.ROPE_COMPLEX_F64, cos.to(DEV), sin.to(DEV), pairs_f, pairs_h)
+    plain.cos, plain.sin = cos.to(DEV), sin.to(DEV)
+    assert tabs.call_args()[0] == _lib.ROPE_COMPLEX_F64_APPROX and plain.call_args()[0] == _lib.ROPE_COMPLEX_F64
+    got = pb.rope_permute(x.to(DEV), ids, grid, n_text, tabs)
+    assert torch.equal(got.view(torch.int16), pb.rope_permute(x.to(DEV), ids, grid, n_text, plain).view(torch.int16))
+    n = torch.arange(grid[0] * grid[1] * grid[2])
+    f, y, w = n // (grid[1] * grid[2]), n // grid[2] % grid[1], n % grid[2]
+    rows = [(f, 0, pairs_f), (grid[0] + y, pairs_f, pairs_f + pairs_h), (grid[0] + grid[1] + w, pairs_f + pairs_h, half)]
+    full = [torch.cat([t[r, a:b] for r, a, b in rows], dim=1) for t in (cos, sin)]
+    want = po.permute_tokens(po.apply_rope_complex(x, *full, n_text), list(range(6)), grid, n_text)
+    got = got.cpu()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num())
+    # a table that is written to afterwards is followed
+    tabs.cos.mul_(0.5)
+    plain.cos, plain.sin = plain.cos * 0.5, plain.sin * 0.5
+    assert torch.equal(pb.rope_permute(x.to(DEV), ids, grid, n_text, tabs).view(torch.int16),
+                       pb.rope_permute(x.to(DEV), ids, grid, n_text, plain).view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,H,N,D", [(1, 1, 1, 64), (1, 2, 63, 128), (1, 1, 257, 64), (2, 64, 2500, 64), (1, 48, 6401, 128)])
+def test_int8_blocks_per_cta(dtype, B, H, N, D):
+    """One 64-token block per CTA (small tensors) and four (large ones), with a ragged last block and a last CTA that is
+    not full: the oracle's bytes and scales."""
+    x = rand((B, H, N, D), dtype, N)
+    for group in (32, 64):
+        want, ws = po.quant_int8(x, group)
+        got = pb.quant._quant_int8(x.to(DEV), "HND", group)
+        assert torch.equal(got[0].cpu(), want) and torch.equal(got[1].cpu(), ws)
+    kp = pb.rope_permute(x.to(DEV), None, (1, N, 1))
+    assert torch.equal(kp.cpu(), x)
+    q8, qs, _ = pb.prep_qk_int8(x.to(DEV), None, (1, N, 1), group=32)
+    assert torch.equal(q8.cpu(), po.quant_int8(x, 32)[0])
