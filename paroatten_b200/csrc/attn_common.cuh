@@ -142,12 +142,12 @@ __device__ __forceinline__ uint32_t commit_token(uint32_t bars_saddr, int half, 
   return (bars_saddr + 32u * (uint32_t)half + 8u * ((uint32_t)step & 3u)) | ((((uint32_t)step >> 2) & 1u) << 31);
 }
 
-// paro_sparse_attn with a pinned host copy of the status words (nullable).
+// paro_sparse_attn with a pinned host copy of the status words (nullable); redo_is_zero: redo[0] has been cleared.
 int sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t* v16, const float* q_scale, int q_group,
                        const float* k_scale, const float* v_scale, const float* vm, const int32_t* pair_ptr,
                        const uint32_t* sched, const int32_t* sched_cnt, int plan_slices, const int32_t* inv_idx, int n_text,
                        void* out, int out_dtype, int64_t out_stride_b, int64_t out_stride_h, int64_t out_stride_n, float* lse,
                        int B, int H, int N, int D, float sm_scale, int mode, int32_t* redo, size_t redo_bytes,
-                       int32_t* status, int32_t* host_status, cudaStream_t s);
+                       int32_t* status, int32_t* host_status, bool redo_is_zero, cudaStream_t s);
 
 }  // namespace paro

@@ -37,7 +37,7 @@ Sections sections(const paro_layer_args& a) {
   s.kp = take(a.smooth_k ? rows * D * 2 : 0);
   s.rms_q = take(a.q_norm_mode == PARO_NORM_RMS_ALL ? (size_t)a.B * a.N * sizeof(float) : 0);
   s.rms_k = take(a.k_norm_mode == PARO_NORM_RMS_ALL ? (size_t)a.B * a.N * sizeof(float) : 0);
-  s.stats = take(paro_channel_stats_scratch_bytes(a.B, a.H, a.N, a.D));
+  s.stats = take(layer_kv_scratch_bytes(a.B, a.H, a.N, a.D));
   s.total = at;
   return s;
 }
@@ -63,7 +63,6 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
   uint16_t* v16 = reinterpret_cast<uint16_t*>(w + at.v16);
   float *qs = reinterpret_cast<float*>(w + at.qs), *ks = reinterpret_cast<float*>(w + at.ks);
   float *vs = reinterpret_cast<float*>(w + at.vs), *vm = reinterpret_cast<float*>(w + at.vm);
-  const size_t stats_bytes = at.total - at.stats;
 
   // the per-token statistic of an RMS norm over all heads
   auto inv_rms = [&](const void* x, const int64_t* st, int mode, float eps, size_t section, const float** out) -> int {
@@ -90,12 +89,12 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
   if (int rc = prep(a.q, a.q_strides, 32, a.q_norm_mode, a.q_norm_weight, a.q_norm_bias, rms, a.q_norm_eps, q8, qs)) return rc;
 
   if (int rc = inv_rms(a.k, a.k_strides, a.k_norm_mode, a.k_norm_eps, at.rms_k, &rms)) return rc;
+  void* kp = nullptr;   // K's rotated and reordered copy, where it is smoothed
   if (!a.smooth_k) {
     if (int rc = prep(a.k, a.k_strides, 64, a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, rms, a.k_norm_eps, k8, ks)) return rc;
   } else {
     // the mean to subtract is that of the rotated values, so the rotated copy is written once and read twice
-    void *kp = w + at.kp, *km = w + at.km;
-    const int64_t sn = a.D, sh = sn * a.N, sb = sh * a.H;
+    kp = w + at.kp;
     const int rc = a.k_norm_mode == PARO_NORM_NONE
         ? paro_rope_permute(a.k, kp, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2], a.n_text,
                             a.F, a.Hh, a.W, a.order_ids, 0, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, stream)
@@ -103,21 +102,16 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
                                  a.n_text, a.F, a.Hh, a.W, a.order_ids, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f,
                                  a.pairs_h, a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, rms, a.k_norm_eps, stream);
     if (rc) return rc;
-    if (int r = paro_channel_mean(kp, a.dtype, a.B, a.H, a.N, a.D, sb, sh, sn, km, nullptr, w + at.stats, stats_bytes, stream))
-      return r;
-    if (int r = paro_quant_int8(kp, a.dtype, a.B, a.H, a.N, a.D, sb, sh, sn, km, 0.f, 64, k8, ks, stream)) return r;
   }
-
-  if (int rc = paro_prep_v_fp8(a.v, a.dtype, a.B, a.H, a.N, a.D, a.v_strides[0], a.v_strides[1], a.v_strides[2], a.n_text,
-                               a.F, a.Hh, a.W, a.order_ids, a.smooth_v, 448.0f, nullptr, v16, vs, a.smooth_v ? vm : nullptr,
-                               w + at.stats, stats_bytes, stream))
-    return rc;
+  // (these passes clear the redo counter as well)
+  const bool fast = a.attn_mode == PARO_ATTN_FAST && a.redo && a.redo_bytes >= paro_sparse_attn_redo_bytes(a.B, a.H, a.N);
+  if (int rc = layer_kv_passes(a, kp, w + at.km, k8, ks, v16, vs, vm, w + at.stats, fast ? a.redo : nullptr, s)) return rc;
 
   if (a.ev_start) PARO_CUDA_OK(cudaEventRecord((cudaEvent_t)a.ev_start, s));
   if (int rc = sparse_attn_launch(q8, k8, v16, qs, 32, ks, vs, a.smooth_v ? vm : nullptr, a.pair_ptr, a.sched, a.sched_cnt,
                                   a.plan_slices, a.inv_idx, a.n_text, a.out, a.dtype, a.out_strides[0], a.out_strides[1],
                                   a.out_strides[2], a.lse, a.B, a.H, a.N, a.D, a.sm_scale, a.attn_mode, a.redo, a.redo_bytes,
-                                  a.status, a.host_status, s))
+                                  a.status, a.host_status, fast, s))
     return rc;
   if (a.ev_stop) PARO_CUDA_OK(cudaEventRecord((cudaEvent_t)a.ev_stop, s));
   return PARO_OK;

@@ -788,7 +788,8 @@ int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t*
                              const uint32_t* sched, const int32_t* sched_cnt, int plan_slices, const int32_t* inv_idx,
                              int n_text, void* out, int out_dtype, int64_t out_stride_b, int64_t out_stride_h,
                              int64_t out_stride_n, float* lse, int B, int H, int N, int D, float sm_scale, int mode,
-                             int32_t* redo, size_t redo_bytes, int32_t* status, int32_t* host_status, cudaStream_t s) {
+                             int32_t* redo, size_t redo_bytes, int32_t* status, int32_t* host_status,
+                             bool redo_is_zero, cudaStream_t s) {
   PARO_REQUIRE(q8 && k8 && v16 && q_scale && k_scale && v_scale && pair_ptr && sched && sched_cnt && out && status, PARO_EINVAL,
                "paro_sparse_attn: null pointer");
   PARO_REQUIRE(B > 0 && H > 0 && N > 0, PARO_ESHAPE, "paro_sparse_attn: empty problem");
@@ -820,7 +821,7 @@ int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t*
   if (mode == PARO_ATTN_EXACT) return launch_attn_exact(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
   // fixed-reference walk over every work item, then the exact walk over the items it gave back (usually none:
   // the second launch's CTAs then leave at once)
-  PARO_CUDA_OK(cudaMemsetAsync(redo, 0, sizeof(int32_t) * REDO_HEADER, s));
+  if (!redo_is_zero) PARO_CUDA_OK(cudaMemsetAsync(redo, 0, sizeof(int32_t) * REDO_HEADER, s));
   if (int rc = launch_attn_fixed(k8, v16, p, D, out_dtype, (unsigned)ctas, s)) return rc;
   p.from_list = 1;
   return launch_attn_exact(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
@@ -839,7 +840,7 @@ extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16
                                 int32_t* status, paro_stream_t stream) {
   return sparse_attn_launch(q8, k8, v16, q_scale, q_group, k_scale, v_scale, vm, pair_ptr, sched, sched_cnt, plan_slices,
                             inv_idx, n_text, out, out_dtype, out_stride_b, out_stride_h, out_stride_n, lse, B, H, N, D,
-                            sm_scale, mode, redo, redo_bytes, status, nullptr, (cudaStream_t)stream);
+                            sm_scale, mode, redo, redo_bytes, status, nullptr, false, (cudaStream_t)stream);
 }
 
 
