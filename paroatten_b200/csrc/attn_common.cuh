@@ -36,7 +36,6 @@ struct AttnParams {
   int64_t osb, osh, osn;
   int plan_slices, q_group, n_text;
   int B, H, N, npairs, nb;
-  int from_list;        // 1: work items are read from the redo list (second launch)
   float scale_log2;     // sm_scale * log2(e)
 };
 

@@ -101,14 +101,21 @@ template <int D> struct AttnCfg {
 //   no per-step maximum, no maximum handed between the warp sets, no accumulator read-modify-write.
 //   A step whose row sum leaves that range (or is not finite) makes the CTA give its work item back
 //   through the redo list instead of storing it; the exact walk then computes that pair.
-template <int D, typename OutT, bool FIXED>
+// LIST: the second launch of a call.  Its work items are the redo list, which is empty for nearly all inputs, so it
+// is a small grid whose CTAs walk the list in strides.  (One CTA per possible item costs 19 us for 2955 of them,
+// 70 us for 13344, 120 us for 23640, to find out that there is nothing to do.)
+template <int D, typename OutT, bool FIXED, bool LIST>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                          const AttnParams p) {
   using Cfg = AttnCfg<D>;
   constexpr int KST = Cfg::K_SLOTS, VST = Cfg::V_SLOTS;
-  // second launch of a call: only the work items the fixed-reference walk gave back
-  if (p.from_list && (int)blockIdx.x >= *reinterpret_cast<volatile int32_t*>(p.redo)) return;
+  static_assert(!(FIXED && LIST), "the redo list is for the exact walk");
+  [[maybe_unused]] int list_at = (int)blockIdx.x, list_len = 0;
+  if constexpr (LIST) {
+    list_len = *reinterpret_cast<volatile int32_t*>(p.redo);
+    if (list_at >= list_len) return;
+  }
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -146,26 +153,34 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   if (threadIdx.x == 0) *s_drain = *reinterpret_cast<volatile int32_t*>(p.status) != 0;
   __syncthreads();
   if (*s_drain) return;
-  const int item = p.from_list ? p.redo[REDO_HEADER + blockIdx.x] : (int)blockIdx.x;
-  const int bh = item / p.npairs, pair = item % p.npairs;
-  const int slice = bh % p.plan_slices;
   // The pair's schedule: entry i = kbA | kbB << 16 (0xFFFF: no tile for that half in step i).  First
   // the k-blocks both halves keep (kbA == kbB: one K/V tile, one full-height MMA group), then the
   // halves' remaining blocks side by side; each half's steps are contiguous from step 0.
-  const int prow = slice * p.npairs + pair;
-  const uint32_t* sched = p.sched + p.pair_ptr[prow];
-  // per half: steps in the low 16 bits; the high 16 bits are 0 (the pair is q-blocks 2p and 2p+1) or hold
+  // cnt, per half: steps in the low 16 bits; the high 16 bits are 0 (the pair is q-blocks 2p and 2p+1) or hold
   // 1 + the q-block the half stands for, when the plan paired q-blocks by the k-blocks they share
-  const uint32_t cnt_a = (uint32_t)p.sched_cnt[2 * prow], cnt_b = (uint32_t)p.sched_cnt[2 * prow + 1];
-  const int n_a = (int)(cnt_a & 0xFFFFu), n_b = (int)(cnt_b & 0xFFFFu);
-  const int n_steps = max(n_a, n_b);
+  int item, bh, pair, n_a, n_b, n_steps;
+  uint32_t cnt_a, cnt_b;
+  const uint32_t* sched;
+  auto set_item = [&](int it) {
+    item = it;
+    bh = item / p.npairs;
+    pair = item % p.npairs;
+    const int prow = (bh % p.plan_slices) * p.npairs + pair;
+    sched = p.sched + p.pair_ptr[prow];
+    cnt_a = (uint32_t)p.sched_cnt[2 * prow];
+    cnt_b = (uint32_t)p.sched_cnt[2 * prow + 1];
+    n_a = (int)(cnt_a & 0xFFFFu);
+    n_b = (int)(cnt_b & 0xFFFFu);
+    n_steps = max(n_a, n_b);
+  };
+  set_item(LIST ? p.redo[REDO_HEADER + list_at] : (int)blockIdx.x);
   // A step is one group of MMAs of each kind: FORM_UPPER / FORM_LOWER when only one half still has blocks (128
   // rows, the other half's accumulator rows masked), FORM_SHARED when both keep the same block (one tile, 128
   // rows) and FORM_DUAL when each half has its own (two tiles, tcgen05.mma.ws: two 64-row products in one
   // instruction).
   enum { FORM_UPPER = 0, FORM_LOWER = 1, FORM_SHARED = 2, FORM_DUAL = 3 };
 
-  if (threadIdx.x == 0) {
+  auto init_barriers = [&]() {
     mbar_init(bar_q, 4);
     for (int i = 0; i < KST; ++i) mbar_init(bar_kfull + i, 1);
     for (int i = 0; i < VST; ++i) mbar_init(bar_vfull + i, 1);
@@ -180,9 +195,12 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
     mbar_init(bar_drain, 1);
     mbar_init(bar_drain + 1, 1);
+    fence_barrier_init();
+  };
+  if (threadIdx.x == 0) {
     *abort_flag = 0;
     *s_redo = 0;
-    fence_barrier_init();
+    init_barriers();
   }
   if (warp == 10) {
     tmem_alloc(tmem_slot, TMEM_COLS);
@@ -194,8 +212,27 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS = tmem_base, tP = tmem_base + 64u, tQ = tmem_base + 96u, tO = tmem_base + 128u;
 
+  // LIST, all warps: on to the CTA's next item, false after the last one.  Every role has left the present item
+  // (its copies have landed and its MMAs have retired), so the barriers start over.
+  auto next_item = [&]() -> bool {
+    if constexpr (!LIST) return false;
+    tc_fence_before();
+    __syncthreads();
+    list_at += (int)gridDim.x;
+    if (*abort_flag || list_at >= list_len) return false;
+    if (threadIdx.x == 0) {
+      for (uint64_t* bar = bar_q; bar < bar_drain + 2; ++bar) mbar_inval(bar);
+      init_barriers();
+    }
+    set_item(p.redo[REDO_HEADER + list_at]);
+    __syncthreads();
+    tc_fence_after();
+    return true;
+  };
+
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    do {
     if (warp <= 9 && lane == 0) {
       // ---------------------------------------------------------------- TMA producers: K ring (warp 8), V ring (warp 9)
       auto produce = [&](auto ktag, const CUtensorMap* tm, uint8_t* ring, uint64_t* bar_full, uint64_t* bar_done) {
@@ -405,9 +442,12 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         mbar_wait_plain_bounded(bar_drain + 1, 0, WAIT_LIMIT);
       }
     }
+    __syncwarp();
+    } while (next_item());
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    do {
     const int qd = warp & 3;                 // TMEM lane quadrant this warp may touch
     const int set = warp >> 2;               // warp set: steps of this parity; also which half of O's columns
     const int r = qd * 32 + lane;            // row inside the 128-row tile
@@ -693,6 +733,7 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if (live && set == 0 && p.lse)
         p.lse[(size_t)bh * p.N + dst] = l > 0.f ? (log2f(l) + m) * 0.6931471805599453f : -INFINITY;
     }
+    } while (next_item());
   }
 
   tc_fence_before();
@@ -736,7 +777,7 @@ static int make_tensor_map(CUtensorMap* map, CUtensorMapDataType dt, int esize, 
   return PARO_OK;
 }
 
-template <int D, typename OutT, bool FIXED>
+template <int D, typename OutT, bool FIXED, bool LIST = false>
 static int launch_walk(const int8_t* k8, const uint16_t* v16, const AttnParams& p, unsigned ctas, cudaStream_t s) {
   using Cfg = AttnCfg<D>;
   const uint64_t BH = (uint64_t)p.B * p.H;
@@ -746,7 +787,7 @@ static int launch_walk(const int8_t* k8, const uint16_t* v16, const AttnParams& 
   if (int rc = make_tensor_map(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k8, D, p.N, BH, D, 64, swz_qk)) return rc;
   if (int rc = make_tensor_map(&tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, v16, npad, D, BH, 64, D, CU_TENSOR_MAP_SWIZZLE_128B))
     return rc;
-  auto kern = sparse_attn_kernel<D, OutT, FIXED>;
+  auto kern = sparse_attn_kernel<D, OutT, FIXED, LIST>;
   PARO_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
   // shared memory for two CTAs per SM and no more: the rest of the 256 KB serves as L1
   constexpr int carveout_pct = (2 * (Cfg::SMEM_BYTES + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024);
@@ -755,13 +796,14 @@ static int launch_walk(const int8_t* k8, const uint16_t* v16, const AttnParams& 
   return check_launch("sparse_attn_kernel");
 }
 
+template <bool LIST>
 static int launch_attn_exact(const int8_t* k8, const uint16_t* v16, const AttnParams& p, int D, int out_dtype, unsigned ctas,
                       cudaStream_t s) {
   if (D == 128)
-    return out_dtype == PARO_F16 ? launch_walk<128, __half, false>(k8, v16, p, ctas, s)
-                                 : launch_walk<128, __nv_bfloat16, false>(k8, v16, p, ctas, s);
-  return out_dtype == PARO_F16 ? launch_walk<64, __half, false>(k8, v16, p, ctas, s)
-                               : launch_walk<64, __nv_bfloat16, false>(k8, v16, p, ctas, s);
+    return out_dtype == PARO_F16 ? launch_walk<128, __half, false, LIST>(k8, v16, p, ctas, s)
+                                 : launch_walk<128, __nv_bfloat16, false, LIST>(k8, v16, p, ctas, s);
+  return out_dtype == PARO_F16 ? launch_walk<64, __half, false, LIST>(k8, v16, p, ctas, s)
+                               : launch_walk<64, __nv_bfloat16, false, LIST>(k8, v16, p, ctas, s);
 }
 
 static int launch_attn_fixed(const int8_t* k8, const uint16_t* v16, const AttnParams& p, int D, int out_dtype, unsigned ctas,
@@ -814,17 +856,15 @@ int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t*
   p.osb = out_stride_b; p.osh = out_stride_h; p.osn = out_stride_n;
   p.plan_slices = plan_slices; p.q_group = q_group; p.n_text = n_text;
   p.B = B; p.H = H; p.N = N; p.nb = (N + 63) / 64; p.npairs = (p.nb + 1) / 2;
-  p.from_list = 0;
   p.scale_log2 = sm_scale * 1.44269504f;
   const uint64_t ctas = (uint64_t)B * H * p.npairs;
   PARO_REQUIRE(ctas < (1ull << 31), PARO_ESHAPE, "paro_sparse_attn: too many work items");
-  if (mode == PARO_ATTN_EXACT) return launch_attn_exact(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
-  // fixed-reference walk over every work item, then the exact walk over the items it gave back (usually none:
-  // the second launch's CTAs then leave at once)
+  if (mode == PARO_ATTN_EXACT) return launch_attn_exact<false>(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
+  // fixed-reference walk over every work item, then the exact walk over the items it gave back (usually none):
+  // as many CTAs as fit the chip at two per SM
   if (!redo_is_zero) PARO_CUDA_OK(cudaMemsetAsync(redo, 0, sizeof(int32_t) * REDO_HEADER, s));
   if (int rc = launch_attn_fixed(k8, v16, p, D, out_dtype, (unsigned)ctas, s)) return rc;
-  p.from_list = 1;
-  return launch_attn_exact(k8, v16, p, D, out_dtype, (unsigned)ctas, s);
+  return launch_attn_exact<true>(k8, v16, p, D, out_dtype, (unsigned)(ctas < 296 ? ctas : 296), s);
 }
 
 extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16_t* v16,
