@@ -88,24 +88,36 @@ int launch_rope(const void* in, void* out, int B, int H, int N, int D, int64_t s
 #undef PARO_ROPE_CASE
 }
 
-// One warp per token: sum of squares over all H*D channels in fp64.
-template <typename T>
+// One warp per token: sum of squares over all H*D channels in fp64.  HBM-bound (2 bytes per element); RMS_LOADS
+// 16-byte loads in flight per thread: 48 -> 41.5 us for 2 x 32760 tokens of 12 x 128 channels (one load at a time before).
+constexpr int RMS_LOADS = 4;
+template <typename T, int D>
 __global__ void __launch_bounds__(256)
-row_inv_rms_kernel(const T* __restrict__ x, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn, float eps,
+row_inv_rms_kernel(const T* __restrict__ x, int H, int N, int64_t sb, int64_t sh, int64_t sn, float eps,
                    float* __restrict__ inv_rms, int rows) {
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const int b = row / N, n = row % N;
   const T* base = x + b * sb + (size_t)n * sn;
-  const int per_head = D / 8;   // 16-byte pieces per head
+  constexpr int PER_HEAD = D / 8;   // 16-byte pieces per head
+  const int pieces = H * PER_HEAD;
   double s = 0.0;
-  for (int i = lane; i < H * per_head; i += 32) {
-    Pack8<T> v;
-    v.v = *reinterpret_cast<const uint4*>(base + (size_t)(i / per_head) * sh + (i % per_head) * 8);
+  for (int i0 = lane; i0 < pieces; i0 += 32 * RMS_LOADS) {
+    Pack8<T> v[RMS_LOADS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float f = F16Traits<T>::to_float(v.e[j]);
-      s += (double)__fmul_rn(f, f);   // exact: 16 significant bits
+    for (int u = 0; u < RMS_LOADS; ++u) {
+      const int i = i0 + 32 * u;
+      v[u].v = make_uint4(0, 0, 0, 0);   // (zeros add nothing)
+      if (i < pieces) v[u].v = *reinterpret_cast<const uint4*>(base + (size_t)(i / PER_HEAD) * sh + (i % PER_HEAD) * 8);
+    }
+#pragma unroll
+    for (int u = 0; u < RMS_LOADS; ++u) {
+      if (i0 - lane + 32 * u >= pieces) break;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float f = F16Traits<T>::to_float(v[u].e[j]);
+        s += (double)__fmul_rn(f, f);   // exact: 16 significant bits
+      }
     }
   }
 #pragma unroll
@@ -173,11 +185,14 @@ extern "C" int paro_row_inv_rms(const void* x, int dtype, int B, int H, int N, i
   PARO_REQUIRE(rows <= 0x7fffffffLL, PARO_ESHAPE, "paro_row_inv_rms: too many rows");
   cudaStream_t s = (cudaStream_t)stream;
   const unsigned grid = (unsigned)((rows + 7) / 8);
-  if (dtype == PARO_F16)
-    row_inv_rms_kernel<__half><<<grid, 256, 0, s>>>((const __half*)x, H, N, D, stride_b, stride_h, stride_n, eps, inv_rms,
-                                                    (int)rows);
-  else
-    row_inv_rms_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, H, N, D, stride_b, stride_h, stride_n,
-                                                           eps, inv_rms, (int)rows);
+  auto launch = [&](auto tag, auto d) {
+    using T = decltype(tag);
+    row_inv_rms_kernel<T, decltype(d)::value><<<grid, 256, 0, s>>>((const T*)x, H, N, stride_b, stride_h, stride_n, eps, inv_rms,
+                                                                  (int)rows);
+  };
+  using D64 = std::integral_constant<int, 64>;
+  using D128 = std::integral_constant<int, 128>;
+  if (dtype == PARO_F16) D == 128 ? launch(__half(), D128()) : launch(__half(), D64());
+  else D == 128 ? launch(__nv_bfloat16(), D128()) : launch(__nv_bfloat16(), D64());
   return check_launch("row_inv_rms_kernel");
 }
