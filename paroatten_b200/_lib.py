@@ -5,6 +5,7 @@ package raises.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import shutil
@@ -180,6 +181,12 @@ def dtype_code(dt) -> int:
     if dt == torch.bfloat16:
         return BF16
     raise ValueError(f"unsupported dtype {dt}: fp16 or bf16 expected")
+
+
+def on_device(device):
+    """torch.cuda.device(device), or nothing to enter when it is the current device already."""
+    import torch
+    return contextlib.nullcontext() if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def stream_ptr() -> int:

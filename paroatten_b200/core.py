@@ -1,7 +1,6 @@
 """Sparse-attention entry points (reference: paroattention/core.py)."""
 from __future__ import annotations
 
-import contextlib
 import ctypes
 from typing import Any, Optional, Sequence, Tuple, Union
 
@@ -152,11 +151,6 @@ def sparse_attn_quantized(q_int8, q_scale, k_int8, k_scale, v16, v_scale, vm, pl
             sink.append(ev)
         _mirror(dev).copy_(_status_words(dev), non_blocking=True)
     return (out, lse) if return_lse else out
-
-
-def _on(device: torch.device):
-    """torch.cuda.device(device), or nothing to enter when it is the current device already."""
-    return contextlib.nullcontext() if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _layer(q, k, v, orders, index, plan: CompactPlan, grid, n_text: int, rope: Optional[RopeTables], tensor_layout: str,
@@ -352,7 +346,7 @@ def paro_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, permute_pl
     if sm_scale is None:
         sm_scale = head_dim_og ** -0.5
     dev = q.device
-    with _on(dev):
+    with _lib.on_device(dev):
         empty = None
         if isinstance(permute_plan, PermutePlan):
             orders, index = permute_plan.orders(i_block), permute_plan.index(i_block)

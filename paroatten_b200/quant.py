@@ -39,7 +39,7 @@ def channel_mean(x: torch.Tensor, tensor_layout: str = "HND", out_dtype=None) ->
     xv = _hnd(x, tensor_layout)
     B, H, N, D = xv.shape
     f32 = out_dtype == torch.float32
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         out = torch.empty(B, H, D, dtype=torch.float32 if f32 else x.dtype, device=x.device)
         scr = _stats_scratch(B, H, N, D, x.device)
         _lib.check(_lib.lib().paro_channel_mean(
@@ -54,7 +54,7 @@ def _quant_int8(x, tensor_layout, group, km=None, fold=0.0):
     xv = _hnd(x, tensor_layout)
     B, H, N, D = xv.shape
     nb = (N + 63) // 64
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         out = torch.empty(B, H, N, D, dtype=torch.int8, device=x.device)
         scale = torch.empty(B, H, nb * (64 // group), dtype=torch.float32, device=x.device)
         if km is not None:
@@ -153,7 +153,7 @@ def per_channel_fp8(v: torch.Tensor, tensor_layout: str = "HND", scale_max: floa
     vv = _hnd(v, tensor_layout)
     B, H, N, D = vv.shape
     npad = (N + 63) // 64 * 64
-    with torch.cuda.device(v.device):
+    with _lib.on_device(v.device):
         v8 = torch.empty(B, H, D, npad, dtype=torch.float8_e4m3fn, device=v.device)
         v16 = torch.empty(B, H, D, npad, dtype=torch.bfloat16, device=v.device) if return_16 else None
         scale = torch.empty(B, H, D, dtype=torch.float32, device=v.device)
@@ -179,7 +179,7 @@ def prep_qk_int8(x: torch.Tensor, order_ids: Optional[torch.Tensor], grid, n_tex
     B, H, N, D = xv.shape
     nb = (N + 63) // 64
     F, Hh, W = (int(g) for g in grid)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         if order_ids is not None:
             order_ids = order_ids.to(device=x.device, dtype=torch.int32).contiguous()
         out = torch.empty(B, H, N, D, dtype=torch.int8, device=x.device)
@@ -214,7 +214,7 @@ def prep_v_fp8(v: torch.Tensor, order_ids: Optional[torch.Tensor], grid, n_text:
     B, H, N, D = vv.shape
     npad = (N + 63) // 64 * 64
     F, Hh, W = (int(g) for g in grid)
-    with torch.cuda.device(v.device):
+    with _lib.on_device(v.device):
         if order_ids is not None:
             order_ids = order_ids.to(device=v.device, dtype=torch.int32).contiguous()
         v16 = torch.empty(B, H, D, npad, dtype=torch.bfloat16, device=v.device)

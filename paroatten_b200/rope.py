@@ -198,7 +198,7 @@ def rope_permute(x: torch.Tensor, order_ids: Optional[torch.Tensor], grid, n_tex
         order_ids = order_ids.to(device=x.device, dtype=torch.int32).contiguous()
         if order_ids.numel() != H:
             raise ValueError("order_ids must hold one id per head")
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         out = torch.empty(B, H, N, D, dtype=x.dtype, device=x.device)
         if norm is not None:
             if inverse:
