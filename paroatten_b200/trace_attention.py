@@ -8,9 +8,9 @@ attention call three times on the named bench workload, reads the table back and
 role's clocks of a step go.  The shipped library is untouched and contains none of this.
 
 Table layout [role][step][event] (int64 SM clocks, 0 = not reached):
-  role 0 / 1   K / V producer       events 2j: waiting for a free stage, 2j+1: copy issued (j = tile of the step)
-  role 2 / 3   Q.K^T / P.V issuer   per tile (offset 0 or 4): 0 polling, 1 barriers complete, 3 MMAs and commit issued
-                                    (a side-by-side step issued in one burst: 0, 1, 3 = first tile done, 7 = done)
+  role 0 / 1   K / V producer       0 waiting for a free slot, 1 the step's copies issued
+  role 2 / 3   Q.K^T / P.V issuer   0 polling, 1 barriers complete, 3 MMAs and commits issued (events 4-7: a second tile
+                                    issued by itself, which the kernel no longer does)
   role 4 + w   softmax warp w       0 waiting for scores, 1 scores ready, 2 scores in registers (S released),
                                     3 exponentials done, 4 previous P.V seen finished, 5 P written and announced
 """
