@@ -64,7 +64,7 @@ int paro_build_perm_index(const int32_t* order_ids, int H, int F, int Hh, int W,
  * sin_tab == NULL (all entry points that take the two tables): cos_tab is then ONE table
  * [F+Hh+W, D/2, 2] with cos and sin of a pair side by side, fetched by a single load.
  * PARO_ROPE_COMPLEX_F64_APPROX: the same results as PARO_ROPE_COMPLEX_F64, faster; cos_tab is the interleaved fp64 table
- * and sin_tab (16-byte aligned) the same table rounded to fp32.
+ * and sin_tab (16-byte aligned) the same table rounded to fp32 (paro_layer makes that copy itself, in every call).
  * Replaces csrc/rope/rope.cu:14-48 (rope_permutation) and permute_qk / permute_attn_out
  * (cogvideox.py:22-110). */
 int paro_rope_permute(const void* in, void* out, int dtype, int B, int H, int N, int D,

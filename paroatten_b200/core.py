@@ -10,7 +10,7 @@ import torch.nn.functional as F
 from . import _lib
 from .plan import (CompactPlan, PermutePlan, PlanStore, SparsePlan, apply_empty_heads, compact_plan, perm_index)
 from .quant import _hnd, channel_mean, per_channel_fp8, per_warp_int8, per_block_int8
-from .rope import RopeTables, _norm_params, _rope_args
+from .rope import RopeTables, _NO_ROPE, _norm_params
 
 _status = {}
 _status_mirror = {}   # device index -> pinned host copy of the status words, refreshed after every launch
@@ -187,7 +187,7 @@ def _layer(q, k, v, orders, index, plan: CompactPlan, grid, n_text: int, rope: O
         for e in ev:
             e.record()       # (creates the event; the call below records both again where they belong)
     cnt = plan.sched_cnt_kernel if plan.sched_cnt_kernel is not None else plan.sched_cnt
-    rope_mode, cos, sin, pairs_f, pairs_h = _rope_args(rope)
+    rope_mode, cos, sin, pairs_f, pairs_h = _NO_ROPE if rope is None else rope.table_args()
     three = ctypes.c_int64 * 3
     a = _lib.LayerArgs(
         qv.data_ptr(), kv.data_ptr(), vv.data_ptr(), three(*qv.stride()[:3]), three(*kv.stride()[:3]),

@@ -8,6 +8,7 @@
 // share their statistics launches and the passes themselves became shorter.
 #include "attn_common.cuh"
 #include "common.cuh"
+#include "rope.cuh"
 
 using namespace paro;
 
@@ -15,8 +16,18 @@ namespace {
 
 // Sections of the work space, each on a 256-byte boundary.
 struct Sections {
-  size_t q8, k8, v16, qs, ks, vs, vm, km, kp, rms_q, rms_k, stats, total;
+  size_t q8, k8, v16, qs, ks, vs, vm, km, kp, rms_q, rms_k, tab32, stats, total;
 };
+
+// Elements of Q from which the passes get the fp32 copy of an interleaved fp64 table, made for the call: 2 us, which Q
+// and K of 2 x 12 x 1560 x 128 give back twice over (bf16: 29.6 -> 24.9 us) and those of 3 x 4200 x 128 do not (18.2 ->
+// 17.0).
+constexpr int64_t FP32_TABLE_ELEMS = 4 << 20;
+bool fp32_table(const paro_layer_args& a) {
+  return a.rope_mode == PARO_ROPE_COMPLEX_F64 && a.cos_tab && !a.sin_tab && a.F > 0 && a.Hh > 0 && a.W > 0 &&
+         (int64_t)a.B * a.H * a.N * a.D >= FP32_TABLE_ELEMS;
+}
+int64_t table_pairs(const paro_layer_args& a) { return ((int64_t)a.F + a.Hh + a.W) * (a.D / 2); }
 
 Sections sections(const paro_layer_args& a) {
   const size_t BH = (size_t)a.B * a.H, rows = BH * a.N, D = a.D, nb = ((size_t)a.N + 63) / 64;
@@ -38,6 +49,7 @@ Sections sections(const paro_layer_args& a) {
   s.kp = take(a.smooth_k ? rows * D * 2 : 0);
   s.rms_q = take(a.q_norm_mode == PARO_NORM_RMS_ALL ? (size_t)a.B * a.N * sizeof(float) : 0);
   s.rms_k = take(a.k_norm_mode == PARO_NORM_RMS_ALL ? (size_t)a.B * a.N * sizeof(float) : 0);
+  s.tab32 = take(fp32_table(a) ? table_pairs(a) * sizeof(float2) : 0);
   s.stats = take(layer_kv_scratch_bytes(a.B, a.H, a.N, a.D));
   s.total = at;
   return s;
@@ -65,6 +77,22 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
   float *qs = reinterpret_cast<float*>(w + at.qs), *ks = reinterpret_cast<float*>(w + at.ks);
   float *vs = reinterpret_cast<float*>(w + at.vs), *vm = reinterpret_cast<float*>(w + at.vm);
 
+  // arguments of every pass, before the first of them
+  if (int rc = check_tensor("paro_layer(q)", a.q, a.dtype, a.B, a.H, a.N, a.D, a.q_strides[0], a.q_strides[1], a.q_strides[2])) return rc;
+  if (int rc = check_tensor("paro_layer(k)", a.k, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2])) return rc;
+  if (int rc = check_tensor("paro_layer(v)", a.v, a.dtype, a.B, a.H, a.N, a.D, a.v_strides[0], a.v_strides[1], a.v_strides[2])) return rc;
+  PARO_REQUIRE(a.F > 0 && a.Hh > 0 && a.W > 0 && a.n_text >= 0 && (int64_t)a.n_text + (int64_t)a.F * a.Hh * a.W == a.N,
+               PARO_ESHAPE, "paro_layer: n_text + F*H*W = %lld != N = %d", (long long)a.n_text + (long long)a.F * a.Hh * a.W, a.N);
+  if (int rc = check_rope("paro_layer", a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, a.D)) return rc;
+
+  int rope_mode = a.rope_mode;
+  const void* sin_tab = a.sin_tab;
+  if (fp32_table(a)) {
+    rope_mode = PARO_ROPE_COMPLEX_F64_APPROX;
+    sin_tab = w + at.tab32;
+    if (int rc = launch_round_table(a.cos_tab, w + at.tab32, table_pairs(a), s)) return rc;
+  }
+
   // the per-token statistic of an RMS norm over all heads
   auto inv_rms = [&](const void* x, const int64_t* st, int mode, float eps, size_t section, const float** out) -> int {
     *out = nullptr;
@@ -78,10 +106,10 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
                   const float* rms, float eps, int8_t* out, float* scale) -> int {
     if (norm != PARO_NORM_NONE)
       return paro_prep_qk_int8_norm(x, a.dtype, a.B, a.H, a.N, a.D, st[0], st[1], st[2], a.n_text, a.F, a.Hh, a.W,
-                                    a.order_ids, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, group, out, scale,
+                                    a.order_ids, rope_mode, a.cos_tab, sin_tab, a.pairs_f, a.pairs_h, group, out, scale,
                                     norm, weight, bias, rms, eps, stream);
     return paro_prep_qk_int8(x, a.dtype, a.B, a.H, a.N, a.D, st[0], st[1], st[2], a.n_text, a.F, a.Hh, a.W, a.order_ids,
-                             a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, group, 0, nullptr, out, scale,
+                             rope_mode, a.cos_tab, sin_tab, a.pairs_f, a.pairs_h, group, 0, nullptr, out, scale,
                              nullptr, 0, stream);
   };
 
@@ -100,9 +128,9 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
     kp = w + at.kp;
     const int rc = a.k_norm_mode == PARO_NORM_NONE
         ? paro_rope_permute(a.k, kp, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2], a.n_text,
-                            a.F, a.Hh, a.W, a.order_ids, 0, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, stream)
+                            a.F, a.Hh, a.W, a.order_ids, 0, rope_mode, a.cos_tab, sin_tab, a.pairs_f, a.pairs_h, stream)
         : paro_rope_permute_norm(a.k, kp, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2],
-                                 a.n_text, a.F, a.Hh, a.W, a.order_ids, a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f,
+                                 a.n_text, a.F, a.Hh, a.W, a.order_ids, rope_mode, a.cos_tab, sin_tab, a.pairs_f,
                                  a.pairs_h, a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, rms, a.k_norm_eps, stream);
     if (rc) return rc;
   }

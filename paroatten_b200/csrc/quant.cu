@@ -801,8 +801,6 @@ size_t paro::layer_kv_scratch_bytes(int B, int H, int N, int D) {
 
 int paro::layer_kv_passes(const paro_layer_args& a, const void* kp, void* km, int8_t* k8, float* ks, uint16_t* v16, float* vs,
                           float* vm, void* scratch, int32_t* zero_word, cudaStream_t s) {
-  if (int rc = check_tensor("paro_layer(v)", a.v, a.dtype, a.B, a.H, a.N, a.D, a.v_strides[0], a.v_strides[1], a.v_strides[2]))
-    return rc;
   Gather g{};
   if (int rc = make_gather(&g, "paro_layer", a.N, a.D, a.n_text, a.F, a.Hh, a.W, a.order_ids, PARO_ROPE_NONE, nullptr, nullptr,
                            0, 0))

@@ -29,6 +29,9 @@ inline RopeArgs make_rope(int mode, const void* cos_tab, const void* sin_tab, in
   return r;
 }
 
+// Rounds an interleaved fp64 table [rows, D/2, 2] to fp32 (rope_permute.cu): the tab32 of paro_layer's passes.
+int launch_round_table(const void* tab64, void* tab32, int64_t pairs, cudaStream_t s);
+
 // Arguments common to the entry points that rotate.
 inline int check_rope(const char* who, int mode, const void* cos_tab, const void* sin_tab, int pairs_f, int pairs_h, int D) {
   PARO_REQUIRE(mode >= PARO_ROPE_NONE && mode <= PARO_ROPE_COMPLEX_F64_APPROX, PARO_EINVAL, "%s: unknown rope_mode %d", who, mode);

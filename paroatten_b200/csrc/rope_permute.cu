@@ -88,6 +88,20 @@ int launch_rope(const void* in, void* out, int B, int H, int N, int D, int64_t s
 #undef PARO_ROPE_CASE
 }
 
+__global__ void __launch_bounds__(256)
+round_table_kernel(const double2* __restrict__ tab64, float2* __restrict__ tab32, int64_t pairs) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= pairs) return;
+  const double2 cs = tab64[i];
+  tab32[i] = make_float2(__double2float_rn(cs.x), __double2float_rn(cs.y));
+}
+
+int launch_round_table(const void* tab64, void* tab32, int64_t pairs, cudaStream_t s) {
+  round_table_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(static_cast<const double2*>(tab64),
+                                                                     static_cast<float2*>(tab32), pairs);
+  return check_launch("round_table_kernel");
+}
+
 // One warp per token: sum of squares over all H*D channels in fp64.  HBM-bound (2 bytes per element); RMS_LOADS
 // 16-byte loads in flight per thread: 48 -> 41.5 us for 2 x 32760 tokens of 12 x 128 channels (one load at a time before).
 constexpr int RMS_LOADS = 4;

@@ -186,19 +186,20 @@ def prep_qk_int8(x: torch.Tensor, order_ids: Optional[torch.Tensor], grid, n_tex
         scale = torch.empty(B, H, nb * (64 // group), dtype=torch.float32, device=x.device)
         km = torch.empty(B, H, D, dtype=x.dtype, device=x.device) if smooth else None
         scr = _stats_scratch(B, H, N, D, x.device) if smooth else None
+        angles, _table = _rope_args(rope, xv.numel())
         if norm is not None:
             if smooth:
                 raise ValueError("prep_qk_int8: norm and smooth cannot be combined (use rope_permute(norm=...) first)")
             mode, w, b, inv, eps, _keep = _norm_call_args(norm, xv)
             _lib.check(_lib.lib().paro_prep_qk_int8_norm(
                 xv.data_ptr(), _lib.dtype_code(x.dtype), B, H, N, D, xv.stride(0), xv.stride(1), xv.stride(2),
-                int(n_text), F, Hh, W, _lib.ptr(order_ids), *_rope_args(rope),
+                int(n_text), F, Hh, W, _lib.ptr(order_ids), *angles,
                 int(group), out.data_ptr(), scale.data_ptr(),
                 mode, _lib.ptr(w), _lib.ptr(b), _lib.ptr(inv), eps, _lib.stream_ptr()))
             return out, scale, None
         _lib.check(_lib.lib().paro_prep_qk_int8(
             xv.data_ptr(), _lib.dtype_code(x.dtype), B, H, N, D, xv.stride(0), xv.stride(1), xv.stride(2),
-            int(n_text), F, Hh, W, _lib.ptr(order_ids), *_rope_args(rope),
+            int(n_text), F, Hh, W, _lib.ptr(order_ids), *angles,
             int(group), int(bool(smooth)), _lib.ptr(km), out.data_ptr(), scale.data_ptr(),
             _lib.ptr(scr), scr.numel() if scr is not None else 0, _lib.stream_ptr()))
     return out, scale, km

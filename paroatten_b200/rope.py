@@ -21,26 +21,36 @@ class RopeTables:
         self.cos = torch.stack([cos, sin], dim=-1).contiguous()
         self.sin = None
         self.pairs_f, self.pairs_h = pairs_f, pairs_h
-        self.call_args()            # (the fp32 copy belongs to the stream that makes the table, not to its first user's)
+
+    def table_args(self):
+        """(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h) of an entry point that reads the tables themselves."""
+        return self.mode, self.cos.data_ptr(), _lib.ptr(self.sin), self.pairs_f, self.pairs_h
 
     def call_args(self):
-        """(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h) of an entry point.  An fp64 table goes with its fp32 copy
-        (PARO_ROPE_COMPLEX_F64_APPROX); the copy is made again when the table has been written to or replaced."""
-        cos, sin = self.cos, self.sin
-        if self.mode != _lib.ROPE_COMPLEX_F64 or sin is not None or cos.dtype != torch.float64:
-            return self.mode, cos.data_ptr(), _lib.ptr(sin), self.pairs_f, self.pairs_h
-        version = 0 if cos.is_inference() else cos._version
-        copy = getattr(self, "_fp32", None)
-        if copy is None or copy[0] is not cos or copy[1] != version:
-            copy = self._fp32 = (cos, version, cos.to(torch.float32))
-        return _lib.ROPE_COMPLEX_F64_APPROX, cos.data_ptr(), copy[2].data_ptr(), self.pairs_f, self.pairs_h
+        """The same for an entry point that also takes an fp64 table's fp32 copy (PARO_ROPE_COMPLEX_F64_APPROX), and
+        that copy, which has to outlive the launch.  It is made for the call and on the call's stream: whatever has
+        been written to the table in stream order before the call, by whatever means, is in it."""
+        cos = self.cos
+        if self.mode != _lib.ROPE_COMPLEX_F64 or self.sin is not None or cos.dtype != torch.float64:
+            return (*self.table_args(), None)
+        copy = cos.to(torch.float32)
+        return _lib.ROPE_COMPLEX_F64_APPROX, cos.data_ptr(), copy.data_ptr(), self.pairs_f, self.pairs_h, copy
 
 
 _NO_ROPE = (_lib.ROPE_NONE, 0, 0, 0, 0)
 
+# Elements of a tensor from which a pass over it takes the fp32 copy of an fp64 table along.  Making the copy costs 2 us on
+# the device and 6 on the host; it takes 2 us off a pass over 5 million elements (2 x 12 x 1560 x 128, INT8 Q in bf16:
+# 16.6 -> 14.5 us) and 8 us off one over 24 million (40 x 4680 x 128: 46.5 -> 38.5 us).
+FP32_COPY_ELEMS = 16 << 20
 
-def _rope_args(rope: Optional[RopeTables]):
-    return _NO_ROPE if rope is None else rope.call_args()
+
+def _rope_args(rope: Optional[RopeTables], numel: int):
+    """(the five arguments of a pass over `numel` elements, a tensor to hold until it is launched)"""
+    if rope is None:
+        return _NO_ROPE, None
+    args = rope.call_args() if numel >= FP32_COPY_ELEMS else (*rope.table_args(), None)
+    return args[:5], args[5]
 
 
 @dataclass
@@ -200,18 +210,19 @@ def rope_permute(x: torch.Tensor, order_ids: Optional[torch.Tensor], grid, n_tex
             raise ValueError("order_ids must hold one id per head")
     with _lib.on_device(x.device):
         out = torch.empty(B, H, N, D, dtype=x.dtype, device=x.device)
+        angles, _table = _rope_args(rope, x.numel())
         if norm is not None:
             if inverse:
                 raise ValueError("the inverse permutation does not normalise")
             mode, w, b, inv, eps, _keep = _norm_call_args(norm, x)
             _lib.check(_lib.lib().paro_rope_permute_norm(
                 x.data_ptr(), out.data_ptr(), _lib.dtype_code(x.dtype), B, H, N, D, x.stride(0), x.stride(1), x.stride(2),
-                int(n_text), F, Hh, W, _lib.ptr(order_ids), *_rope_args(rope), mode, _lib.ptr(w), _lib.ptr(b), _lib.ptr(inv), eps, _lib.stream_ptr()))
+                int(n_text), F, Hh, W, _lib.ptr(order_ids), *angles, mode, _lib.ptr(w), _lib.ptr(b), _lib.ptr(inv), eps, _lib.stream_ptr()))
             return out
         _lib.check(_lib.lib().paro_rope_permute(
             x.data_ptr(), out.data_ptr(), _lib.dtype_code(x.dtype), B, H, N, D, x.stride(0), x.stride(1), x.stride(2),
             int(n_text), F, Hh, W, _lib.ptr(order_ids), int(bool(inverse)),
-            *_rope_args(rope), _lib.stream_ptr()))
+            *angles, _lib.stream_ptr()))
     return out
 
 
