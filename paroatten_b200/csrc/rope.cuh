@@ -100,13 +100,14 @@ __device__ __forceinline__ uint32_t rotate_pair_f32(float x0, float x1, float c,
 // most 3 * 2^-24 * (|x0|+|x1|) * (|c|+|s|); e is twice that (the rounding of r-e, r+e itself included), 2^-100 and
 // 2^-140 cover table entries and products below the normal range.  Rounding is monotonic: where r-e and r+e round to
 // the same 16-bit value the fp64 result between them does too.  Uncertain are about one value in 2^13 for bf16 and
-// 2^10 for fp16, and zeros, Inf and NaN.
+// 2^10 for fp16, zeros, and everything whose e is not finite: an Inf or NaN operand, or a product past the range of fp32
+// (r-e and r+e may then be the same NaN, where fp64 has a value).
 template <typename T>
 __device__ __forceinline__ uint32_t rotate_pair_checked(float x0, float x1, float c, float s, uint32_t& out) {
   const float re = fmaf(x0, c, -__fmul_rn(x1, s)), im = fmaf(x0, s, __fmul_rn(x1, c));
   const float e = fmaf(__fmul_rn(fabsf(x0) + fabsf(x1), fabsf(c) + fabsf(s) + 0x1p-100f), 0x3p-23f, 0x1p-140f);
   out = pack_pair<T>(re - e, im - e);
-  return out ^ pack_pair<T>(re + e, im + e);
+  return (out ^ pack_pair<T>(re + e, im + e)) | (e < INFINITY ? 0u : 1u);
 }
 
 template <int MODE>

@@ -99,3 +99,30 @@ def test_captured_layer_follows_the_table():
     got = out.clone()
     del graph
     assert torch.equal(got, layer(separate(r)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("scale", [1.0, 300.0, 1e35, 1e300, 1e-38, 1e-44, 1e-300])
+def test_fp32_shortcut_at_the_ends_of_the_ranges(dtype, scale):
+    """The fp64 rotation with the fp32 copy against the one without, bit for bit: every pair of zeros, subnormals, values at
+    the end of the range, Inf and NaN, on tables up to and past the ends of fp32's range."""
+    fi = torch.finfo(dtype)
+    special = [0.0, -0.0, fi.smallest_normal / 4, -fi.smallest_normal, 1.0, -1.5, 1e4, -fi.max, fi.max, float("inf"),
+               float("-inf"), float("nan")]
+    pair = torch.tensor([[a, b] for a in special for b in special]).to(dtype)         # [144, 2]
+    D, H = 64, 2
+    N = pair.shape[0] * 6
+    x = pair.repeat(6, 1).unsqueeze(1).expand(N, D // 2, 2).reshape(1, 1, N, D).expand(1, H, N, D).contiguous().to(DEV)
+    g = torch.Generator().manual_seed(3)
+    ang = torch.rand(1 + 1 + N, D // 2, dtype=torch.float64, generator=g) * 7
+    tab = torch.stack([ang.cos(), ang.sin()], dim=-1).mul(scale).to(DEV)
+    copy = tab.to(torch.float32)
+    outs = []
+    for mode, sin in ((_lib.ROPE_COMPLEX_F64, None), (_lib.ROPE_COMPLEX_F64_APPROX, copy)):
+        out = torch.empty(1, H, N, D, dtype=dtype, device=DEV)
+        _lib.check(_lib.lib().paro_rope_permute(
+            x.data_ptr(), out.data_ptr(), _lib.dtype_code(dtype), 1, H, N, D, x.stride(0), x.stride(1), x.stride(2), 0, 1, 1, N,
+            None, 0, mode, tab.data_ptr(), _lib.ptr(sin), 0, 0, _lib.stream_ptr()))
+        outs.append(out.view(torch.int16))
+    assert torch.equal(*outs)
