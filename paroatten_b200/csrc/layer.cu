@@ -20,8 +20,8 @@ struct Sections {
 };
 
 // Elements of Q from which the passes get the fp32 copy of an interleaved fp64 table, made for the call: 2 us, which Q
-// and K of 2 x 12 x 1560 x 128 give back twice over (bf16: 29.6 -> 24.9 us) and those of 3 x 4200 x 128 do not (18.2 ->
-// 17.0).
+// and K of 2 x 12 x 1560 x 128 give back twice over (bf16: 29.6 -> 24.9 us) and those of 3 x 4200 x 128 barely (18.2 ->
+// 15.2), where the launches of a layer take longer than its passes.
 constexpr int64_t FP32_TABLE_ELEMS = 4 << 20;
 bool fp32_table(const paro_layer_args& a) {
   return a.rope_mode == PARO_ROPE_COMPLEX_F64 && a.cos_tab && !a.sin_tab && a.F > 0 && a.Hh > 0 && a.W > 0 &&

@@ -96,18 +96,26 @@ __device__ __forceinline__ uint32_t rotate_pair_f32(float x0, float x1, float c,
   return pack_pair<T>(__fadd_rn(__fmul_rn(x0, c), __fmul_rn(-x1, s)), __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s)));
 }
 
-// The fp64 result's bits from fp32 arithmetic, or a non-zero return where these are not certain.  fp32 is off by at
-// most 3 * 2^-24 * (|x0|+|x1|) * (|c|+|s|); e is twice that (the rounding of r-e, r+e itself included), 2^-100 and
-// 2^-140 cover table entries and products below the normal range.  Rounding is monotonic: where r-e and r+e round to
-// the same 16-bit value the fp64 result between them does too.  Uncertain are about one value in 2^13 for bf16 and
-// 2^10 for fp16, zeros, and everything whose e is not finite: an Inf or NaN operand, or a product past the range of fp32
-// (r-e and r+e may then be the same NaN, where fp64 has a value).
+// The fp64 result's bits from fp32 arithmetic, or a non-zero return where these are not certain.  With u = 2^-24, p and q
+// the rounded products and r their rounded sum, r is off by at most u * (2|p| + 2|q| + |r|) (the copy's entries, the
+// products and the sum, each rounded once), and r-e, r+e are themselves rounded by u * (|r| + e): e = 4u * (|p| + |q|) and
+// 2^-8 of that for the second-order terms.  2^-146 * (|x0| + |x1|) covers table entries below fp32's normal range (2^-130
+// where x is fp16, at most 2^16) and 2^-140 products below it.  Rounding is monotonic: where r-e and r+e round to the same
+// 16-bit value the fp64 result between them does too.  On N(0,1) inputs one pair of values in 2^10.6 is uncertain for
+// bf16 and in 2^7.9 for fp16; so are zeros and everything whose e is not finite: an Inf or NaN operand, or a product past
+// the range of fp32 (r-e and r+e may then be the same NaN, where fp64 has a value).  Those show in `worst`, the largest
+// e so far or NaN.  Of 2 x 12 x 32760 x 128, bf16 and fp16: INT8 Q 142 and 148 us, rotation + reorder 107 and 113; with one
+// e from (|x0|+|x1|) * (|c|+|s|), four times as many unsettled pairs and all four of a thread settled together 149 and
+// 172, 115 and 133; with fp64 alone 167 and 164, 138 and 144.
 template <typename T>
-__device__ __forceinline__ uint32_t rotate_pair_checked(float x0, float x1, float c, float s, uint32_t& out) {
-  const float re = fmaf(x0, c, -__fmul_rn(x1, s)), im = fmaf(x0, s, __fmul_rn(x1, c));
-  const float e = fmaf(__fmul_rn(fabsf(x0) + fabsf(x1), fabsf(c) + fabsf(s) + 0x1p-100f), 0x3p-23f, 0x1p-140f);
-  out = pack_pair<T>(re - e, im - e);
-  return (out ^ pack_pair<T>(re + e, im + e)) | (e < INFINITY ? 0u : 1u);
+__device__ __forceinline__ uint32_t rotate_pair_checked(float x0, float x1, float c, float s, uint32_t& out, float& worst) {
+  const float tiny = std::is_same<T, __half>::value ? 0x1p-130f : fmaf(fabsf(x0) + fabsf(x1), 0x1p-146f, 0x1p-140f);
+  const float p = __fmul_rn(x0, c), q = __fmul_rn(x1, s), re = __fsub_rn(p, q);
+  const float v = __fmul_rn(x0, s), w = __fmul_rn(x1, c), im = __fadd_rn(v, w);
+  const float er = fmaf(fabsf(p) + fabsf(q), 0x1.01p-22f, tiny), ei = fmaf(fabsf(v) + fabsf(w), 0x1.01p-22f, tiny);
+  out = pack_pair<T>(re - er, im - ei);
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(worst) : "f"(worst), "f"(er), "f"(ei));
+  return out ^ pack_pair<T>(re + er, im + ei);
 }
 
 template <int MODE>
@@ -126,8 +134,8 @@ __device__ __forceinline__ void load_angles(const RopeArgs& r, size_t t,
 }
 
 // Rows rotated at a time.  Two hide more of the table's latency (LayerNorm + rotation + reorder of 2 x 48 x 17776 x 64:
-// 187 -> 168 us), but with the fp64 fallback the second row's registers cost more than that (RMS norm, 2 x 12 x 32760 x
-// 128: 167 us one at a time, 217 two).
+// 187 -> 168 us), but with the fp64 fallback the second row's registers cost more than that (rotation + reorder of
+// 2 x 12 x 32760 x 128: 109 us one at a time, 117 two; with RMS norm 150 and 156).
 constexpr int ROTATE_ROWS_F32 = 2, ROTATE_ROWS_F64 = 1;
 
 // Rotates the four channel pairs held in each of x[0..NR), rows r, r + step, ... of the table.  The angles of all NR
@@ -137,7 +145,6 @@ constexpr int ROTATE_ROWS_F32 = 2, ROTATE_ROWS_F64 = 1;
 template <int NR, typename T, int MODE, int ROWS>
 __device__ __forceinline__ void rotate8(Pack8<T>* x, const PairAxes& pa, const RowTable<ROWS>& rows, int r, int step,
                                         const RopeArgs& rope) {
-  uint32_t bad = 1;
   if (rope.tab32) {
     // Two pairs per 16-byte load.  Where an axis ends between the two, the second one's angles are loaded by
     // themselves.
@@ -160,26 +167,33 @@ __device__ __forceinline__ void rotate8(Pack8<T>* x, const PairAxes& pa, const R
           cs[u][h].z = second.x; cs[u][h].w = second.y;
         }
       }
-    uint32_t out[NR][4];
-    bad = 0;
 #pragma unroll
     for (int u = 0; u < NR; ++u) {
-      uint32_t b = 0;
+      uint32_t out[4], unsettled[4];
+      float worst = 0.f;
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
         const float c = p & 1 ? cs[u][p >> 1].z : cs[u][p >> 1].x, s = p & 1 ? cs[u][p >> 1].w : cs[u][p >> 1].y;
         const float x0 = F16Traits<T>::to_float(x[u].e[2 * p]), x1 = F16Traits<T>::to_float(x[u].e[2 * p + 1]);
-        if constexpr (MODE == PARO_ROPE_REAL_F32) out[u][p] = rotate_pair_f32<T>(x0, x1, c, s);
-        else b |= rotate_pair_checked<T>(x0, x1, c, s, out[u][p]);
+        if constexpr (MODE == PARO_ROPE_REAL_F32) out[p] = rotate_pair_f32<T>(x0, x1, c, s);
+        else unsettled[p] = rotate_pair_checked<T>(x0, x1, c, s, out[p], worst);
       }
-      if (o0[u] >= 0) bad |= b;
-    }
-    if (MODE == PARO_ROPE_REAL_F32 || !bad) {
+      if (o0[u] < 0) continue;
+      if constexpr (MODE == PARO_ROPE_COMPLEX_F64) {
+        const bool lost = !(worst < INFINITY);
+        if ((unsettled[0] | unsettled[1] | unsettled[2] | unsettled[3]) || lost) {
+          // one pair at a time: a warp rarely has more than one to settle, and their angles would take 16 registers
 #pragma unroll
-      for (int u = 0; u < NR; ++u)
-        if (o0[u] >= 0) x[u].v = make_uint4(out[u][0], out[u][1], out[u][2], out[u][3]);
-      return;
+          for (int p = 0; p < 4; ++p)
+            if (unsettled[p] || lost) {
+              const double2 a = static_cast<const double2*>(rope.cos_tab)[2 * rows.off[pa.ax[p]][r + u * step] + pa.pair0 + p];
+              out[p] = rotate_pair_f64<T>(F16Traits<T>::to_float(x[u].e[2 * p]), F16Traits<T>::to_float(x[u].e[2 * p + 1]), a.x, a.y);
+            }
+        }
+      }
+      x[u].v = make_uint4(out[0], out[1], out[2], out[3]);
     }
+    return;
   }
 #pragma unroll
   for (int u = 0; u < NR; ++u) {
