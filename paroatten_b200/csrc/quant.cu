@@ -218,10 +218,12 @@ channel_finalize_kernel(const FinalizeDst<T> dst0, const FinalizeDst<T> dst1, in
 // ---------------------------------------------------------------------------------------------
 // INT8: one CTA = `blocks` consecutive 64-token blocks of one (b,h); warp w owns 64/WARPS tokens of each.
 // 2 bytes in, 1 byte out per element.
-// Passes that rotate (INT8_TABLE): 256 threads; source tokens and table rows of all the CTA's blocks are worked out once
+// Passes that rotate (TABLE): 256 threads; source tokens and table rows of all the CTA's blocks are worked out once
 // into shared memory.  Four blocks per CTA against one: 190 -> 140 us for 2 x 48 x 17776 x 64 with the fp32 rotation,
 // 257 -> 204 us for 2 x 12 x 32760 x 128 with RMS norm and the fp64 rotation.  (Loading the next block's rows ahead
-// costs the registers of a third CTA per SM: 148, 239 us.)
+// costs the registers of a third CTA per SM: 148, 239 us.  Four CTAs per SM at D = 64, where a thread holds two rows and
+// not four: Q of 2 x 48 x 17776 x 64 184 -> 168 us with the fp64 rotation, 244 -> 221 with LayerNorm and the fp32 one; at
+// D = 128 with a norm the fourth costs spills, RMS 197 -> 205 us.)
 // Passes that do not: 128 threads with twice the rows in flight each, one block per CTA, source tokens by shuffle (the
 // form above takes 90 us instead of 72 for 2 x 48 x 17776 x 64 in plain order, 29 instead of 22 for 40 x 4680 x 128
 // reordered).
@@ -231,8 +233,9 @@ template <int GM> struct Int8Cfg {
   static constexpr int WARPS = TABLE ? 8 : 4;
 };
 template <typename T, int D, int GROUP, int GM, int NM>
-__global__ void __launch_bounds__(32 * Int8Cfg<GM>::WARPS, !Int8Cfg<GM>::TABLE ? (NM != PARO_NORM_NONE ? 5 : 6)
-                                                           : (GM == GM_ROPE_F64 || NM != PARO_NORM_NONE ? 3 : 4))
+__global__ void __launch_bounds__(32 * Int8Cfg<GM>::WARPS,
+                                  !Int8Cfg<GM>::TABLE ? (NM != PARO_NORM_NONE ? 5 : 6)
+                                  : D == 64 || (GM == GM_ROPE_F32 && NM == PARO_NORM_NONE) ? 4 : 3)
 quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __restrict__ out,
                   float* __restrict__ scale, int H, int N, int64_t sb, int64_t sh, int64_t sn,
                   float fold, int n_scale_per_bh, int blocks, const Gather gather, const NormArgs norm) {
@@ -506,9 +509,12 @@ void launch_int8_norm(const void* x, const void* km, int8_t* out, float* scale, 
   const int nb = (N + 63) / 64;
   dispatch_gather(g, [&](auto gm) {
     constexpr int GM = decltype(gm)::value;
-    // several blocks per CTA where that leaves every SM a few CTAs; below that one each, for the latency
+    // Several blocks per CTA where that leaves every SM a few CTAs; below that one each, for the latency.  Three or four
+    // CTAs fit an SM: four blocks each from 21 blocks per SM on, two from five blocks per SM on (1, 2, 4 blocks, us, Q in bf16
+    // with the fp64 rotation: 12 x 32760 x 128 92, 82, 78; 20 x 7800 x 128 39, 35, 39; 24 x 2926 x 64 14.5, 12.5, 12.5;
+    // 2 x 12 x 1560 x 128 14.5, 14.5, 18.6, with LayerNorm 19, 21, 29).
     const int64_t total = (int64_t)nb * B * H;
-    const int blocks = !Int8Cfg<GM>::TABLE ? 1 : total >= 148 * 16 ? INT8_BLOCKS : total >= 148 * 8 ? 2 : 1;
+    const int blocks = !Int8Cfg<GM>::TABLE ? 1 : total >= 148 * 21 ? INT8_BLOCKS : total >= 148 * 5 ? 2 : 1;
     const dim3 grid((nb + blocks - 1) / blocks, B * H);
     if (group == 64)
       quant_int8_kernel<T, D, 64, GM, NM><<<grid, 32 * Int8Cfg<GM>::WARPS, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N,

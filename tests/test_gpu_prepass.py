@@ -322,8 +322,8 @@ def test_fp64_rotation_settled_in_fp32_has_the_fp64_bits(dtype, D, pairs_f, pair
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("B,H,N,D", [(1, 1, 1, 64), (1, 2, 63, 128), (1, 1, 257, 64), (2, 64, 2500, 64), (1, 48, 6401, 128)])
 def test_int8_blocks_per_cta(dtype, B, H, N, D):
-    """One 64-token block per CTA (small tensors) and four (large ones), with a ragged last block and a last CTA that is
-    not full: the oracle's bytes and scales."""
+    """The INT8 passes that do not rotate, one 64-token block per CTA at every size, with a ragged last block: the
+    oracle's bytes and scales."""
     x = rand((B, H, N, D), dtype, N)
     for group in (32, 64):
         want, ws = po.quant_int8(x, group)
@@ -333,3 +333,25 @@ def test_int8_blocks_per_cta(dtype, B, H, N, D):
     assert torch.equal(kp.cpu(), x)
     q8, qs, _ = pb.prep_qk_int8(x.to(DEV), None, (1, N, 1), group=32)
     assert torch.equal(q8.cpu(), po.quant_int8(x, 32)[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("family", ["wan", "cogvideox"])
+@pytest.mark.parametrize("B,H,D", [(1, 3, 128), (1, 47, 64), (1, 47, 128), (2, 97, 64), (2, 97, 128)])
+def test_rotating_int8_with_several_blocks_per_cta(dtype, family, B, H, D):
+    """The INT8 pass that rotates takes one, two or four 64-token blocks per CTA (57, 893 and 3686 blocks here); 19 blocks
+    per head leave the last CTA with one or three, the last of them with 16 tokens.  Bytes and scales of rotating and
+    reordering first and quantising the copy, which goes block by block."""
+    grid, n_text = (3, 13, 29), 37
+    N = n_text + grid[0] * grid[1] * grid[2]
+    g = torch.Generator(DEV).manual_seed(H + D)
+    x = torch.randn(B, N, H, D, device=DEV, generator=g).to(dtype)
+    ids = torch.arange(H, dtype=torch.int32, device=DEV) % 6
+    rope = pb.rope_tables(grid, D, family)
+    w = torch.rand(H * D, device=DEV, generator=g) + 0.5
+    for norm in (None, pb.QKNorm("layer", w[:D], w[-D:], 1e-6), pb.QKNorm("rms", w, None, 1e-6)):
+        kp = pb.rope_permute(x, ids, grid, n_text, rope, tensor_layout="NHD", norm=norm)
+        for group in (32, 64):
+            want, ws = pb.quant._quant_int8(kp, "HND", group)
+            got, gs, _ = pb.prep_qk_int8(x, ids, grid, n_text, rope, group=group, tensor_layout="NHD", norm=norm)
+            assert torch.equal(got, want) and torch.equal(gs, ws)
