@@ -15,7 +15,8 @@ constexpr long long WAIT_LIMIT = 400000000;  // SM cycles (~0.2 s) before a wait
 constexpr float SCORE_BIAS = 12582912.0f;    // 1.5 * 2^23, bit pattern 0x4B400000
 
 // Words of the redo work space handed to paro_sparse_attn: [0] number of work items the fixed-reference walk
-// gave back, [1..] the items (block indices of the fast launch).
+// gave back, [1..] the items (block indices of the fast launch), and behind room for all of them, where the work space
+// has it, the number of items that the exact walk's CTAs have fetched beyond their first.
 constexpr int REDO_HEADER = 1;
 
 struct AttnParams {
@@ -33,6 +34,7 @@ struct AttnParams {
   int32_t* status;
   int32_t* host_status; // nullable: pinned host copy of the status words, written when a wait expires
   int32_t* redo;        // work space described above
+  int32_t* redo_next;   // its last word, or nullptr
   int64_t osb, osh, osn;
   int plan_slices, q_group, n_text;
   int B, H, N, npairs, nb;

@@ -135,7 +135,7 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
     if (rc) return rc;
   }
   // (these passes clear the redo counter as well)
-  const bool fast = a.attn_mode == PARO_ATTN_FAST && a.redo && a.redo_bytes >= paro_sparse_attn_redo_bytes(a.B, a.H, a.N);
+  const bool fast = a.attn_mode == PARO_ATTN_FAST && a.redo && a.redo_bytes >= sizeof(int32_t);
   if (int rc = layer_kv_passes(a, kp, w + at.km, k8, ks, v16, vs, vm, w + at.stats, fast ? a.redo : nullptr, s)) return rc;
 
   if (a.ev_start) PARO_CUDA_OK(cudaEventRecord((cudaEvent_t)a.ev_start, s));

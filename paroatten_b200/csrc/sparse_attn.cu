@@ -102,8 +102,10 @@ template <int D> struct AttnCfg {
 //   A step whose row sum leaves that range (or is not finite) makes the CTA give its work item back
 //   through the redo list instead of storing it; the exact walk then computes that pair.
 // LIST: the second launch of a call.  Its work items are the redo list, which is empty for nearly all inputs, so it
-// is a small grid whose CTAs walk the list in strides.  (One CTA per possible item costs 19 us for 2955 of them,
-// 70 us for 13344, 120 us for 23640, to find out that there is nothing to do.)
+// is a small grid whose CTAs fetch one item after another.  (One CTA per possible item costs 19 us for 2955 of them,
+// 70 us for 13344, 120 us for 23640, to find out that there is nothing to do.  A fixed stride instead of a counter leaves
+// CTAs idle where the items differ in length: 40 heads x 3001 x 128 whose text rows keep every block, all given back,
+// 277 us against 243 for the call.)
 template <int D, typename OutT, bool FIXED, bool LIST>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -139,12 +141,13 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   volatile int* s_drain = abort_flag + 1;                  // 1: an earlier launch or CTA failed, leave at once
   volatile int* s_redo = s_drain + 1;                      // 1: a row sum left the fixed-reference range
   volatile int* s_mstep = s_redo + 1;                      // [4]  steps whose row maxima are published, per quadrant
+  [[maybe_unused]] volatile int* s_next = s_mstep + 4;     // LIST: position of the CTA's next item
   float* s_vscale = reinterpret_cast<float*>(aux + 512);   // [D]
   float* s_vm = s_vscale + D;                              // [D]
   volatile float* s_mrow = reinterpret_cast<volatile float*>(aux + 1536);   // [128] running row maximum
   float* s_xl = reinterpret_cast<float*>(aux + 2048);                       // [2][128] row-sum exchange
   static_assert(512 + 2 * D * 4 <= 1536 && 2048 + 2 * 128 * 4 <= Cfg::AUX_BYTES, "aux area too small");
-  static_assert((27 + KST + VST) * 8 + 8 + 28 <= 512, "barrier area too small");
+  static_assert((27 + KST + VST) * 8 + 8 + 32 <= 512, "barrier area too small");
 
   // (the warp index through a shuffle: provably the same in all lanes, so the role branches are uniform)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -174,6 +177,7 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     n_steps = max(n_a, n_b);
   };
   set_item(LIST ? p.redo[REDO_HEADER + list_at] : (int)blockIdx.x);
+  if (FIXED && p.redo_next && blockIdx.x == 0 && threadIdx.x == 0) *p.redo_next = 0;   // (read by the launch after this one)
   // A step is one group of MMAs of each kind: FORM_UPPER / FORM_LOWER when only one half still has blocks (128
   // rows, the other half's accumulator rows masked), FORM_SHARED when both keep the same block (one tile, 128
   // rows) and FORM_DUAL when each half has its own (two tiles, tcgen05.mma.ws: two 64-row products in one
@@ -218,15 +222,19 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     if constexpr (!LIST) return false;
     tc_fence_before();
     __syncthreads();
-    list_at += (int)gridDim.x;
-    if (*abort_flag || list_at >= list_len) return false;
     if (threadIdx.x == 0) {
-      for (uint64_t* bar = bar_q; bar < bar_drain + 2; ++bar) mbar_inval(bar);
-      init_barriers();
+      const int next = (int)gridDim.x + (p.redo_next ? atomicAdd(p.redo_next, 1) : list_at);
+      *s_next = next;
+      if (!*abort_flag && next < list_len) {
+        for (uint64_t* bar = bar_q; bar < bar_drain + 2; ++bar) mbar_inval(bar);
+        init_barriers();
+      }
     }
-    set_item(p.redo[REDO_HEADER + list_at]);
     __syncthreads();
+    list_at = *s_next;
+    if (*abort_flag || list_at >= list_len) return false;
     tc_fence_after();
+    set_item(p.redo[REDO_HEADER + list_at]);
     return true;
   };
 
@@ -822,7 +830,7 @@ using namespace paro;
 extern "C" size_t paro_sparse_attn_redo_bytes(int B, int H, int N) {
   if (B <= 0 || H <= 0 || N <= 0) return 0;
   const size_t nb = ((size_t)N + 63) / 64;
-  return sizeof(int32_t) * (REDO_HEADER + (size_t)B * H * ((nb + 1) / 2));
+  return sizeof(int32_t) * (REDO_HEADER + (size_t)B * H * ((nb + 1) / 2) + 1);
 }
 
 int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t* v16, const float* q_scale, int q_group,
@@ -847,12 +855,14 @@ int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t*
                PARO_EALIGN, "paro_sparse_attn: output strides must be multiples of 8 elements");
   PARO_REQUIRE(sm_scale > 0.f, PARO_EINVAL, "paro_sparse_attn: sm_scale must be positive");
   PARO_REQUIRE(mode == PARO_ATTN_FAST || mode == PARO_ATTN_EXACT, PARO_EINVAL, "paro_sparse_attn: unknown mode %d", mode);
-  PARO_REQUIRE(mode == PARO_ATTN_EXACT || (redo && redo_bytes >= paro_sparse_attn_redo_bytes(B, H, N)), PARO_ECAP,
+  const size_t redo_full = paro_sparse_attn_redo_bytes(B, H, N);   // (all but the last word is enough: see redo_next)
+  PARO_REQUIRE(mode == PARO_ATTN_EXACT || (redo && redo_bytes >= redo_full - sizeof(int32_t)), PARO_ECAP,
                "paro_sparse_attn: PARO_ATTN_FAST needs a redo work space of paro_sparse_attn_redo_bytes() bytes");
   AttnParams p;
   p.q8 = q8; p.q_scale = q_scale; p.k_scale = k_scale; p.v_scale = v_scale; p.vm = vm;
   p.pair_ptr = pair_ptr; p.sched = sched; p.sched_cnt = sched_cnt; p.inv_idx = inv_idx;
   p.out = out; p.lse = lse; p.status = status; p.host_status = host_status; p.redo = redo;
+  p.redo_next = mode == PARO_ATTN_FAST && redo_bytes >= redo_full ? redo + redo_full / sizeof(int32_t) - 1 : nullptr;
   p.osb = out_stride_b; p.osh = out_stride_h; p.osn = out_stride_n;
   p.plan_slices = plan_slices; p.q_group = q_group; p.n_text = n_text;
   p.B = B; p.H = H; p.N = N; p.nb = (N + 63) / 64; p.npairs = (p.nb + 1) / 2;
@@ -864,7 +874,10 @@ int paro::sparse_attn_launch(const int8_t* q8, const int8_t* k8, const uint16_t*
   // as many CTAs as fit the chip at two per SM
   if (!redo_is_zero) PARO_CUDA_OK(cudaMemsetAsync(redo, 0, sizeof(int32_t) * REDO_HEADER, s));
   if (int rc = launch_attn_fixed(k8, v16, p, D, out_dtype, (unsigned)ctas, s)) return rc;
-  return launch_attn_exact<true>(k8, v16, p, D, out_dtype, (unsigned)(ctas < 296 ? ctas : 296), s);
+  int dev = 0, sms = 0;
+  PARO_CUDA_OK(cudaGetDevice(&dev));
+  PARO_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return launch_attn_exact<true>(k8, v16, p, D, out_dtype, (unsigned)(ctas < 2ull * sms ? ctas : 2ull * sms), s);
 }
 
 extern "C" int paro_sparse_attn(const int8_t* q8, const int8_t* k8, const uint16_t* v16,

@@ -8,6 +8,7 @@ import torch
 
 import paroatten_b200 as pb
 from oracle import paro_oracle as po
+from paroatten_b200 import _lib, core
 
 pytestmark = pytest.mark.gpu
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
@@ -119,6 +120,58 @@ def test_redo_list_longer_than_its_grid(D, H, nb):
             assert torch.equal(got, want) and torch.equal(lse, wlse)
         else:                             # (items that stayed on the fast walk differ in the rounding of P)
             assert (got.float() - want.float()).norm() <= 1e-2 * want.float().norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("spare", [1, 0])
+def test_items_of_the_redo_list_have_the_exact_walks_bits(D, spare, monkeypatch):
+    """Growing keys in most heads and text rows that keep every block, pairs chosen by overlap, two batch entries, rows
+    stored through an inverse permutation: the rows of exactly the items that the list names have the bits of an all-exact
+    call, the others differ in the rounding of P only.  spare: the work space holds the counter from which the exact walk's
+    CTAs fetch their items, or it is one word shorter and they go by a fixed stride."""
+    B, H, grid, n_text = 2, 20, (3, 16, 41), 9
+    N = n_text + grid[0] * grid[1] * grid[2]
+    nb = (N + 63) // 64
+    npairs = (nb + 1) // 2
+    q, k, v, orders = po.make_inputs(B, H, N, D, torch.bfloat16, seed=79)
+    f = (1.0 + 9.0 * torch.arange(nb, dtype=torch.float32)).repeat_interleave(64)[:N].expand(H, N).clone()
+    f[15:] = 1.0
+    k = (k.float() * f.reshape(1, H, N, 1)).to(torch.bfloat16)
+    mask = po.make_mask(H, nb, 0.4, seed=7)
+    mask[:, :, 0] = True
+    mask[:, :1] = True
+    plan = pb.compact_plan(mask.to(DEV), pairing="overlap")
+    assert plan.pair_q is not None
+    inv = pb.perm_index(torch.tensor(orders), grid)
+    q8, qs, k8, ks = pb.per_warp_int8(q.to(DEV), k.to(DEV), pb.channel_mean(k.to(DEV)), BLKQ=64)
+    _, vs, vm, v16 = pb.per_channel_fp8(v.to(DEV), return_16=True)
+    words = _lib.lib().paro_sparse_attn_redo_bytes(B, H, N) // 4 - 1 + spare
+    redo = torch.full((words,), -1, dtype=torch.int32, device=DEV)
+    monkeypatch.setattr(core, "_redo_space", lambda *args: redo)
+    runs = {}
+    for mode in ("exact", "fast", "fast again"):
+        out = torch.full((B, H, N, D), float("nan"), dtype=torch.bfloat16, device=DEV)
+        runs[mode] = pb.sparse_attn_quantized(q8, qs, k8, ks, v16, vs, vm, plan, D ** -0.5, inv_index=inv, n_text=n_text,
+                                              return_lse=True, out=out, mode=mode.split()[0])
+        pb.check_status()
+    items = redo[1:1 + int(redo[0])].cpu().long()
+    assert 296 < items.numel() < B * H * npairs and items.unique().numel() == items.numel()
+    redone = torch.zeros(B, H, N, dtype=torch.bool)          # by output token
+    for item in items.tolist():
+        bh, pair = divmod(item, npairs)
+        b, h = divmod(bh, H)
+        for qb in plan.pair_q[h * npairs + pair].tolist():
+            if qb >= 0:
+                tok = torch.arange(qb * 64, min(N, qb * 64 + 64))
+                dst = torch.where(tok < n_text, tok, n_text + inv[h].cpu().long()[(tok - n_text).clamp_min(0)])
+                redone[b, h, dst] = True
+    redone = redone.to(DEV)
+    want, wlse = runs["exact"]
+    for mode in ("fast", "fast again"):
+        got, lse = runs[mode]
+        assert torch.equal(got[redone], want[redone]) and torch.equal(lse[redone], wlse[redone])
+        # (P in bf16 relative to another exponent: 5e-4 of the norm on N(0,1) inputs, stated at four times that)
+        assert (got[~redone].float() - want[~redone].float()).norm() <= 2e-3 * want[~redone].float().norm()
 
 
 def test_c1_plumbing_fixture():
