@@ -4,6 +4,8 @@
 //   paro_merge_attn_states  combines two partial attention results (O, LSE) computed over disjoint sets
 //                           of key blocks into the result over their union -- what the LSE output is for
 //                           (sequence-parallel / ring composition, reference core.py:55-57).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace paro {
@@ -73,10 +75,12 @@ __global__ void plan_validate_kernel(const int32_t* __restrict__ pair_ptr, const
 // LSE is -inf (no kept block for that row) contributes nothing.
 // HBM-bound (6 bytes per element): 16 bytes = 8 channels of a row per load, MERGE_ROWS rows of both tensors in
 // flight per thread.  A row's weights take two exponentials, a logarithm and two divisions: one lane computes
-// them and hands them to the D/8 lanes of the row (computed by every lane, with the row found by 64-bit
-// divisions, they took about as long as the loads: 12 x 32760 x 128 bf16 70.0 -> 67.8 us; 45 us are its bytes).
-constexpr int MERGE_ROWS = 4;
-template <typename T, int D>
+// them, from LSEs requested before the rows, and hands them to the D/8 lanes of the row (computed by every lane, with
+// the row found by 64-bit divisions, they took about as long as the loads).
+// Two rows in bf16, four in fp16, whose conversions take fewer instructions: 12 x 32760 x 128 with one, two, four rows 68,
+// 53, 57 us in bf16 and 64, 49, 47 in fp16 (one row per thread, weights by every lane: 70, 68).  46 us are its bytes.
+// Two rows as well where a CTA's four would be past a short sequence's end: 2000 x 16 x 128 in fp16 8.3 and 11 us.
+template <typename T, int D, int MERGE_ROWS>
 __global__ void __launch_bounds__(256)
 merge_states_kernel(const T* __restrict__ oa, const float* __restrict__ la, const T* __restrict__ ob,
                     const float* __restrict__ lb, T* __restrict__ out, float* __restrict__ lo, int H, int N, int BH,
@@ -88,6 +92,8 @@ merge_states_kernel(const T* __restrict__ oa, const float* __restrict__ la, cons
   for (int bh = blockIdx.y; bh < BH; bh += gridDim.y) {
     const int64_t base = (bh / H) * sb + (bh % H) * sh + c8;
     const size_t row0 = (size_t)bh * N;
+    const bool mine = lane < WROWS && n0 + lane < N;
+    const float a = mine ? la[row0 + n0 + lane] : 0.f, c = mine ? lb[row0 + n0 + lane] : 0.f;
     Pack8<T> pa[MERGE_ROWS], pb[MERGE_ROWS];
 #pragma unroll
     for (int u = 0; u < MERGE_ROWS; ++u) {
@@ -98,8 +104,7 @@ merge_states_kernel(const T* __restrict__ oa, const float* __restrict__ la, cons
       }
     }
     float wa = 0.f, wb = 0.f;                     // of row n0 + lane
-    if (lane < WROWS && n0 + lane < N) {
-      const float a = la[row0 + n0 + lane], c = lb[row0 + n0 + lane];
+    if (mine) {
       const float m = fmaxf(a, c);
       float l = -INFINITY;
       if (m > -INFINITY) {
@@ -128,15 +133,16 @@ merge_states_kernel(const T* __restrict__ oa, const float* __restrict__ la, cons
   }
 }
 
-template <typename T>
+template <typename T, int D>
 void launch_merge(const void* oa, const float* la, const void* ob, const float* lb, void* out, float* lo, int B, int H, int N,
-                  int D, int64_t sb, int64_t sh, int64_t sn, cudaStream_t s) {
-  const int rows = 8 * MERGE_ROWS * (256 / D);   // rows per CTA
-  const dim3 grid((N + rows - 1) / rows, (unsigned)min((long long)B * H, 65535ll));
-  if (D == 128)
-    merge_states_kernel<T, 128><<<grid, 256, 0, s>>>((const T*)oa, la, (const T*)ob, lb, (T*)out, lo, H, N, B * H, sb, sh, sn);
-  else
-    merge_states_kernel<T, 64><<<grid, 256, 0, s>>>((const T*)oa, la, (const T*)ob, lb, (T*)out, lo, H, N, B * H, sb, sh, sn);
+                  int64_t sb, int64_t sh, int64_t sn, cudaStream_t s) {
+  auto launch = [&](auto rows) {
+    constexpr int R = decltype(rows)::value, CTA_ROWS = 8 * R * (256 / D);
+    const dim3 grid((N + CTA_ROWS - 1) / CTA_ROWS, (unsigned)min((long long)B * H, 65535ll));
+    merge_states_kernel<T, D, R><<<grid, 256, 0, s>>>((const T*)oa, la, (const T*)ob, lb, (T*)out, lo, H, N, B * H, sb, sh, sn);
+  };
+  if (std::is_same<T, __half>::value && N >= 256) launch(std::integral_constant<int, 4>{});
+  else launch(std::integral_constant<int, 2>{});
 }
 
 }  // namespace paro
@@ -176,9 +182,12 @@ extern "C" int paro_merge_attn_states(const void* o_a, const float* lse_a, const
   if (int rc = check_tensor("paro_merge_attn_states(o_b)", o_b, dtype, B, H, N, D, stride_b, stride_h, stride_n)) return rc;
   if (int rc = check_tensor("paro_merge_attn_states(out)", out, dtype, B, H, N, D, stride_b, stride_h, stride_n)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == PARO_F16)
-    launch_merge<__half>(o_a, lse_a, o_b, lse_b, out, lse_out, B, H, N, D, stride_b, stride_h, stride_n, s);
-  else
-    launch_merge<__nv_bfloat16>(o_a, lse_a, o_b, lse_b, out, lse_out, B, H, N, D, stride_b, stride_h, stride_n, s);
+  auto merge = [&](auto tag) {
+    using T = decltype(tag);
+    if (D == 128) launch_merge<T, 128>(o_a, lse_a, o_b, lse_b, out, lse_out, B, H, N, stride_b, stride_h, stride_n, s);
+    else launch_merge<T, 64>(o_a, lse_a, o_b, lse_b, out, lse_out, B, H, N, stride_b, stride_h, stride_n, s);
+  };
+  if (dtype == PARO_F16) merge(__half{});
+  else merge(__nv_bfloat16{});
   return check_launch("merge_states_kernel");
 }

@@ -357,3 +357,27 @@ def test_one_layer_call_equals_its_passes(layout, norm, smooth_k, n_text):
     want, wlse = pb.sparse_attn_quantized(q8, qs, k8, ks, v16, vs, vm, plan, D ** -0.5, inv_index=pb.perm_index(ids, grid),
                                           n_text=n_text, return_lse=True, out_layout=layout)
     assert torch.equal(got, want) and torch.equal(lse, wlse)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,H,N,D", [(1, 3, 1, 64), (2, 300, 16, 128), (1, 5, 255, 64), (1, 2, 256, 128), (1, 3, 1000, 128),
+                                     (2, 2, 2049, 64)])
+def test_merge_at_the_edges_of_its_tiles(dtype, B, H, N, D):
+    """Short sequences (two rows per thread) and longer ones (four in fp16), rows with one side or both empty, NaN on an
+    empty side: the fp64 result rounded once, give or take the fp32 weights (2^-20 of the summands)."""
+    g = torch.Generator(DEV).manual_seed(N)
+    a, b = (torch.randn(B, H, N, D, device=DEV, generator=g).to(dtype) for _ in range(2))
+    la, lb = (torch.randn(B, H, N, device=DEV, generator=g) * 3 for _ in range(2))
+    la[torch.rand(la.shape, device=DEV, generator=g) < 0.2] = -float("inf")
+    lb[torch.rand(lb.shape, device=DEV, generator=g) < 0.2] = -float("inf")
+    a[la == -float("inf")] = float("nan")
+    o, lse = pb.merge_attention_states(a, la, b, lb)
+    wl = torch.logaddexp(la.double(), lb.double())
+    wa, wb = ((x.double() - wl).exp().nan_to_num(0.0).unsqueeze(-1) for x in (la, lb))
+    want = torch.where(wa > 0, a.double() * wa, 0.0) + torch.where(wb > 0, b.double() * wb, 0.0)
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11      # of an 8- and an 11-bit significand
+    size = torch.where(wa > 0, a.double() * wa, 0.0).abs() + (b.double() * wb).abs()
+    assert ((o.double() - want).abs() <= want.abs() * half_ulp + size * 2.0 ** -20 + 2.0 ** -25).all()
+    assert torch.equal(lse == -float("inf"), wl == -float("inf"))
+    ok = wl > -float("inf")
+    assert ((lse.double() - wl)[ok].abs() <= 2.0 ** -22 * (8 + wl[ok].abs())).all()
