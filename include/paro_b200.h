@@ -62,7 +62,8 @@ int paro_build_perm_index(const int32_t* order_ids, int H, int F, int Hh, int W,
  * apply_rotary_emb at cogvideox.py:167-172), fp64 for PARO_ROPE_COMPLEX_F64 (wan.py:161-164).
  * pairs_f/pairs_h: how many leading channel pairs follow the f / h coordinate (rest: w).
  * sin_tab == NULL (all entry points that take the two tables): cos_tab is then ONE table
- * [F+Hh+W, D/2, 2] with cos and sin of a pair side by side, fetched by a single load.
+ * [F+Hh+W, D/2, 2] with cos and sin of a pair side by side, fetched by a single load (aligned to a pair: 8 bytes
+ * in fp32, 16 in fp64).
  * PARO_ROPE_COMPLEX_F64_APPROX: the same results as PARO_ROPE_COMPLEX_F64, faster; cos_tab is the interleaved fp64 table
  * and sin_tab (16-byte aligned) the same table rounded to fp32 (paro_layer makes that copy itself, in every call).
  * Replaces csrc/rope/rope.cu:14-48 (rope_permutation) and permute_qk / permute_attn_out
@@ -215,7 +216,8 @@ int paro_plan_schedule(const int32_t* pair_ptr, const int32_t* pair_ent, int sli
  * paro_plan_offsets writes row_ptr, pair_ptr and totals[4] (device): kept blocks, merged entries, 1 if any slice was paired
  * by overlap, 1 if a bounded device-side wait expired (the lists are then invalid).  The caller reads the totals back, allocates cols [kept] and pair_ent, sched [merged entries] (at
  * least one element each), and paro_plan_lists fills them, sched_cnt, and (nullable, overlap only) sched_cnt_kernel: the
- * step counts with (q-block id + 1) << 16, as paro_sparse_attn reads them.
+ * step counts with (q-block id + 1) << 16, as paro_sparse_attn reads them.  pair_q, sched_cnt and sched_cnt_kernel are
+ * 8-byte aligned.
  * scratch: paro_plan_scratch_bytes(), 16-byte aligned, kept unchanged from the first call to the second. */
 size_t paro_plan_scratch_bytes(int slices, int nbq, int nbk, int overlap);
 int paro_plan_offsets(const uint8_t* mask, int slices, int nbq, int nbk, int overlap,

@@ -39,6 +39,7 @@ inline int check_launch(const char* what, int n_kernels = 1) {
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
 // Common argument checks for a [B,H,N,D] tensor addressed through element strides.
 int check_tensor(const char* name, const void* p, int dtype, int B, int H, int N, int D,

@@ -484,6 +484,7 @@ extern "C" int paro_plan_offsets(const uint8_t* mask, int slices, int nbq, int n
                                  int32_t* pair_ptr, int32_t* pair_q, int32_t* totals, void* scratch, size_t scratch_bytes,
                                  paro_stream_t stream) {
   PARO_REQUIRE(mask && row_ptr && pair_ptr && totals && (!overlap || pair_q), PARO_EINVAL, "paro_plan_offsets: null pointer");
+  PARO_REQUIRE(!overlap || aligned8(pair_q), PARO_EALIGN, "paro_plan_offsets: pair_q not 8-byte aligned");
   PlanScratch sc;
   if (int rc = check_plan_args("paro_plan_offsets", slices, nbq, nbk, overlap, scratch, scratch_bytes, &sc)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
@@ -515,6 +516,8 @@ extern "C" int paro_plan_lists(int slices, int nbq, int nbk, int overlap, const 
                                int32_t* sched_cnt_kernel, const void* scratch, size_t scratch_bytes, paro_stream_t stream) {
   PARO_REQUIRE(row_ptr && pair_ptr && cols && pair_ent && sched && sched_cnt && (!overlap || pair_q), PARO_EINVAL,
                "paro_plan_lists: null pointer");
+  PARO_REQUIRE(aligned8(sched_cnt) && aligned8(sched_cnt_kernel), PARO_EALIGN,
+               "paro_plan_lists: sched_cnt / sched_cnt_kernel not 8-byte aligned");
   PlanScratch sc;
   if (int rc = check_plan_args("paro_plan_lists", slices, nbq, nbk, overlap, scratch, scratch_bytes, &sc)) return rc;
   const int npairs = (nbq + 1) / 2, prows = slices * npairs;

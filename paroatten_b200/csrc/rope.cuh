@@ -40,6 +40,9 @@ inline int check_rope(const char* who, int mode, const void* cos_tab, const void
   PARO_REQUIRE(pairs_f >= 0 && pairs_h >= 0 && pairs_f + pairs_h <= D / 2, PARO_ESHAPE, "%s: pairs_f + pairs_h exceeds D/2", who);
   PARO_REQUIRE(mode != PARO_ROPE_COMPLEX_F64_APPROX || (sin_tab && aligned16(sin_tab)), PARO_EALIGN,
                "%s: the fp32 table is missing or not 16-byte aligned", who);
+  const bool interleaved = mode == PARO_ROPE_COMPLEX_F64_APPROX || !sin_tab;   // (cos and sin of a pair by one load)
+  PARO_REQUIRE(!interleaved || (mode == PARO_ROPE_REAL_F32 ? aligned8(cos_tab) : aligned16(cos_tab)), PARO_EALIGN,
+               "%s: an interleaved table must be aligned to a pair (8 bytes in fp32, 16 in fp64)", who);
   return PARO_OK;
 }
 

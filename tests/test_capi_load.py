@@ -60,3 +60,29 @@ def test_ops_refuse_cpu_tensors():
         pb.per_warp_int8(x, x, BLKQ=64, WARPQ=32, BLKK=64)
     with pytest.raises(RuntimeError, match="no CPU path"):
         pb.compact_plan(torch.ones(1, 2, 2, dtype=torch.bool))
+
+
+def aligned_buffer(size):
+    buf = ctypes.create_string_buffer(size + 64)
+    return buf, (ctypes.addressof(buf) + 63) & ~63
+
+
+def test_pointers_that_are_read_or_written_as_vectors_must_be_aligned():
+    """Refused before any CUDA call: a store of two counts, or a load of a pair's (cos, sin), at an address that is no
+    multiple of its size would fault on the GPU."""
+    L = _lib.lib()
+    buf, a = aligned_buffer(1 << 16)
+    need = L.paro_plan_scratch_bytes(1, 8, 8, 1)
+    rc = L.paro_plan_offsets(a, 1, 8, 8, 1, a, a, a + 4, a, a, need, None)
+    assert rc == _lib.PARO_EALIGN and b"pair_q" in L.paro_last_error()
+    for cnt, kernel in ((a + 4, a), (a, a + 4)):
+        rc = L.paro_plan_lists(1, 8, 8, 1, a, a, a, a, a, a, cnt, kernel, a, need, None)
+        assert rc == _lib.PARO_EALIGN and b"sched_cnt" in L.paro_last_error()
+    for mode, cos, sin in ((_lib.ROPE_REAL_F32, a + 4, None), (_lib.ROPE_COMPLEX_F64, a + 8, None),
+                           (_lib.ROPE_COMPLEX_F64_APPROX, a + 8, a), (_lib.ROPE_COMPLEX_F64_APPROX, a, a + 8),
+                           (_lib.ROPE_COMPLEX_F64_APPROX, a, None)):
+        rc = L.paro_rope_permute(a, a + 4096, 1, 1, 1, 6, 64, 0, 0, 64, 0, 1, 2, 3, None, 0, mode, cos, sin, 0, 0, None)
+        assert rc == _lib.PARO_EALIGN
+        rc = L.paro_prep_qk_int8(a, 1, 1, 1, 6, 64, 0, 0, 64, 0, 1, 2, 3, None, mode, cos, sin, 0, 0, 32, 0, None, a, a,
+                                 None, 0, None)
+        assert rc == _lib.PARO_EALIGN
