@@ -80,8 +80,13 @@ def _raise_if_earlier_launch_failed(device: torch.device) -> None:
     when a wait expires); each new call looks at that copy first (no synchronisation).  A launch that gave up a wait
     therefore stops the caller at the next attention call at the latest, instead of every later launch
     returning at once and leaving its output unwritten."""
-    if ctypes.c_int32.from_address(_mirror(device).data_ptr()).value != 0:
+    mirror = _mirror(device)
+    if ctypes.c_int32.from_address(mirror.data_ptr()).value != 0:
         check_status(device)      # synchronises, clears the words and raises with the waiter's position
+        # The failure has been reported already (its copy came in after the words were cleared).  The words are looked
+        # at once more: a wait that expired in between has set them before it writes the copy.
+        mirror.zero_()
+        check_status(device)
 
 
 def sparse_attn_quantized(q_int8, q_scale, k_int8, k_scale, v16, v_scale, vm, plan: CompactPlan, sm_scale: float,

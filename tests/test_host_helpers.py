@@ -43,3 +43,26 @@ def test_pairing_by_overlap_is_a_permutation_and_saves_tiles():
         assert tiles(order) <= adjacent
         if nb >= 64:
             assert tiles(order) < 0.99 * adjacent
+
+
+def test_a_status_copy_that_came_late_is_taken_back(monkeypatch):
+    """The pinned copy says that a wait expired, the device words do not (they were read and cleared before the copy came
+    in): the call goes on, and the next one does not synchronise again.  A failure that shows at the second look raises."""
+    import pytest
+    import torch
+    from paroatten_b200 import core
+    mirror, looks = torch.tensor([-4, 8, 3, 5], dtype=torch.int32), []
+    monkeypatch.setattr(core, "_mirror", lambda device: mirror)
+    monkeypatch.setattr(core, "check_status", lambda device: looks.append(int(mirror[0])))
+    for _ in range(2):
+        core._raise_if_earlier_launch_failed(torch.device("cuda", 0))
+    assert looks == [-4, 0] and int(mirror[0]) == 0
+
+    def second_look_fails(device):
+        looks.append(int(mirror[0]))
+        if looks[-1] == 0:
+            raise RuntimeError("wait expired")
+    monkeypatch.setattr(core, "check_status", second_look_fails)
+    mirror[0] = -4
+    with pytest.raises(RuntimeError):
+        core._raise_if_earlier_launch_failed(torch.device("cuda", 0))
