@@ -8,6 +8,7 @@
 // share their statistics launches and the passes themselves became shorter.
 #include "attn_common.cuh"
 #include "common.cuh"
+#include "norm.cuh"
 #include "rope.cuh"
 
 using namespace paro;
@@ -77,13 +78,16 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
   float *qs = reinterpret_cast<float*>(w + at.qs), *ks = reinterpret_cast<float*>(w + at.ks);
   float *vs = reinterpret_cast<float*>(w + at.vs), *vm = reinterpret_cast<float*>(w + at.vm);
 
-  // arguments of every pass, before the first of them
+  // what the pre-attention passes would refuse, before the first of them
   if (int rc = check_tensor("paro_layer(q)", a.q, a.dtype, a.B, a.H, a.N, a.D, a.q_strides[0], a.q_strides[1], a.q_strides[2])) return rc;
   if (int rc = check_tensor("paro_layer(k)", a.k, a.dtype, a.B, a.H, a.N, a.D, a.k_strides[0], a.k_strides[1], a.k_strides[2])) return rc;
   if (int rc = check_tensor("paro_layer(v)", a.v, a.dtype, a.B, a.H, a.N, a.D, a.v_strides[0], a.v_strides[1], a.v_strides[2])) return rc;
   PARO_REQUIRE(a.F > 0 && a.Hh > 0 && a.W > 0 && a.n_text >= 0 && (int64_t)a.n_text + (int64_t)a.F * a.Hh * a.W == a.N,
                PARO_ESHAPE, "paro_layer: n_text + F*H*W = %lld != N = %d", (long long)a.n_text + (long long)a.F * a.Hh * a.W, a.N);
   if (int rc = check_rope("paro_layer", a.rope_mode, a.cos_tab, a.sin_tab, a.pairs_f, a.pairs_h, a.D)) return rc;
+  const float* const section = reinterpret_cast<const float*>(w);   // (stands for the RMS statistics, computed below)
+  if (int rc = check_norm("paro_layer(q)", a.q_norm_mode, a.q_norm_weight, a.q_norm_bias, section, a.q_norm_eps)) return rc;
+  if (int rc = check_norm("paro_layer(k)", a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, section, a.k_norm_eps)) return rc;
 
   int rope_mode = a.rope_mode;
   const void* sin_tab = a.sin_tab;

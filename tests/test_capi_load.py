@@ -86,3 +86,67 @@ def test_pointers_that_are_read_or_written_as_vectors_must_be_aligned():
         rc = L.paro_prep_qk_int8(a, 1, 1, 1, 6, 64, 0, 0, 64, 0, 1, 2, 3, None, mode, cos, sin, 0, 0, 32, 0, None, a, a,
                                  None, 0, None)
         assert rc == _lib.PARO_EALIGN
+
+
+def test_layer_refuses_bad_arguments_before_its_first_launch():
+    L = _lib.lib()
+    buf, a = aligned_buffer(1 << 20)
+    three = ctypes.c_int64 * 3
+    st = three(128 * 64, 128 * 64, 64)
+    good = dict(q=a, k=a, v=a, q_strides=st, k_strides=st, v_strides=st, dtype=_lib.BF16, B=1, H=1, N=128, D=64, n_text=8, F=2,
+                Hh=3, W=20, order_ids=a, rope_mode=_lib.ROPE_COMPLEX_F64, cos_tab=a, pairs_f=10, pairs_h=11, smooth_k=1,
+                smooth_v=1, plan_slices=1, out=a, out_strides=st, sm_scale=0.125, workspace=a, workspace_bytes=1 << 20)
+
+    def refused(code, text, **changed):
+        args = _lib.LayerArgs(**dict(good, **changed))
+        assert L.paro_layer(args, None) == code and text in L.paro_last_error(), changed
+    assert L.paro_layer(None, None) == _lib.PARO_EINVAL
+    need = L.paro_layer_workspace_bytes(_lib.LayerArgs(**good))
+    assert 0 < need <= 1 << 20
+    assert L.paro_layer_workspace_bytes(_lib.LayerArgs(**dict(good, D=96))) == 0 and L.paro_layer_workspace_bytes(None) == 0
+    refused(_lib.PARO_ESHAPE, b"sizes", N=0)
+    refused(_lib.PARO_ESHAPE, b"sizes", D=96)
+    refused(_lib.PARO_ECAP, b"work space", workspace_bytes=need - 1)
+    refused(_lib.PARO_ECAP, b"work space", workspace=a + 8)
+    refused(_lib.PARO_ECAP, b"work space", workspace=None)
+    for t in "qkv":
+        refused(_lib.PARO_EINVAL, t.encode() + b"): null", **{t: None})
+        refused(_lib.PARO_EALIGN, t.encode() + b")", **{t: a + 2})
+        refused(_lib.PARO_EALIGN, t.encode() + b")", **{t + "_strides": three(128 * 64, 128 * 64, 68)})
+    refused(_lib.PARO_EINVAL, b"dtype", dtype=5)
+    refused(_lib.PARO_ESHAPE, b"!= N", n_text=9)
+    refused(_lib.PARO_ESHAPE, b"!= N", F=-2, n_text=248)
+    refused(_lib.PARO_EINVAL, b"rope_mode", rope_mode=4)
+    refused(_lib.PARO_EINVAL, b"tables missing", cos_tab=None)
+    refused(_lib.PARO_ESHAPE, b"pairs_f", pairs_f=30)
+    refused(_lib.PARO_EINVAL, b"norm_mode", q_norm_mode=3)
+    refused(_lib.PARO_EINVAL, b"norm weight", k_norm_mode=_lib.NORM_RMS_ALL)
+    refused(_lib.PARO_EINVAL, b"takes no bias", k_norm_mode=_lib.NORM_RMS_ALL, k_norm_weight=a, k_norm_bias=a)
+    refused(_lib.PARO_EINVAL, b"eps", q_norm_mode=_lib.NORM_LAYER_HEAD, q_norm_weight=a, q_norm_eps=-1.0)
+
+
+def test_plan_calls_refuse_bad_arguments():
+    L = _lib.lib()
+    buf, a = aligned_buffer(1 << 16)
+    need = L.paro_plan_scratch_bytes(1, 8, 8, 1)
+    assert 0 < L.paro_plan_scratch_bytes(1, 8, 8, 0) < need and L.paro_plan_scratch_bytes(0, 8, 8, 1) == 0
+
+    def offsets(code, mask=a, slices=1, nbq=8, nbk=8, overlap=1, row_ptr=a, pair_q=a, scratch=a, size=need):
+        assert L.paro_plan_offsets(mask, slices, nbq, nbk, overlap, row_ptr, a, pair_q, a, scratch, size, None) == code
+
+    def lists(code, slices=1, nbq=8, nbk=8, overlap=1, pair_q=a, cols=a, sched=a, scratch=a, size=need):
+        assert L.paro_plan_lists(slices, nbq, nbk, overlap, a, a, pair_q, cols, a, sched, a, None, scratch, size, None) == code
+    for call in (offsets, lists):
+        call(_lib.PARO_EINVAL, pair_q=None)
+        call(_lib.PARO_ESHAPE, slices=0)
+        call(_lib.PARO_ESHAPE, nbk=0)
+        call(_lib.PARO_ESHAPE, nbk=0xFFFF)
+        call(_lib.PARO_ESHAPE, nbq=0xFFFF, nbk=1)
+        call(_lib.PARO_ESHAPE, slices=1 << 15, nbq=1 << 8, nbk=1 << 8)
+        call(_lib.PARO_ECAP, size=need - 1)
+        call(_lib.PARO_ECAP, scratch=None)
+        call(_lib.PARO_ECAP, scratch=a + 8)
+    offsets(_lib.PARO_EINVAL, mask=None)
+    offsets(_lib.PARO_EINVAL, row_ptr=None)
+    lists(_lib.PARO_EINVAL, cols=None)
+    lists(_lib.PARO_EINVAL, sched=None)

@@ -4,6 +4,7 @@ import torch
 
 import paroatten_b200 as pb
 from oracle import paro_oracle as po
+from paroatten_b200 import _lib
 from paroatten_b200.plan import pair_rows_by_overlap
 
 pytestmark = pytest.mark.gpu
@@ -48,3 +49,34 @@ def test_pairing_and_lists(mask):
     pq[:, :nbq] = order.to(torch.int32)
     assert torch.equal(plan.pair_q.cpu().view(S, -1), pq)
     assert torch.equal(plan.sched_cnt_kernel.cpu(), cnt | ((pq.view(-1, 2) + 1) << 16))
+
+
+@pytest.mark.parametrize("mask", [bernoulli(1, 1182, 64, 0.2), bernoulli(1, 1701, 65, 0.3), bernoulli(1, 2100, 64, 0.2),
+                                  bernoulli(1, 3333, 40, 0.4), twins(1216), twins(2177)], ids=lambda m: "x".join(map(str, m.shape)))
+def test_pairing_of_long_slices(mask):
+    """Up to eight warps, fewer than 32 rows of overlaps in shared memory at a time, and more than one pass over the
+    candidates (2048 q-blocks)."""
+    test_pairing_and_lists(mask)
+
+
+@pytest.mark.parametrize("mask", [bernoulli(1, 1, 1, 1.0), bernoulli(3, 4, 4, 0.5), bernoulli(2, 5, 9, 0.5), bernoulli(2, 31, 33, 0.3),
+                                  bernoulli(2, 65, 1025, 0.1), bernoulli(1, 130, 2100, 0.6), bernoulli(2, 40, 40, 0.0)],
+                         ids=lambda m: "x".join(map(str, m.shape)))
+def test_the_three_call_form_gives_the_lists_of_adjacent_pairs(mask):
+    """paro_plan_count, _fill and _schedule against the lists of the two-call form, word by word."""
+    plan = pb.compact_plan(mask.cuda())
+    L, s = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    S, nbq, nbk = mask.shape
+    m = mask.to(torch.uint8).cuda()
+    npairs = (nbq + 1) // 2
+    new = lambda *n: torch.full(n, -7, dtype=torch.int32, device="cuda")
+    row_ptr, pair_ptr = new(S * nbq + 1), new(S * npairs + 1)
+    _lib.check(L.paro_plan_count(m.data_ptr(), S, nbq, nbk, row_ptr.data_ptr(), pair_ptr.data_ptr(), s))
+    kept, tiles = int(row_ptr[-1]), int(pair_ptr[-1])
+    cols, pair_ent, sched, cnt = new(kept), new(tiles), new(tiles), new(S * npairs, 2)
+    _lib.check(L.paro_plan_fill(m.data_ptr(), S, nbq, nbk, row_ptr.data_ptr(), cols.data_ptr(), kept, pair_ptr.data_ptr(),
+                                pair_ent.data_ptr(), tiles, s))
+    _lib.check(L.paro_plan_schedule(pair_ptr.data_ptr(), pair_ent.data_ptr(), S, nbq, nbk, sched.data_ptr(), cnt.data_ptr(), s))
+    for got, want in ((row_ptr, plan.row_ptr), (pair_ptr, plan.pair_ptr), (cols, plan.cols), (pair_ent, plan.pair_ent),
+                      (sched, plan.sched), (cnt, plan.sched_cnt)):
+        assert torch.equal(got, want)
