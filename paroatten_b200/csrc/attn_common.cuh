@@ -113,9 +113,6 @@ __device__ __forceinline__ int ld_acquire_shared(const volatile int* ptr) {
                : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_shared(volatile int* ptr, int v) {
-  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(umma::smem_u32(const_cast<int*>(ptr))), "r"(v) : "memory");
-}
 // The same by the lanes for which `pred` holds, as one predicated instruction (no divergent branch: see
 // umma::mbar_arrive_if).
 __device__ __forceinline__ void st_release_shared_if(volatile int* ptr, int v, bool pred) {

@@ -88,12 +88,6 @@ template <int D> struct AttnCfg {
   static constexpr int SMEM_BYTES = TILE_BYTES + AUX_BYTES + 1024 /* alignment slack */;
 };
 
-#define ATT_WAIT(bar, parity, where, iter)                                   \
-  if (!mbar_wait_bounded((bar), (parity), abort_flag, WAIT_LIMIT)) {         \
-    report_timeout(p, abort_flag, (where), (iter));                          \
-    break;                                                                   \
-  }
-
 // FIXED = false: exact running row maximum (online softmax, lazy rescaling of O).
 // FIXED = true:  the row's reference exponent is fixed when its FIRST kept block has been seen (that
 //   block's maximum + REF_OFFSET) and P = 2^(s - m_ref) is kept in bf16 (8 exponent bits) and summed in

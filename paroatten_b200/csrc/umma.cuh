@@ -237,55 +237,9 @@ __device__ __forceinline__ void mma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]^T, int8 operands (A: four values per 32-bit TMEM column), int32 accumulator.
-__device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]^T, fp16 operands, fp32 accumulator.
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Same two operations with a 128-bit mask of accumulator lanes (rows) that are NOT written.
-__device__ __forceinline__ void mma_i8_ts_masked(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate, uint32_t m0, uint32_t m1, uint32_t m2,
-                                                 uint32_t m3) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
-      : "memory");
-}
-__device__ __forceinline__ void mma_f16_ts_masked(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                  uint32_t accumulate, uint32_t m0, uint32_t m1, uint32_t m2,
-                                                  uint32_t m3) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
-      : "memory");
-}
 // Arrives once on `bar` when every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void mma_commit_at(uint32_t bar_saddr) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_saddr)
                : "memory");
 }
 
@@ -302,6 +256,8 @@ __device__ __forceinline__ uint32_t elect_one() {
       : "=r"(lead));
   return lead;
 }
+// D[tmem] (+)= A[tmem] * B[smem]^T: int8 operands (A: four values per 32-bit TMEM column) with an int32 accumulator, 16-bit
+// operands with an fp32 one; _masked: with a 128-bit mask of accumulator lanes (rows) that are NOT written.
 __device__ __forceinline__ void mma_i8_ts_p(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -350,6 +306,9 @@ __device__ __forceinline__ void mma_f16_ts_masked_p(uint32_t lead, uint32_t d_tm
 // hold accumulator columns of B's rows 0..N/2-1, lanes 64-127 those of rows N/2..N-1, and each half of the
 // lanes multiplies by the A rows that lie in its own lanes.  With different A rows in the two halves ONE
 // instruction therefore computes two independent 64-row products, A_lo * B_lo^T and A_hi * B_hi^T.
+// (The split of N is the PTX ISA's accumulator layout of M = 64 with .ws.  Which A rows a half reads is not spelled out
+// there for halves that differ: it was measured here, random int8 and bf16 operands against the host's products, and
+// every side-by-side step of the attention tests depends on it.)
 __device__ __forceinline__ void mma_ws_i8_ts_p(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
                                                uint32_t idesc, uint32_t accumulate) {
   asm volatile(
