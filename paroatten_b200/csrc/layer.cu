@@ -20,9 +20,9 @@ struct Sections {
   size_t q8, k8, v16, qs, ks, vs, vm, km, kp, rms_q, rms_k, tab32, stats, total;
 };
 
-// Elements of Q from which the passes get the fp32 copy of an interleaved fp64 table, made for the call: 2 us, which Q
-// and K of 2 x 12 x 1560 x 128 give back twice over (bf16: 29.6 -> 24.9 us) and those of 3 x 4200 x 128 barely (18.2 ->
-// 15.2), where the launches of a layer take longer than its passes.
+// Elements of Q from which the passes get the fp32 copy of an interleaved fp64 table, made for the call: a launch of 2 us.
+// Layers without it and with it, bf16: 4 x 2080 x 128 63.4 and 65.1 us, 8 x 4160 x 128 91.8 and 92.0, 8 x 6240 x 128 136.4 and
+// 130.9, 24 x 6240 x 128 302 and 290 (fp16 300 and 292; with RMS norm level from here on).
 constexpr int64_t FP32_TABLE_ELEMS = 4 << 20;
 bool fp32_table(const paro_layer_args& a) {
   return a.rope_mode == PARO_ROPE_COMPLEX_F64 && a.cos_tab && !a.sin_tab && a.F > 0 && a.Hh > 0 && a.W > 0 &&

@@ -40,9 +40,9 @@ class RopeTables:
 _NO_ROPE = (_lib.ROPE_NONE, 0, 0, 0, 0)
 
 # Elements of a tensor from which a pass over it takes the fp32 copy of an fp64 table along.  Making the copy costs 2 us on
-# the device and 6 on the host; it takes 2 us off a pass over 5 million elements (2 x 12 x 1560 x 128, INT8 Q in bf16:
-# 16.6 -> 14.5 us) and 8 us off one over 24 million (40 x 4680 x 128: 46.5 -> 38.5 us).
-FP32_COPY_ELEMS = 16 << 20
+# the device and 10 on the host.  Q, smoothed K and V in bf16 without it and with it: 8 x 6240 x 128 89 and 109 us (host),
+# 14 x 5989 x 128 122 and 118, 24 x 6240 x 128 162 and 153; in fp16 the last two 122 and 123, 159 and 158.
+FP32_COPY_ELEMS = 10 << 20
 
 
 def _rope_args(rope: Optional[RopeTables], numel: int):
