@@ -147,7 +147,10 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // one thread decides for the whole CTA whether an earlier failure makes this launch drain (every
   // thread reading the word for itself could split the CTA around the collective operations below)
-  if (threadIdx.x == 0) *s_drain = *reinterpret_cast<volatile int32_t*>(p.status) != 0;
+  if (threadIdx.x == 0) {
+    *s_drain = *reinterpret_cast<volatile int32_t*>(p.status) != 0;
+    if (FIXED && p.redo_next && blockIdx.x == 0) *p.redo_next = 0;   // (the launch after this one counts there)
+  }
   __syncthreads();
   if (*s_drain) return;
   // The pair's schedule: entry i = kbA | kbB << 16 (0xFFFF: no tile for that half in step i).  First
@@ -171,7 +174,6 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     n_steps = max(n_a, n_b);
   };
   set_item(LIST ? p.redo[REDO_HEADER + list_at] : (int)blockIdx.x);
-  if (FIXED && p.redo_next && blockIdx.x == 0 && threadIdx.x == 0) *p.redo_next = 0;   // (read by the launch after this one)
   // A step is one group of MMAs of each kind: FORM_UPPER / FORM_LOWER when only one half still has blocks (128
   // rows, the other half's accumulator rows masked), FORM_SHARED when both keep the same block (one tile, 128
   // rows) and FORM_DUAL when each half has its own (two tiles, tcgen05.mma.ws: two 64-row products in one
