@@ -126,8 +126,8 @@ extern "C" int paro_layer(const paro_layer_args* args, paro_stream_t stream) {
   if (!a.smooth_k) {
     if (int rc = prep(a.k, a.k_strides, 64, a.k_norm_mode, a.k_norm_weight, a.k_norm_bias, rms, a.k_norm_eps, k8, ks)) return rc;
   } else {
-    // The mean to subtract is that of the rotated values.  The rotated copy is written once and read twice: 122 us for
-    // 5 x 75600 x 128 with the fp64 rotation, 235 us for 2 x 48 x 17776 x 64 with the fp32 one, against 163 and 265 us for
+    // The mean to subtract is that of the rotated values.  The rotated copy is written once and read twice: 127 us for
+    // 5 x 75600 x 128 with the fp64 rotation, 227 us for 2 x 48 x 17776 x 64 with the fp32 one, against 152 and 264 us for
     // rotating K in the statistics pass and again in the quantiser.
     kp = w + at.kp;
     const int rc = a.k_norm_mode == PARO_NORM_NONE

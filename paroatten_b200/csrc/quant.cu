@@ -219,9 +219,9 @@ channel_finalize_kernel(const FinalizeDst<T> dst0, const FinalizeDst<T> dst1, in
 // INT8: one CTA = `blocks` consecutive 64-token blocks of one (b,h); warp w owns 64/WARPS tokens of each.
 // 2 bytes in, 1 byte out per element.
 // Passes that rotate (TABLE): 256 threads; source tokens and table rows of all the CTA's blocks are worked out once
-// into shared memory.  Four blocks per CTA against one: 190 -> 140 us for 2 x 48 x 17776 x 64 with the fp32 rotation,
-// 257 -> 204 us for 2 x 12 x 32760 x 128 with RMS norm and the fp64 rotation.  (Loading the next block's rows ahead
-// costs the registers of a third CTA per SM: 148, 239 us.  Four CTAs per SM at D = 64, where a thread holds two rows and
+// into shared memory.  Four blocks per CTA against one: 109 -> 73 us for 48 x 17776 x 64 with the fp32 rotation,
+// 113 -> 100 us for 12 x 32760 x 128 with RMS norm and the fp64 rotation.  (Loading the next block's rows ahead
+// costs the registers of a third CTA per SM, 6 and 17 % more.  Four CTAs per SM at D = 64, where a thread holds two rows and
 // not four: Q of 2 x 48 x 17776 x 64 184 -> 168 us with the fp64 rotation, 244 -> 221 with LayerNorm and the fp32 one; at
 // D = 128 with a norm the fourth costs spills, RMS 197 -> 205 us.)
 // Passes that do not: 128 threads with twice the rows in flight each, one block per CTA, source tokens by shuffle (the
