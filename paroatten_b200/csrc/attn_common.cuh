@@ -83,6 +83,14 @@ __device__ __forceinline__ uint32_t ld_pinned_u32(const uint32_t* ptr) {
   asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(ptr));
   return v;
 }
+__device__ __forceinline__ float ld_pinned_f32(const float* ptr) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(ptr));
+  return v;
+}
+__device__ __forceinline__ void ld_shared_scale(uint32_t saddr, float& scale, int& valid) {
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(scale), "=r"(valid) : "r"(saddr) : "memory");
+}
 __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }

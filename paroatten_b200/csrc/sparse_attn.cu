@@ -69,6 +69,7 @@ __device__ long long g_trace[16][160][8];
 #endif
 constexpr float RESCALE_TAU = 8.0f;            // exact walk: rescale O only when the row max grows by > 2^8
 constexpr float REF_OFFSET = 20.f;             // fixed reference: the first block's maximum maps to P = 2^-20
+constexpr int KS_RING = 8;                     // steps whose K scales are kept (more than a ring holds and one)
 constexpr float ROWSUM_LIMIT = 1.2676506e30f;  // 2^100: a step's row sum beyond it gives the pair back
 
 template <int D> struct AttnCfg {
@@ -140,7 +141,12 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   float* s_vm = s_vscale + D;                              // [D]
   volatile float* s_mrow = reinterpret_cast<volatile float*>(aux + 1536);   // [128] running row maximum
   float* s_xl = reinterpret_cast<float*>(aux + 2048);                       // [2][128] row-sum exchange
-  static_assert(512 + 2 * D * 4 <= 1536 && 2048 + 2 * 128 * 4 <= Cfg::AUX_BYTES, "aux area too small");
+  // What the softmax warps need of a step's k-block: [half][step mod KS_RING] scale of K and columns inside the
+  // sequence, written by the K producer before it asks for the tile.  Looked up by the softmax warps themselves (plan entry,
+  // then scale, both from global memory) it held each of them for 300 clocks of a step of 3150: 5 heads x 75600 x 128 at
+  // density 0.2 2.234 -> 2.170 ms, 2 x 12 x 32760 x 128 at 0.3 3.037 -> 2.968, 2 x 48 x 17776 x 64 3.716 -> 3.607.
+  float2* s_kstep = reinterpret_cast<float2*>(aux + 3072);
+  static_assert(512 + 2 * D * 4 <= 1536 && 3072 + 2 * KS_RING * 8 <= Cfg::AUX_BYTES, "aux area too small");
   static_assert((27 + KST + VST) * 8 + 8 + 32 <= 512, "barrier area too small");
 
   // (the warp index through a shuffle: provably the same in all lanes, so the role branches are uniform)
@@ -255,10 +261,24 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         };
         // schedule entries are fetched two steps ahead of their use
         uint32_t e_cur = n_steps > 0 ? sched[0] : 0u, e_nxt = n_steps > 1 ? sched[1] : 0u;
+        // the scales one step ahead (a k-block id beyond the sequence can only be the filler or come from a
+        // malformed plan; clamped so that the look-up stays inside its array)
+        [[maybe_unused]] const float* kscale_bh = p.k_scale + (size_t)bh * p.nb;
+        [[maybe_unused]] auto k_scale = [&](uint32_t id) { return ld_pinned_f32(kscale_bh + min((int)id, p.nb - 1)); };
+        [[maybe_unused]] float sa = 0.f, sb = 0.f;
+        if (IS_K && n_steps > 0) {
+          sa = k_scale(e_cur & 0xFFFFu);
+          sb = k_scale(e_cur >> 16);
+        }
         for (int i = 0; i < n_steps; ++i) {
           const uint32_t ka = e_cur & 0xFFFFu, kb = e_cur >> 16;
           e_cur = e_nxt;
           if (i + 2 < n_steps) e_nxt = ld_pinned_u32(sched + i + 2);
+          [[maybe_unused]] const float sa_i = sa, sb_i = sb;
+          if (IS_K && i + 1 < n_steps) {
+            sa = k_scale(e_cur & 0xFFFFu);
+            sb = k_scale(e_cur >> 16);
+          }
           const uint32_t first = ka != 0xFFFFu ? ka : kb;   // the tile at the front of the slot
           if (first == 0xFFFFu) continue;
           const bool two = ka != 0xFFFFu && kb != 0xFFFFu && ka != kb;
@@ -271,6 +291,11 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           held.push(commit_token(a_done, ka != 0xFFFFu ? 0 : 1, i));   // (a step of both halves commits to both)
           ++t;
           TR(trole, i, 1);
+          if constexpr (IS_K) {   // (the slot's previous readers copied their scores before the K slot came back)
+            auto valid = [&](uint32_t id) { return __int_as_float(min(64, p.N - min((int)id, p.nb - 1) * 64)); };
+            if (ka != 0xFFFFu) s_kstep[i % KS_RING] = make_float2(sa_i, valid(ka));
+            if (kb != 0xFFFFu) s_kstep[KS_RING + i % KS_RING] = make_float2(sb_i, valid(kb));
+          }
           mbar_arrive_expect_tx(bar_full + st, two ? 2 * BYTES : BYTES);
           load(ring + st * 2 * BYTES, first, bar_full + st);
           if (two) load(ring + st * 2 * BYTES + BYTES, kb, bar_full + st);
@@ -458,7 +483,6 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int half = qd >> 1;                // which q-block of the pair
     const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
     const int n_mine = half ? n_b : n_a;
-    auto my_kb = [&](int i) { return (int)((sched[i] >> (16 * half)) & 0xFFFFu); };   // this half's k-block of step i
     if (threadIdx.x < D) {
       s_vscale[threadIdx.x] = p.v_scale[(size_t)bh * D + threadIdx.x];
       s_vm[threadIdx.x] = p.vm ? p.vm[(size_t)bh * D + threadIdx.x] : 0.f;
@@ -506,26 +530,19 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     uint64_t* const my_sfree = bar_sfree + 2 * half + set;
     uint64_t* const my_pready = bar_pready + 2 * half + set;
     const uint32_t my_sready = smem_u32(bar_sready + 4 * half), my_pvdone = smem_u32(bar_pvdone + 4 * half);   // [step mod 4]
-    const float* kscale_bh = p.k_scale + (size_t)bh * p.nb;
-    // (a k-block id beyond the sequence can only come from a malformed plan; clamped so that the scale
-    // look-up stays inside its array)
-    int kb_next = set < n_mine ? min(my_kb(set), p.nb - 1) : 0;
-    float ks_next = set < n_mine ? kscale_bh[kb_next] : 0.f;
+    const uint32_t my_kstep = smem_u32(s_kstep + KS_RING * half);
     // One step of this thread's half (the two halves only meet in the issuers' queues).  `first` is a
     // compile-time tag: the thread's first step, where the fixed-reference walk settles the row's
     // reference exponent; every later step of that walk is straight-line code from scores to P.
     auto do_step = [&](const int i, auto first) -> bool {
       [[maybe_unused]] constexpr bool FIRST = decltype(first)::value;
-      const int kb = kb_next;
-      const float kscale = ks_next;
-      if (i + 2 < n_mine) {   // fetched one step ahead so that the loads are off the critical path
-        kb_next = min(my_kb(i + 2), p.nb - 1);
-        ks_next = kscale_bh[kb_next];
-      }
       [[maybe_unused]] const int trole = 4 + warp;
       TR(trole, i, 0);
       if (!wait_bar(my_sready + 8u * (i & 3), i >> 2, 6, i)) return false;
       TR(trole, i, 1);
+      float kscale;
+      int valid;   // columns inside the sequence
+      ld_shared_scale(my_kstep + 8u * (uint32_t)(i % KS_RING), kscale, valid);
       float f[64];
       {
         uint32_t s[64];
@@ -549,7 +566,6 @@ sparse_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 64; ++j) f[j] = __int_as_float((int)s[j] + 0x4B400000);
       }
-      const int valid = min(64, p.N - kb * 64);   // columns inside the sequence
       const float sc = rowscale * kscale;
       if (!FIXED && valid < 64) {   // (the fixed-reference walk corrects its row sum instead, below)
 #pragma unroll
