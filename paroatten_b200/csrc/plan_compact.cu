@@ -9,8 +9,8 @@
 //   lists     the CSR lists, the merged lists and the walk schedule of a pair, written by one warp
 //
 // The host reads three totals back between count and lists (the lists' lengths), once per call.
-// Measured on a 40 x 1182 x 1182 mask at density 0.2: 0.58 ms on the device (pack 48 us, overlap 98, pair 290, count and
-// scans 17, lists 110) and 0.8 ms for the whole call; a fp32 bmm with 591 rounds of small torch kernels took 67 ms.
+// Measured on a 40 x 1182 x 1182 mask at density 0.2: 0.39 ms on the device (pack 25 us, overlap 96, pair 184, count and
+// scans 12, lists 74); a fp32 bmm with 591 rounds of small torch kernels took 67 ms.
 #include "common.cuh"
 #include "umma.cuh"
 
@@ -23,7 +23,7 @@ struct PlanScratch {
   uint32_t* bits;      // [slices*nbq][words]
   int32_t* row_cnt;    // [slices*nbq] kept blocks per q-block, mask order
   int32_t* part;       // [2][scan blocks] partial sums of the two scans
-  uint16_t* ov;        // [slices*nbq][pitch] overlaps (pairing by overlap only); entries left of the diagonal tile are not written
+  uint16_t* ov;        // [slices*nbq][pitch] overlaps + 1 (pairing by overlap only); entries left of the diagonal tile are not written
   int words, pitch, scan_blocks;
   size_t bytes;
 };
@@ -50,31 +50,56 @@ static PlanScratch plan_scratch(void* base, int slices, int nbq, int nbk, int ov
   return s;
 }
 
-// One warp per mask row; bound by the mask's bytes.  A row starts at any byte, so lanes read single bytes (32 of them are
-// one sector) and a ballot makes the word; eight words are in flight per warp.
+// One bit per byte: 1 where the byte is not 0, byte 0 in bit 0.
+__device__ __forceinline__ uint32_t nonzero_bits(uint32_t x) {
+  const uint32_t m = ((((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) >> 7) & 0x01010101u;
+  return m * 0x01020408u >> 24;
+}
+// One warp per mask row; bound by the mask's bytes.  A row starts at any byte: lanes load the aligned 16-byte pieces that
+// it lies in, all of a turn first, turn each into 16 bits and shift words together from three neighbours.  (Single bytes and
+// a ballot per word, eight in flight: 47 us for 40 x 1182 x 1182; one piece per lane ahead 26; this 25.)
+constexpr int PACK_PIECES = 3;   // pieces of 32 x 16 bytes in flight per row
 __global__ void __launch_bounds__(256)
 plan_pack_kernel(const uint8_t* __restrict__ mask, int rows, int nbk, int words, uint32_t* __restrict__ bits,
                  int32_t* __restrict__ row_cnt) {
   const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  const uint8_t* const end = mask + (size_t)rows * nbk;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
-    const uint8_t* src = mask + (size_t)r * nbk;
+    const uint8_t* row = mask + (size_t)r * nbk;
+    const int shift = (int)(reinterpret_cast<uintptr_t>(row) & 15u);
+    const uint8_t* src = row - shift;
     int cnt = 0;
-    for (int w0 = 0; w0 < words; w0 += 8) {
-      uint8_t v[8];
+    for (int w0 = 0; w0 < words; w0 += 16 * PACK_PIECES) {   // (one turn for up to 1520 k-blocks)
+      uint4 v[PACK_PIECES + 1];
+      uint32_t b[PACK_PIECES + 1];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int kb = (w0 + u) * 32 + lane;
-        v[u] = kb < nbk ? src[kb] : 0;
+      for (int u = 0; u <= PACK_PIECES; ++u) {   // (of the last piece only what the one before is shifted together with)
+        const uint8_t* at = src + 16 * (size_t)(2 * w0 + 32 * u + lane);
+        v[u] = make_uint4(0, 0, 0, 0);
+        if ((u < PACK_PIECES || lane == 0) && at < row + nbk && at >= mask && at + 16 <= end) v[u] = *reinterpret_cast<const uint4*>(at);
       }
-      uint32_t mine = 0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const uint32_t b = __ballot_sync(0xffffffffu, v[u] != 0);
-        cnt += __popc(b);
-        if (lane == u) mine = b;
+      for (int u = 0; u <= PACK_PIECES; ++u) {
+        const uint8_t* at = src + 16 * (size_t)(2 * w0 + 32 * u + lane);
+        b[u] = nonzero_bits(v[u].x) | nonzero_bits(v[u].y) << 4 | nonzero_bits(v[u].z) << 8 | nonzero_bits(v[u].w) << 12;
+        if ((u < PACK_PIECES || lane == 0) && at < row + nbk && (at < mask || at + 16 > end))   // reaches past an end of the mask: byte by byte
+          for (int k = 0; k < 16; ++k)
+            if (at + k >= mask && at + k < end && at[k]) b[u] |= 1u << k;
       }
-      if (lane < 8 && w0 + lane < words) bits[(size_t)r * words + w0 + lane] = mine;
+#pragma unroll
+      for (int u = 0; u < PACK_PIECES; ++u) {
+        const uint32_t lo = __shfl_sync(0xffffffffu, b[u], 2 * lane), mid = __shfl_sync(0xffffffffu, b[u], 2 * lane + 1);
+        const uint32_t next0 = __shfl_sync(0xffffffffu, b[u + 1], 0), after = __shfl_sync(0xffffffffu, b[u], 2 * lane + 2);
+        const int w = w0 + 16 * u + lane, left = nbk - 32 * w;   // (columns of the row from this word on)
+        if (lane < 16 && w < words) {
+          uint32_t word = __funnelshift_r(lo | mid << 16, lane < 15 ? after : next0, shift);
+          word &= left >= 32 ? 0xffffffffu : left > 0 ? (1u << left) - 1u : 0u;
+          bits[(size_t)r * words + w] = word;
+          cnt += __popc(word);
+        }
+      }
     }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
     if (lane == 0) row_cnt[r] = cnt;
   }
 }
@@ -157,6 +182,7 @@ plan_overlap_kernel(const uint32_t* __restrict__ bits, int slices, int nbq, int 
     // warp w: lanes (rows) of quadrant w & 3, 64 of the 128 columns
     const int orow = ti * OV_TILE + (warp & 3) * 32 + lane, col0 = tj * OV_TILE + (warp >> 2) * 64;
     uint16_t* dst = ov + ((size_t)slice * nbq + orow) * pitch;
+    constexpr uint32_t ONE = 0x00010001u;   // (at most 65534 k-blocks: the increment stays in its half)
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       uint32_t o[32];
@@ -166,8 +192,8 @@ plan_overlap_kernel(const uint32_t* __restrict__ bits, int slices, int nbq, int 
       for (int g = 0; g < 4; ++g) {
         const int c8 = col0 + 32 * q + 8 * g;   // (the pitch is a multiple of 8: a group is inside or outside as a whole)
         if (orow < nbq && c8 < pitch)
-          *reinterpret_cast<uint4*>(dst + c8) = make_uint4(o[8 * g] | o[8 * g + 1] << 16, o[8 * g + 2] | o[8 * g + 3] << 16,
-                                                           o[8 * g + 4] | o[8 * g + 5] << 16, o[8 * g + 6] | o[8 * g + 7] << 16);
+          *reinterpret_cast<uint4*>(dst + c8) = make_uint4((o[8 * g] | o[8 * g + 1] << 16) + ONE, (o[8 * g + 2] | o[8 * g + 3] << 16) + ONE,
+                                                           (o[8 * g + 4] | o[8 * g + 5] << 16) + ONE, (o[8 * g + 6] | o[8 * g + 7] << 16) + ONE);
       }
     }
     tc_fence_before();
@@ -184,125 +210,148 @@ plan_overlap_kernel(const uint32_t* __restrict__ bits, int slices, int nbq, int 
   }
 }
 
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src)
-               : "memory");
-}
-
 // Greedy pairing of one slice per CTA: the first q-block not yet paired takes the free q-block it shares most
-// k-blocks with (ties: the lowest index).  The nbq/2 rounds are a serial chain, so the latency of a round is what
-// counts: one barrier per round (the bit of the q-block taken last may not have reached every thread yet; it is
-// carried in a register instead), eight candidates per thread and load, the word of the free map around the current row in a
-// register, and, since the first free q-block only moves forward, the overlap rows are brought to shared memory
-// `1 << chunk_log` rows at a time, one chunk ahead.  chunk_log < 0: rows too long for shared memory, read where they are.
-// (591 rounds: 290 us; with two-byte candidates and the free map searched in shared memory 500 us.)
+// k-blocks with (ties: the lowest index).  The rounds are a serial chain, so they are run PAIR_WARPS at a time: warp k finds
+// the best partner of the (k+1)-th free q-block on the assumption that none of the q-blocks before it takes anything it
+// wants, and the results are accepted in order up to the first that wanted a q-block already taken (a q-block that was
+// itself taken as a partner is passed over).  What the others found is kept: it is still the best as long as the
+// partner is free.  (1182 rows at density 0.2: 86 turns of seven pairs.  591 rounds of one pair, all warps on one row, 290 us;
+// this 184, the rows read from L2 where they lie.  Staged through shared memory 16 rows at a time they arrive too
+// late, 228 us.)  A candidate's key is its overlap + 1 (0: not free); a lane looks at eight per load.
 // A pairing that does not need fewer tiles than adjacency is replaced by adjacency; any[0] = 1 if one was kept.
-constexpr int PAIR_THREADS = 256, PAIR_MAX_ROWS = 65536;
+constexpr int PAIR_WARPS = 8, PAIR_THREADS = 32 * PAIR_WARPS, PAIR_MAX_ROWS = 65536, PAIR_LOADS = 5;
 __global__ void __launch_bounds__(PAIR_THREADS)
-plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs, int chunk_log, int32_t* __restrict__ pair_q,
+plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs, int32_t* __restrict__ pair_q,
                  int32_t* __restrict__ any) {
-  extern __shared__ __align__(16) uint16_t s_rows[];
-  __shared__ uint32_t s_free[PAIR_MAX_ROWS / 32];   // bit per q-block, as words and as bytes (byte t: rows 8t..8t+7)
-  __shared__ __align__(16) uint32_t s_part[2][8];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x;
+  __shared__ uint32_t s_free[PAIR_MAX_ROWS / 32 + 1];   // bit per q-block, as words and as bytes (byte t: rows 8t..8t+7)
+  __shared__ int2 s_found[32];             // [row mod 32] (row, its best partner so far or -1); the window spans 32 rows
+  __shared__ uint32_t s_overlap[32];       // their overlap + 1
+  __shared__ uint32_t s_part[PAIR_WARPS];
+  __shared__ int s_keep;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint8_t* s_free8 = reinterpret_cast<const uint8_t*>(s_free);
   const uint16_t* o = ov + (size_t)blockIdx.x * nbq * pitch;
   int32_t* out = pair_q + (size_t)blockIdx.x * npairs * 2;
-  for (int w = tid; w < (nbq + 31) / 32; w += threads)
-    s_free[w] = nbq - 32 * w >= 32 ? 0xffffffffu : (1u << (nbq - 32 * w)) - 1u;
-  if (tid < 16) s_part[tid >> 3][tid & 7] = 0;
-
-  int loaded = -1;   // newest chunk requested
-  auto load = [&](int c) {
-    loaded = c;
-    const int r0 = c << chunk_log;
-    if (r0 >= nbq) return;
-    const int n16 = min(1 << chunk_log, nbq - r0) * (pitch / 8);
-    const uint4* src = reinterpret_cast<const uint4*>(o + (size_t)r0 * pitch);
-    uint4* dst = reinterpret_cast<uint4*>(s_rows + (size_t)(c & 1) * ((size_t)pitch << chunk_log));
-    for (int k = tid; k < n16; k += threads) cp_async16(dst + k, src + k);
-  };
-  if (chunk_log >= 0) load(0);
+  const int words = (nbq + 31) / 32, groups = (nbq + 7) / 8;
+  for (int w = tid; w <= words; w += PAIR_THREADS)
+    s_free[w] = nbq - 32 * w >= 32 ? 0xffffffffu : nbq > 32 * w ? (1u << (nbq - 32 * w)) - 1u : 0u;
+  if (tid < 32) s_found[tid] = make_int2(-1, -1);
   __syncthreads();
 
-  int cur = -1, i = -1, gone = -1;
-  long long shared_greedy = 0;
-  int fw = 0;                      // word of the free map that holds the next free q-block after i, as far as known
-  uint32_t fm = s_free[0];         // its bits after i
-  auto next_free = [&]() {         // (the caller knows there is one)
-    for (;;) {
-      if (gone >= 0 && (gone >> 5) == fw) fm &= ~(1u << (gone & 31));
-      if (fm) {
-        const int bit = __ffs(fm) - 1;
-        fm &= fm - 1;
-        return fw * 32 + bit;
-      }
-      fm = s_free[++fw];           // all but the bit of `gone` are up to date: the round before last is behind a barrier
-    }
-  };
-  for (int p = 0; p < nbq / 2; ++p) {
-    i = next_free();
-    const uint16_t* row = o + (size_t)i * pitch;
-    if (chunk_log >= 0) {
-      const int c = i >> chunk_log;
-      if (c != cur) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        if (c != loaded) {          // (the chunks in between held no free q-block)
-          load(c);
-          asm volatile("cp.async.wait_all;" ::: "memory");
-        }
-        __syncthreads();            // the chunk before this one was last read before the previous round's barrier
-        load(c + 1);
-        cur = c;
-      }
-      row = s_rows + (size_t)(c & 1) * ((size_t)pitch << chunk_log) + (size_t)(i - (c << chunk_log)) * pitch;
-    }
-    uint32_t best = 0;
-    for (int j8 = tid * 8; j8 < nbq; j8 += threads * 8) {
-      const uint4 v = *reinterpret_cast<const uint4*>(row + j8);
-      uint32_t m = s_free8[j8 >> 3];
-      if (j8 + 7 <= i) m = 0;
-      else if (j8 <= i) m &= 0xFFu << (i - j8 + 1);
-      if ((gone >> 3) == (j8 >> 3)) m &= ~(1u << (gone & 7));
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  int cursor = 0, done = 0;       // rows before `cursor` are settled; pairs written
+  long long shared_greedy = 0;    // (of warp 0's lanes)
+  while (cursor < nbq) {
+    // the window: up to PAIR_WARPS free rows from the first one on
+    int fw = cursor >> 5;
+    uint32_t fm = s_free[fw] & (0xffffffffu << (cursor & 31));
+    while (!fm && ++fw < words) fm = s_free[fw];
+    if (!fm) break;
+    const int i0 = fw * 32 + __ffs(fm) - 1;
+    const uint32_t win = __funnelshift_r(s_free[fw], s_free[fw + 1], i0 & 31);
+    const int n = min(__popc(win), PAIR_WARPS);
+    if (warp < n) {
+      uint32_t b = win;
+      for (int k = 0; k < warp; ++k) b &= b - 1;
+      const int i = i0 + __ffs(b) - 1;
+      const int2 kept = s_found[i & 31];
+      if (kept.x != i || kept.y < 0 || !(s_free[kept.y >> 5] >> (kept.y & 31) & 1u)) {
+        const uint16_t* row = o + (size_t)i * pitch;
+        // clears the keys of the candidates v of group g that are not free; the largest that is left
+        auto masked = [&](uint4& v, int g) {
+          uint32_t m = s_free8[g];
+          if (g == i >> 3) m &= 0xFEu << (i & 7);   // (only partners after the row)
+          const uint32_t t = m | m << 15;           // bit 2k of the low half: candidate 2k, of the high half: 2k+1
+          v.x &= (t & 0x00010001u) * 0xFFFFu;
+          v.y &= (t >> 2 & 0x00010001u) * 0xFFFFu;
+          v.z &= (t >> 4 & 0x00010001u) * 0xFFFFu;
+          v.w &= (t >> 6 & 0x00010001u) * 0xFFFFu;
+          const uint32_t m2 = __vmaxu2(__vmaxu2(v.x, v.y), __vmaxu2(v.z, v.w));
+          return max(m2 & 0xFFFFu, m2 >> 16);
+        };
+        uint32_t best = 0;   // key << 16 | complement of the group that has it
+        for (int g0 = (i >> 3) + lane; g0 < groups; g0 += 32 * PAIR_LOADS) {
+          uint4 v[PAIR_LOADS];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t key = ((k & 1 ? w[k >> 1] >> 16 : w[k >> 1] & 0xFFFFu) << 16) | (uint32_t)(0xFFFF - j8 - k);
-        best = max(best, m >> k & 1u ? key : 0u);
+          for (int u = 0; u < PAIR_LOADS; ++u)
+            if (g0 + 32 * u < groups) v[u] = *reinterpret_cast<const uint4*>(row + 8 * (g0 + 32 * u));
+#pragma unroll
+          for (int u = 0; u < PAIR_LOADS; ++u)
+            if (g0 + 32 * u < groups) best = max(best, masked(v[u], g0 + 32 * u) << 16 | (uint32_t)(0xFFFF - g0 - 32 * u));
+        }
+        best = __reduce_max_sync(0xffffffffu, best);
+        int partner = -1;
+        if (best >> 16) {
+          const int g = 0xFFFF - (int)(best & 0xFFFFu);
+          uint4 v = *reinterpret_cast<const uint4*>(row + 8 * g);
+          masked(v, g);
+          const uint32_t w = lane & 4 ? (lane & 2 ? v.w : v.z) : (lane & 2 ? v.y : v.x);
+          partner = 8 * g + __ffs(__ballot_sync(0xffffffffu, lane < 8 && (lane & 1 ? w >> 16 : w & 0xFFFFu) == best >> 16)) - 1;
+        }
+        if (lane == 0) {
+          s_found[i & 31] = make_int2(i, partner);
+          s_overlap[i & 31] = best >> 16;
+        }
       }
     }
-    best = __reduce_max_sync(0xffffffffu, best);
-    if (lane == 0) s_part[p & 1][warp] = best;
     __syncthreads();
-    const uint4 x = *reinterpret_cast<const uint4*>(s_part[p & 1]), y = *reinterpret_cast<const uint4*>(s_part[p & 1] + 4);
-    best = max(max(max(x.x, x.y), max(x.z, x.w)), max(max(y.x, y.y), max(y.z, y.w)));
-    gone = 0xFFFF - (int)(best & 0xFFFFu);
-    shared_greedy += best >> 16;
-    if (tid == 0) {
-      s_free[i >> 5] &= ~(1u << (i & 31));
-      s_free[gone >> 5] &= ~(1u << (gone & 31));
-      *reinterpret_cast<int2*>(out + 2 * p) = make_int2(i, gone);
+    // lane k < n: the window's row k and what it found
+    int i = -1, g = -1;
+    uint32_t b = win;
+    for (int k = 0; k < (lane & 7); ++k) b &= b - 1;
+    if ((lane & 7) < n) {
+      i = i0 + __ffs(b) - 1;
+      g = s_found[i & 31].y;
     }
+    // lanes 0-7 hold the partners, 8-15 the rows: who else wants my partner (bits 0-7), which row it is (8-15)
+    static_assert(PAIR_WARPS == 8, "lanes of the match");
+    const int value = lane < 8 ? (g >= 0 ? g : -1 - lane) : lane < 16 ? (i >= 0 ? i : -1 - lane) : -1 - lane;
+    const uint32_t same = __match_any_sync(0xffffffffu, value);
+    const uint32_t others = lane < n ? same & 0xFFFFu & ~(1u << lane) : 0u;
+    // only the rows that meet another one are gone through
+    uint32_t meet = __ballot_sync(0xffffffffu, others != 0) | __reduce_or_sync(0xffffffffu, others >> 8);
+    uint32_t passed = 0;                        // rows taken as a partner
+    uint32_t takers = ((1u << n) - 1u) & ~meet;   // rows that take their partner
+    int stop = n;                               // the first row to be looked at again
+    for (; meet; meet &= meet - 1) {
+      const int k = __ffs(meet) - 1;
+      const uint32_t s = __shfl_sync(0xffffffffu, others, k);
+      if (passed >> k & 1u) continue;
+      if (s & takers & ((1u << k) - 1u)) {
+        stop = k;
+        break;
+      }
+      takers |= 1u << k;
+      passed |= s >> 8;
+    }
+    const uint32_t accepted = takers & ((1u << stop) - 1u);
+    const int last = __shfl_sync(0xffffffffu, i, min(stop, n - 1));
+    cursor = stop < n ? last : last + 1;
+    if (warp == 0 && lane < 8 && (accepted >> lane & 1u)) {
+      const int at = done + __popc(accepted & ((1u << lane) - 1u));
+      atomicAnd(&s_free[i >> 5], ~(1u << (i & 31)));
+      if (g >= 0) atomicAnd(&s_free[g >> 5], ~(1u << (g & 31)));
+      *reinterpret_cast<int2*>(out + 2 * at) = make_int2(i, g);
+      if (g >= 0) shared_greedy += s_overlap[i & 31] - 1;
+    }
+    done += __popc(accepted);
+    __syncthreads();
   }
-  if (nbq & 1) {
-    i = next_free();
-    if (tid == 0) *reinterpret_cast<int2*>(out + nbq - 1) = make_int2(i, -1);
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  // adjacency's shared blocks
-  __syncthreads();
+  // against adjacency's shared blocks
   uint32_t mine = 0;
-  for (int p = tid; p < nbq / 2; p += threads) mine += o[(size_t)(2 * p) * pitch + 2 * p + 1];
+  for (int p = tid; p < nbq / 2; p += PAIR_THREADS) mine += o[(size_t)(2 * p) * pitch + 2 * p + 1] - 1u;
   mine = __reduce_add_sync(0xffffffffu, mine);
-  if (lane == 0) s_part[0][warp] = mine;
+  if (lane == 0) s_part[warp] = mine;
+  for (int k = 4; k > 0; k >>= 1) shared_greedy += __shfl_xor_sync(0xffffffffu, shared_greedy, k);
   __syncthreads();
-  long long shared_adjacent = 0;
-  for (int k = 0; k < threads / 32; ++k) shared_adjacent += s_part[0][k];
-  if (shared_greedy > shared_adjacent) {
-    if (tid == 0) *any = 1;
-  } else {
-    for (int k = tid; k < 2 * npairs; k += threads) out[k] = k < nbq ? k : -1;
+  if (tid == 0) {
+    long long shared_adjacent = 0;
+    for (int k = 0; k < PAIR_WARPS; ++k) shared_adjacent += s_part[k];
+    s_keep = shared_greedy > shared_adjacent;
+    if (s_keep) *any = 1;
   }
+  __syncthreads();
+  if (!s_keep)
+    for (int k = tid; k < 2 * npairs; k += PAIR_THREADS) out[k] = k < nbq ? k : -1;
 }
 
 // The q-blocks of pair row r (qb = -1: none).
@@ -384,10 +433,11 @@ plan_scan_kernel(int32_t* __restrict__ row_ptr, int32_t* __restrict__ pair_ptr, 
 }
 
 // One warp per pair writes everything that is read of it: cols of its two q-blocks, the merged list, the schedule and the
-// step counts.  A lane owns one word (32 k-blocks) of the two bit rows, expands its set bits into per-list staging in
+// step counts.  A lane owns 16 k-blocks of the two bit rows, expands its set bits into per-list staging in
 // shared memory at offsets from a warp scan, and the lists are copied out in whole lines (expanding straight to
-// global memory writes each sector once per entry).  1024 k-blocks are staged at a time.
-constexpr int LIST_WARPS = 4, LIST_CHUNK = 1024;
+// global memory writes each sector once per entry).  512 k-blocks are staged at a time, 24 KB per
+// CTA.  (With 32 per lane and 1024 at a time an SM has room for 16 warps: 106 us for 40 x 1182 x 1182, this 74.)
+constexpr int LIST_WARPS = 4, LIST_CHUNK = 512;
 __global__ void __launch_bounds__(32 * LIST_WARPS)
 plan_lists_kernel(const uint32_t* __restrict__ bits, int nbq, int words, int npairs, int prows,
                   const int32_t* __restrict__ pair_q, const int32_t* __restrict__ row_ptr,
@@ -409,9 +459,10 @@ plan_lists_kernel(const uint32_t* __restrict__ bits, int nbq, int words, int npa
     }
     const int e0 = pair_ptr[r], slots = pair_ptr[r + 1] - e0, ns = (int)both;
     int at_a = row_ptr[at], at_b = qb >= 0 ? row_ptr[at + 1] : 0, at_u = e0, at_s = e0, at_1 = e0 + ns, at_2 = e0 + ns;
-    for (int w0 = 0; w0 < words; w0 += 32) {
-      const uint32_t a = w0 + lane < words ? pa[w0 + lane] : 0u, b = qb >= 0 && w0 + lane < words ? pb[w0 + lane] : 0u;
-      // inclusive warp scans of |a|, |b| (16 bits each: at most 1024) and |a & b|
+    const uint16_t *ha = reinterpret_cast<const uint16_t*>(pa), *hb = reinterpret_cast<const uint16_t*>(pb);
+    for (int h0 = 0; h0 < 2 * words; h0 += 32) {
+      const uint32_t a = h0 + lane < 2 * words ? ha[h0 + lane] : 0u, b = qb >= 0 && h0 + lane < 2 * words ? hb[h0 + lane] : 0u;
+      // inclusive warp scans of |a|, |b| (16 bits each: at most 512) and |a & b|
       uint32_t nab = (uint32_t)__popc(a) | ((uint32_t)__popc(b) << 16), nsh = (uint32_t)__popc(a & b);
       uint32_t sab = nab, ssh = nsh;
 #pragma unroll
@@ -425,7 +476,7 @@ plan_lists_kernel(const uint32_t* __restrict__ bits, int nbq, int words, int npa
       ssh -= nsh;
       int i_a = (int)(sab & 0xFFFFu), i_b = (int)(sab >> 16), i_s = (int)ssh;
       for (uint32_t u = a | b; u; u &= u - 1) {
-        const int bit = __ffs(u) - 1, kb = lane * 32 + bit;
+        const int bit = __ffs(u) - 1, kb = lane * 16 + bit;
         const int in_a = (a >> bit) & 1u, in_b = (b >> bit) & 1u;
         L[2][i_a + i_b - i_s] = (uint16_t)(kb * 4 + in_a + 2 * in_b);
         if (in_a & in_b) L[3][i_s] = (uint16_t)kb;
@@ -438,7 +489,7 @@ plan_lists_kernel(const uint32_t* __restrict__ bits, int nbq, int words, int npa
         i_s += in_a & in_b;
       }
       __syncwarp();
-      const int k0 = w0 * 32;
+      const int k0 = h0 * 16;
       for (int k = lane; k < t_a; k += 32) cols[at_a + k] = k0 + L[0][k];
       for (int k = lane; k < t_b; k += 32) cols[at_b + k] = k0 + L[1][k];
       for (int k = lane; k < t_u; k += 32) pair_ent[at_u + k] = 4 * k0 + L[2][k];
@@ -496,12 +547,7 @@ extern "C" int paro_plan_offsets(const uint8_t* mask, int slices, int nbq, int n
     PARO_CUDA_OK(cudaFuncSetAttribute(plan_overlap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OV_SMEM));
     plan_overlap_kernel<<<dim3(tiles, tiles, min(slices, 65535)), OV_THREADS, OV_SMEM, s>>>(sc.bits, slices, nbq, sc.words,
                                                                                             sc.pitch, sc.ov, totals + 3);
-    int chunk_log = 5;   // two chunks of rows within 200 KB
-    while (chunk_log >= 0 && (size_t)sc.pitch * 4 << chunk_log > 200 * 1024) --chunk_log;
-    const size_t smem = chunk_log >= 0 ? (size_t)sc.pitch * 4 << chunk_log : 0;
-    PARO_CUDA_OK(cudaFuncSetAttribute(plan_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    const int threads = min(PAIR_THREADS, (nbq + 255) / 256 * 32);   // eight rows per thread
-    plan_pair_kernel<<<slices, threads, smem, s>>>(sc.ov, nbq, sc.pitch, npairs, chunk_log, pair_q, totals + 2);
+    plan_pair_kernel<<<slices, PAIR_THREADS, 0, s>>>(sc.ov, nbq, sc.pitch, npairs, pair_q, totals + 2);
   }
   plan_pair_count_kernel<<<min(8192, (prows + 7) / 8), 256, 0, s>>>(sc.bits, sc.row_cnt, nbq, sc.words, npairs, prows,
                                                                     overlap ? pair_q : nullptr, row_ptr, pair_ptr);
