@@ -38,6 +38,7 @@ struct AttnParams {
   int64_t osb, osh, osn;
   int plan_slices, q_group, n_text;
   int B, H, N, npairs, nb;
+  int text_pairs;       // pairs at the front of every head that are walked before all others
   float scale_log2;     // sm_scale * log2(e)
 };
 
@@ -95,15 +96,15 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-__device__ __forceinline__ void report_timeout(const AttnParams& p, volatile int* abort_flag, int where, int iter) {
+__device__ __forceinline__ void report_timeout(const AttnParams& p, int item, volatile int* abort_flag, int where, int iter) {
   if (atomicCAS(p.status, 0, PARO_ETIMEOUT) == 0) {
     p.status[1] = where;
-    p.status[2] = (int)blockIdx.x;
+    p.status[2] = item;
     p.status[3] = iter;
     if (p.host_status) {
       volatile int32_t* h = p.host_status;
       h[1] = where;
-      h[2] = (int)blockIdx.x;
+      h[2] = item;
       h[3] = iter;
       __threadfence_system();
       h[0] = PARO_ETIMEOUT;
