@@ -9,7 +9,7 @@
 //   lists     the CSR lists, the merged lists and the walk schedule of a pair, written by one warp
 //
 // The host reads three totals back between count and lists (the lists' lengths), once per call.
-// Measured on a 40 x 1182 x 1182 mask at density 0.2: 0.39 ms on the device (pack 25 us, overlap 96, pair 184, count and
+// Measured on a 40 x 1182 x 1182 mask at density 0.2: 0.35 ms on the device (pack 25 us, overlap 90, pair 153, count and
 // scans 12, lists 74); a fp32 bmm with 591 rounds of small torch kernels took 67 ms.
 #include "common.cuh"
 #include "umma.cuh"
@@ -146,9 +146,13 @@ plan_overlap_kernel(const uint32_t* __restrict__ bits, int slices, int nbq, int 
   bool ok = true;
   for (int slice = blockIdx.z; slice < slices && ok; slice += gridDim.z) {
     const uint32_t* src = bits + ((size_t)slice * nbq + (row < nbq ? row : 0)) * words;
+    auto fetch = [&](int c) { return row < nbq && c < chunks ? *reinterpret_cast<const uint4*>(src + 4 * c) : make_uint4(0, 0, 0, 0); };
+    uint4 ahead[2] = {fetch(0), fetch(1)};   // (fetched when they are expanded, the bits hold every stage up for their latency)
     for (int c = 0; c < chunks; ++c, ++done) {
       const int st = done & 1;
-      uint4 v = row < nbq ? *reinterpret_cast<const uint4*>(src + 4 * c) : make_uint4(0, 0, 0, 0);
+      const uint4 v = ahead[0];
+      ahead[0] = ahead[1];
+      ahead[1] = fetch(c + 2);
       if (done >= 2 && !mbar_wait_plain_bounded(&s_bar[st], ((done >> 1) - 1) & 1, OV_WAIT_LIMIT)) s_failed = 1;
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -216,16 +220,17 @@ plan_overlap_kernel(const uint32_t* __restrict__ bits, int slices, int nbq, int 
 // wants, and the results are accepted in order up to the first that wanted a q-block already taken (a q-block that was
 // itself taken as a partner is passed over).  What the others found is kept: it is still the best as long as the
 // partner is free.  (1182 rows at density 0.2: 86 turns of seven pairs.  591 rounds of one pair, all warps on one row, 290 us;
-// this 184, the rows read from L2 where they lie.  Staged through shared memory 16 rows at a time they arrive too
-// late, 228 us.)  A candidate's key is its overlap + 1 (0: not free); a lane looks at eight per load.
+// this 153, the rows asked for a turn ahead and read where they lie (184 without that and with a warp-wide match in
+// place of the comparisons; staged through shared memory 16 rows at a time they arrive too late, 228).)  A candidate's key is its overlap + 1 (0: not free); a lane looks at eight per load.
 // A pairing that does not need fewer tiles than adjacency is replaced by adjacency; any[0] = 1 if one was kept.
 constexpr int PAIR_WARPS = 8, PAIR_THREADS = 32 * PAIR_WARPS, PAIR_MAX_ROWS = 65536, PAIR_LOADS = 5;
 __global__ void __launch_bounds__(PAIR_THREADS)
 plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs, int32_t* __restrict__ pair_q,
                  int32_t* __restrict__ any) {
-  __shared__ uint32_t s_free[PAIR_MAX_ROWS / 32 + 1];   // bit per q-block, as words and as bytes (byte t: rows 8t..8t+7)
+  __shared__ uint32_t s_free[PAIR_MAX_ROWS / 32 + 2];   // bit per q-block, as words and as bytes (byte t: rows 8t..8t+7)
   __shared__ int2 s_found[32];             // [row mod 32] (row, its best partner so far or -1); the window spans 32 rows
   __shared__ uint32_t s_overlap[32];       // their overlap + 1
+  __shared__ __align__(16) int2 s_win[PAIR_WARPS];      // the turn's rows and what they found
   __shared__ uint32_t s_part[PAIR_WARPS];
   __shared__ int s_keep;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -233,7 +238,7 @@ plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs
   const uint16_t* o = ov + (size_t)blockIdx.x * nbq * pitch;
   int32_t* out = pair_q + (size_t)blockIdx.x * npairs * 2;
   const int words = (nbq + 31) / 32, groups = (nbq + 7) / 8;
-  for (int w = tid; w <= words; w += PAIR_THREADS)
+  for (int w = tid; w <= words + 1; w += PAIR_THREADS)
     s_free[w] = nbq - 32 * w >= 32 ? 0xffffffffu : nbq > 32 * w ? (1u << (nbq - 32 * w)) - 1u : 0u;
   if (tid < 32) s_found[tid] = make_int2(-1, -1);
   __syncthreads();
@@ -247,13 +252,29 @@ plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs
     while (!fm && ++fw < words) fm = s_free[fw];
     if (!fm) break;
     const int i0 = fw * 32 + __ffs(fm) - 1;
-    const uint32_t win = __funnelshift_r(s_free[fw], s_free[fw + 1], i0 & 31);
+    const uint32_t f0 = s_free[fw], f1 = s_free[fw + 1], f2 = s_free[fw + 2];
+    const uint32_t win = __funnelshift_r(f0, f1, i0 & 31);
     const int n = min(__popc(win), PAIR_WARPS);
+    {   // a row that the next turns will look at: its sectors into L1, 32 bytes per lane and load
+      uint64_t ahead = win | (uint64_t)__funnelshift_r(f1, f2, i0 & 31) << 32;
+      for (int k = 0; k < PAIR_WARPS + warp; ++k) ahead &= ahead - 1;
+      if (ahead) {
+        const int r = i0 + __ffsll((long long)ahead) - 1;
+        const char* at = reinterpret_cast<const char*>(o + (size_t)r * pitch + (r & ~15)) + 32 * lane;
+        const char* const end = reinterpret_cast<const char*>(o + (size_t)r * pitch + 8 * groups);
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          [[maybe_unused]] uint32_t sink;
+          if (at + 1024 * u < end) asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(sink) : "l"(at + 1024 * u));
+        }
+      }
+    }
     if (warp < n) {
       uint32_t b = win;
       for (int k = 0; k < warp; ++k) b &= b - 1;
       const int i = i0 + __ffs(b) - 1;
       const int2 kept = s_found[i & 31];
+      int partner = kept.y;
       if (kept.x != i || kept.y < 0 || !(s_free[kept.y >> 5] >> (kept.y & 31) & 1u)) {
         const uint16_t* row = o + (size_t)i * pitch;
         // clears the keys of the candidates v of group g that are not free; the largest that is left
@@ -269,6 +290,7 @@ plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs
           return max(m2 & 0xFFFFu, m2 >> 16);
         };
         uint32_t best = 0;   // key << 16 | complement of the group that has it
+        uint4 bv = make_uint4(0, 0, 0, 0);   // that group
         for (int g0 = (i >> 3) + lane; g0 < groups; g0 += 32 * PAIR_LOADS) {
           uint4 v[PAIR_LOADS];
 #pragma unroll
@@ -276,54 +298,68 @@ plan_pair_kernel(const uint16_t* __restrict__ ov, int nbq, int pitch, int npairs
             if (g0 + 32 * u < groups) v[u] = *reinterpret_cast<const uint4*>(row + 8 * (g0 + 32 * u));
 #pragma unroll
           for (int u = 0; u < PAIR_LOADS; ++u)
-            if (g0 + 32 * u < groups) best = max(best, masked(v[u], g0 + 32 * u) << 16 | (uint32_t)(0xFFFF - g0 - 32 * u));
+            if (g0 + 32 * u < groups) {
+              const uint32_t key = masked(v[u], g0 + 32 * u) << 16 | (uint32_t)(0xFFFF - g0 - 32 * u);
+              if (key > best) {
+                best = key;
+                bv = v[u];
+              }
+            }
         }
-        best = __reduce_max_sync(0xffffffffu, best);
-        int partner = -1;
-        if (best >> 16) {
-          const int g = 0xFFFF - (int)(best & 0xFFFFu);
-          uint4 v = *reinterpret_cast<const uint4*>(row + 8 * g);
-          masked(v, g);
-          const uint32_t w = lane & 4 ? (lane & 2 ? v.w : v.z) : (lane & 2 ? v.y : v.x);
-          partner = 8 * g + __ffs(__ballot_sync(0xffffffffu, lane < 8 && (lane & 1 ? w >> 16 : w & 0xFFFFu) == best >> 16)) - 1;
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        partner = -1;
+        if (top >> 16) {
+          // the lane that holds it: its first candidate with that key
+          const uint32_t w[4] = {bv.x, bv.y, bv.z, bv.w};
+          int at = 0;
+#pragma unroll
+          for (int k = 7; k >= 0; --k)
+            if ((k & 1 ? w[k >> 1] >> 16 : w[k >> 1] & 0xFFFFu) == top >> 16) at = k;
+          const int who = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
+          partner = 8 * (0xFFFF - (int)(top & 0xFFFFu)) + __shfl_sync(0xffffffffu, at, who);
         }
         if (lane == 0) {
           s_found[i & 31] = make_int2(i, partner);
-          s_overlap[i & 31] = best >> 16;
+          s_overlap[i & 31] = top >> 16;
         }
       }
+      if (lane == 0) s_win[warp] = make_int2(i, partner);
     }
     __syncthreads();
-    // lane k < n: the window's row k and what it found
+    // lane k: which rows before the window's row k want its partner, and which row behind k the partner is
+    static_assert(PAIR_WARPS == 8, "eight rows in four loads");
+    int row[PAIR_WARPS], par[PAIR_WARPS];
+#pragma unroll
+    for (int k = 0; k < PAIR_WARPS; k += 2) {
+      const int4 t = *reinterpret_cast<const int4*>(s_win + k);
+      row[k] = t.x; par[k] = t.y; row[k + 1] = t.z; par[k + 1] = t.w;
+    }
     int i = -1, g = -1;
-    uint32_t b = win;
-    for (int k = 0; k < (lane & 7); ++k) b &= b - 1;
-    if ((lane & 7) < n) {
-      i = i0 + __ffs(b) - 1;
-      g = s_found[i & 31].y;
-    }
-    // lanes 0-7 hold the partners, 8-15 the rows: who else wants my partner (bits 0-7), which row it is (8-15)
-    static_assert(PAIR_WARPS == 8, "lanes of the match");
-    const int value = lane < 8 ? (g >= 0 ? g : -1 - lane) : lane < 16 ? (i >= 0 ? i : -1 - lane) : -1 - lane;
-    const uint32_t same = __match_any_sync(0xffffffffu, value);
-    const uint32_t others = lane < n ? same & 0xFFFFu & ~(1u << lane) : 0u;
-    // only the rows that meet another one are gone through
-    uint32_t meet = __ballot_sync(0xffffffffu, others != 0) | __reduce_or_sync(0xffffffffu, others >> 8);
-    uint32_t passed = 0;                        // rows taken as a partner
-    uint32_t takers = ((1u << n) - 1u) & ~meet;   // rows that take their partner
-    int stop = n;                               // the first row to be looked at again
-    for (; meet; meet &= meet - 1) {
-      const int k = __ffs(meet) - 1;
-      const uint32_t s = __shfl_sync(0xffffffffu, others, k);
-      if (passed >> k & 1u) continue;
-      if (s & takers & ((1u << k) - 1u)) {
-        stop = k;
-        break;
+#pragma unroll
+    for (int k = 0; k < PAIR_WARPS; ++k)
+      if (lane == k && k < n) { i = row[k]; g = par[k]; }
+    uint32_t others = 0;
+#pragma unroll
+    for (int k = 0; k < PAIR_WARPS; ++k)
+      if (k < n && g >= 0) others |= (par[k] == g && k < lane ? 1u : 0u) << k | (row[k] == g ? 0x100u : 0u) << k;
+    uint32_t passed = 0, accepted = 0;   // rows taken as a partner; rows that take their partner
+    int stop = n;                        // the first row to be looked at again
+    if (__any_sync(0xffffffffu, others != 0)) {
+      uint32_t o_k[PAIR_WARPS];
+#pragma unroll
+      for (int k = 0; k < PAIR_WARPS; ++k) o_k[k] = __shfl_sync(0xffffffffu, others, k);
+#pragma unroll
+      for (int k = 0; k < PAIR_WARPS; ++k) {
+        const bool live = k < stop && !(passed >> k & 1u);
+        if (live && (o_k[k] & accepted)) stop = k;
+        else if (live) {
+          accepted |= 1u << k;
+          passed |= o_k[k] >> 8;
+        }
       }
-      takers |= 1u << k;
-      passed |= s >> 8;
+    } else {
+      accepted = (1u << n) - 1u;
     }
-    const uint32_t accepted = takers & ((1u << stop) - 1u);
     const int last = __shfl_sync(0xffffffffu, i, min(stop, n - 1));
     cursor = stop < n ? last : last + 1;
     if (warp == 0 && lane < 8 && (accepted >> lane & 1u)) {
