@@ -55,6 +55,41 @@ template <> struct F16Traits<__nv_bfloat16> {
   static __device__ __forceinline__ __nv_bfloat16 from_float(float v) { return __float2bfloat16_rn(v); }
 };
 
+// Packed pairs of fp32: sm_100a has 2-wide fp32 arithmetic, one issue slot for two operations.  A packed sum of packed
+// products may come out contracted (rounded once): where the product has to be rounded by itself, the sum is taken with
+// the scalar intrinsics.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t r, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+template <typename T> struct Inf16;   // bits of the 16-bit type's Inf: larger magnitudes are NaN
+template <> struct Inf16<__half> { static constexpr uint32_t BITS = 0x7C00u; };
+template <> struct Inf16<__nv_bfloat16> { static constexpr uint32_t BITS = 0x7F80u; };
+
 // Passes of a layer over V and over K's rotated copy (quant.cu), issued by paro_layer.
 size_t layer_kv_scratch_bytes(int B, int H, int N, int D);
 int layer_kv_passes(const paro_layer_args& a, const void* kp, void* km, int8_t* k8, float* ks, uint16_t* v16, float* vs,

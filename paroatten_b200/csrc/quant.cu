@@ -3,6 +3,7 @@
 // pass, results compared bit-for-bit with the CPU oracle (IEEE divide/multiply, no fast-math).
 #include <cuda_fp8.h>
 
+#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -218,29 +219,34 @@ channel_finalize_kernel(const FinalizeDst<T> dst0, const FinalizeDst<T> dst1, in
 // ---------------------------------------------------------------------------------------------
 // INT8: one CTA = `blocks` consecutive 64-token blocks of one (b,h); warp w owns 64/WARPS tokens of each.
 // 2 bytes in, 1 byte out per element.
-// Passes that rotate (TABLE): 256 threads; source tokens and table rows of all the CTA's blocks are worked out once
-// into shared memory.  Four blocks per CTA against one: 109 -> 73 us for 48 x 17776 x 64 with the fp32 rotation,
-// 113 -> 100 us for 12 x 32760 x 128 with RMS norm and the fp64 rotation.  (Loading the next block's rows ahead
-// costs the registers of a third CTA per SM, 6 and 17 % more.  Four CTAs per SM at D = 64, where a thread holds two rows and
-// not four: Q of 2 x 48 x 17776 x 64 184 -> 168 us with the fp64 rotation, 244 -> 221 with LayerNorm and the fp32 one; at
-// D = 128 with a norm the fourth costs spills, RMS 197 -> 205 us.)
-// Passes that do not: 128 threads with twice the rows in flight each, one block per CTA, source tokens by shuffle (the
-// form above takes 90 us instead of 72 for 2 x 48 x 17776 x 64 in plain order, 29 instead of 22 for 40 x 4680 x 128
-// reordered).
+// Bound by instructions (ncu: 75-81 % of the issue slots): a pass that rotates has 16 of them per element at HBM's rate.  Hence
+// packed fp32 arithmetic, the maximum taken over the 16-bit patterns where nothing is subtracted first (SH_NONE), and
+// rounding to an integer by adding 1.5 * 2^23 instead of a conversion.  An Inf or NaN takes its thread through the general
+// form of both.  Scalar arithmetic with conversions before, us: Q of 5 x 75600 x 128 with the fp64 rotation 77 -> 67,
+// of 2 x 48 x 17776 x 64 with the fp32 one 140 -> 105, with LayerNorm 232 -> 205, of 2 x 12 x 32760 x 128 with RMS norm 189 -> 168;
+// K of the first two without a rotation 35 -> 31 and 74 -> 65.
+// Passes that rotate (TABLE): source tokens and table rows of all the CTA's blocks are worked out once into shared memory.
+// The others: one block per CTA, source tokens by shuffle.
 constexpr int INT8_BLOCKS = 4;               // most blocks per CTA
-template <int GM> struct Int8Cfg {
+template <int GM, int D> struct Int8Cfg {
   static constexpr bool TABLE = GM == GM_ROPE_F32 || GM == GM_ROPE_F64;
-  static constexpr int WARPS = TABLE ? 8 : 4;
+  static constexpr int WARPS = TABLE && D == 128 ? 8 : 4;   // (four rows per thread; eight without a rotation at D = 128)
 };
-template <typename T, int D, int GROUP, int GM, int NM>
-__global__ void __launch_bounds__(32 * Int8Cfg<GM>::WARPS,
-                                  !Int8Cfg<GM>::TABLE ? (NM != PARO_NORM_NONE ? 5 : 6)
-                                  : D == 64 || (GM == GM_ROPE_F32 && NM == PARO_NORM_NONE) ? 4 : 3)
+enum { SH_NONE = 0, SH_MEAN = 1, SH_ANY = 2 };   // rows as they are; minus the channel means; minus means and times `fold`, where given
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {   // (NaN if one of them is)
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+template <typename T, int D, int GROUP, int GM, int NM, int SH>
+__global__ void __launch_bounds__(32 * Int8Cfg<GM, D>::WARPS,
+                                  Int8Cfg<GM, D>::WARPS == 8 ? (NM != PARO_NORM_NONE ? 3 : 4)
+                                  : D == 64 && NM == PARO_NORM_NONE ? 8 : NM != PARO_NORM_NONE ? 5 : 6)
 quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __restrict__ out,
                   float* __restrict__ scale, int H, int N, int64_t sb, int64_t sh, int64_t sn,
                   float fold, int n_scale_per_bh, int blocks, const Gather gather, const NormArgs norm) {
-  constexpr bool TABLE = Int8Cfg<GM>::TABLE;
-  constexpr int WARPS = Int8Cfg<GM>::WARPS, ROWS = 64 / WARPS;   // ROWS: tokens per warp and block
+  constexpr bool TABLE = Int8Cfg<GM, D>::TABLE;
+  constexpr int WARPS = Int8Cfg<GM, D>::WARPS, ROWS = 64 / WARPS;   // ROWS: tokens per warp and block
   constexpr int TPR = D / 8;          // threads per token row
   constexpr int RPL = 32 / TPR;       // rows covered by one warp-wide load
   constexpr int LOADS = ROWS / RPL;   // loads per thread and block
@@ -267,21 +273,19 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
     else return first + blk * 64 + r0 + i * RPL;
   };
 
-  float mean[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) mean[j] = 0.f;
-  if (km) {
+  [[maybe_unused]] uint64_t mean2[4] = {0ull, 0ull, 0ull, 0ull};
+  if (SH != SH_NONE && km) {
     Pack8<T> m;
     m.v = *reinterpret_cast<const uint4*>(km + (size_t)bh * D + c8);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) mean[j] = F16Traits<T>::to_float(m.e[j]);
+    for (int j = 0; j < 4; ++j) mean2[j] = pack2(F16Traits<T>::to_float(m.e[2 * j]), F16Traits<T>::to_float(m.e[2 * j + 1]));
   }
-  // the (rotated) rows stay packed in registers; they are widened once for the maximum and once more
-  // for the rounding, which costs a shift per element and halves the registers held across the barrier
+  // Elements 2j and 2j+1 of a row as they are quantised.  The (rotated) rows stay packed in registers; they are widened once
+  // for the maximum and once more for the rounding, which halves the registers held across the barrier.
   auto widen = [&](const Pack8<T>& p, int j) {
-    float f = F16Traits<T>::to_float(p.e[j]);
-    if (km) f = __fsub_rn(f, mean[j]);
-    if (fold != 0.f) f = __fmul_rn(f, fold);
+    uint64_t f = pack2(F16Traits<T>::to_float(p.e[2 * j]), F16Traits<T>::to_float(p.e[2 * j + 1]));
+    if (SH == SH_MEAN || (SH == SH_ANY && km)) f = sub2(f, mean2[j]);
+    if (SH == SH_ANY && fold != 0.f) f = mul2(f, pack2(fold, fold));
     return f;
   };
 #pragma unroll 1
@@ -297,7 +301,6 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
       row[i].v = make_uint4(0, 0, 0, 0);
       if (first + blk * 64 + r0 + i * RPL < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn);
     }
-    float amax = 0.f;
     if constexpr (NM != PARO_NORM_NONE) {
 #pragma unroll
       for (int i = 0; i < LOADS; ++i) {   // all lanes: the row statistics are reduced with full-warp shuffles
@@ -310,15 +313,50 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
 #pragma unroll
       for (int i = 0; i < LOADS; i += NR) gc.template rotate<NR>(row + i, pa, rows, blk * 64 + r0 + i * RPL, RPL);
     }
+    // the thread's maximum; rows past the end count as zeros
+    float amax = 0.f;
+    bool special;   // an Inf or NaN among the thread's elements
+    if constexpr (SH == SH_NONE) {
+      uint32_t m2 = 0;
 #pragma unroll
-    for (int i = 0; i < LOADS; ++i) {
-      if (first + blk * 64 + r0 + i * RPL < N) {
+      for (int i = 0; i < LOADS; ++i) {
+        if (NM != PARO_NORM_NONE && first + blk * 64 + r0 + i * RPL >= N) continue;   // (a norm may have made them other than 0)
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(&row[i].v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(widen(row[i], j)));
+        for (int j = 0; j < 4; ++j) m2 = __vmaxu2(m2, w[j] & 0x7fff7fffu);
+      }
+      const uint16_t m = (uint16_t)max(m2 & 0xFFFFu, m2 >> 16);
+      special = m >= Inf16<T>::BITS;
+      T as_t;
+      memcpy(&as_t, &m, 2);
+      amax = F16Traits<T>::to_float(as_t);
+    } else {
+#pragma unroll
+      for (int i = 0; i < LOADS; ++i) {
+        if (first + blk * 64 + r0 + i * RPL >= N) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float f0, f1;
+          unpack2(widen(row[i], j), f0, f1);
+          amax = max3_nan(amax, fabsf(f0), fabsf(f1));
+        }
+      }
+      special = !(amax < INFINITY);
+    }
+    if (special) {   // the maximum ignores NaN
+      amax = 0.f;
+#pragma unroll
+      for (int i = 0; i < LOADS; ++i) {
+        if (first + blk * 64 + r0 + i * RPL >= N) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float f0, f1;
+          unpack2(widen(row[i], j), f0, f1);
+          amax = fmaxf(amax, fmaxf(fabsf(f0), fabsf(f1)));
+        }
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));   // (not negative: ordered as integers)
     if (lane == 0) s_amax[blk & 1][warp] = amax;   // (two buffers: one barrier per block)
     __syncthreads();
     constexpr int GW = WARPS * GROUP / 64;   // warps per scale group
@@ -329,24 +367,38 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
     if (lane == 0 && warp == g0)
       scale[(size_t)bh * n_scale_per_bh + (first / 64 + blk) * (64 / GROUP) + warp / GW] = __fdiv_rn(amax, 127.0f);
     const float inv = __fdiv_rn(127.0f, amax);
+    const uint64_t inv2 = pack2(inv, inv);
+    constexpr float ROUND = 12582912.0f;   // 1.5 * 2^23: the sum's low bits are the integer, rounded to nearest even
 #pragma unroll
     for (int i = 0; i < LOADS; ++i) {
       const int tok = first + blk * 64 + r0 + i * RPL;
-      if (tok < N) {
-        // round to nearest even (NaN -> 0), then saturate and pack two values per instruction
-        int qi[8];
+      if (tok >= N) continue;
+      uint32_t w[2];
+      if (!special) {   // |element * inv| is at most 127 and rounding errors of it
+        float y[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) qi[j] = __float2int_rn(__fmul_rn(widen(row[i], j), inv));
-        uint32_t w[2];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t hi16, word;
-          asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(hi16) : "r"(qi[half * 4 + 3]), "r"(qi[half * 4 + 2]), "r"(0));
-          asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(word) : "r"(qi[half * 4 + 1]), "r"(qi[half * 4 + 0]), "r"(hi16));
-          w[half] = word;
+        for (int j = 0; j < 4; ++j) {
+          unpack2(mul2(widen(row[i], j), inv2), y[2 * j], y[2 * j + 1]);
+          y[2 * j] = __fadd_rn(y[2 * j], ROUND);
+          y[2 * j + 1] = __fadd_rn(y[2 * j + 1], ROUND);
         }
-        *reinterpret_cast<uint2*>(out + ((size_t)bh * N + tok) * D + c8) = make_uint2(w[0], w[1]);
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+          w[half] = __byte_perm(__byte_perm(__float_as_uint(y[4 * half]), __float_as_uint(y[4 * half + 1]), 0x0040),
+                                __byte_perm(__float_as_uint(y[4 * half + 2]), __float_as_uint(y[4 * half + 3]), 0x0040), 0x5410);
+      } else {
+        // round to nearest even (NaN -> 0), then saturate
+        w[0] = w[1] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float f0, f1;
+          unpack2(widen(row[i], j), f0, f1);
+          const int q0 = min(127, max(-128, __float2int_rn(__fmul_rn(f0, inv))));
+          const int q1 = min(127, max(-128, __float2int_rn(__fmul_rn(f1, inv))));
+          w[j >> 1] |= ((uint32_t)(q0 & 0xFF) | (uint32_t)(q1 & 0xFF) << 8) << (16 * (j & 1));
+        }
       }
+      *reinterpret_cast<uint2*>(out + ((size_t)bh * N + tok) * D + c8) = make_uint2(w[0], w[1]);
     }
   }
 }
@@ -514,14 +566,25 @@ void launch_int8_norm(const void* x, const void* km, int8_t* out, float* scale, 
     // with the fp64 rotation: 12 x 32760 x 128 92, 82, 78; 20 x 7800 x 128 39, 35, 39; 24 x 2926 x 64 14.5, 12.5, 12.5;
     // 2 x 12 x 1560 x 128 14.5, 14.5, 18.6, with LayerNorm 19, 21, 29).
     const int64_t total = (int64_t)nb * B * H;
-    const int blocks = !Int8Cfg<GM>::TABLE ? 1 : total >= 148 * 21 ? INT8_BLOCKS : total >= 148 * 5 ? 2 : 1;
+    const int blocks = !Int8Cfg<GM, D>::TABLE ? 1 : total >= 148 * 21 ? INT8_BLOCKS : total >= 148 * 5 ? 2 : 1;
     const dim3 grid((nb + blocks - 1) / blocks, B * H);
-    if (group == 64)
-      quant_int8_kernel<T, D, 64, GM, NM><<<grid, 32 * Int8Cfg<GM>::WARPS, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N,
-                                                                                   sb, sh, sn, fold, nb, blocks, g, nm);
-    else
-      quant_int8_kernel<T, D, 32, GM, NM><<<grid, 32 * Int8Cfg<GM>::WARPS, 0, s>>>((const T*)x, (const T*)km, out, scale, H, N,
-                                                                                   sb, sh, sn, fold, nb * 2, blocks, g, nm);
+    auto launch = [&](auto grp, auto shift) {
+      constexpr int GROUP = decltype(grp)::value, SH = decltype(shift)::value;
+      quant_int8_kernel<T, D, GROUP, GM, NM, SH><<<grid, 32 * Int8Cfg<GM, D>::WARPS, 0, s>>>(
+          (const T*)x, (const T*)km, out, scale, H, N, sb, sh, sn, fold, nb * (64 / GROUP), blocks, g, nm);
+    };
+    auto with_group = [&](auto shift) {
+      if (group == 64) launch(std::integral_constant<int, 64>{}, shift);
+      else launch(std::integral_constant<int, 32>{}, shift);
+    };
+    // (only plain input is ever folded; a norm and a mean are never combined)
+    if constexpr (NM == PARO_NORM_NONE) {
+      if (GM == GM_PLAIN && fold != 0.f) { if constexpr (GM == GM_PLAIN) with_group(std::integral_constant<int, SH_ANY>{}); }
+      else if (km) with_group(std::integral_constant<int, SH_MEAN>{});
+      else with_group(std::integral_constant<int, SH_NONE>{});
+    } else {
+      with_group(std::integral_constant<int, SH_NONE>{});
+    }
   });
 }
 

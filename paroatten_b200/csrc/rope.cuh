@@ -110,15 +110,48 @@ __device__ __forceinline__ uint32_t rotate_pair_f32(float x0, float x1, float c,
 // e so far or NaN.  Of 2 x 12 x 32760 x 128, bf16 and fp16: INT8 Q 142 and 148 us, rotation + reorder 107 and 113; with one
 // e from (|x0|+|x1|) * (|c|+|s|), four times as many unsettled pairs and all four of a thread settled together 149 and
 // 172, 115 and 133; with fp64 alone 167 and 164, 138 and 144.
+//
+// Two pairs at a time (x0, x1: their even and odd channels; c, s: their angles), in packed fp32 arithmetic.  (A contracted
+// sum is closer to the exact one than the bound allows for.)
 template <typename T>
-__device__ __forceinline__ uint32_t rotate_pair_checked(float x0, float x1, float c, float s, uint32_t& out, float& worst) {
-  const float tiny = std::is_same<T, __half>::value ? 0x1p-130f : fmaf(fabsf(x0) + fabsf(x1), 0x1p-146f, 0x1p-140f);
-  const float p = __fmul_rn(x0, c), q = __fmul_rn(x1, s), re = __fsub_rn(p, q);
-  const float v = __fmul_rn(x0, s), w = __fmul_rn(x1, c), im = __fadd_rn(v, w);
-  const float er = fmaf(fabsf(p) + fabsf(q), 0x1.01p-22f, tiny), ei = fmaf(fabsf(v) + fabsf(w), 0x1.01p-22f, tiny);
-  out = pack_pair<T>(re - er, im - ei);
-  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(worst) : "f"(worst), "f"(er), "f"(ei));
-  return out ^ pack_pair<T>(re + er, im + ei);
+__device__ __forceinline__ void rotate_pairs_checked(uint64_t x0, uint64_t x1, uint64_t c, uint64_t s, uint32_t* out,
+                                                     uint32_t* unsettled, float& worst) {
+  const uint64_t p = mul2(x0, c), q = mul2(x1, s), v = mul2(x0, s), w = mul2(x1, c);
+  const uint64_t re = sub2(p, q), im = add2(v, w);
+  auto abs_sum = [](uint64_t a, uint64_t b) {
+    float a0, a1, b0, b1;
+    unpack2(a, a0, a1);
+    unpack2(b, b0, b1);
+    return pack2(fabsf(a0) + fabsf(b0), fabsf(a1) + fabsf(b1));
+  };
+  uint64_t tiny = pack2(0x1p-130f, 0x1p-130f);
+  if constexpr (!std::is_same<T, __half>::value) tiny = fma2(abs_sum(x0, x1), pack2(0x1p-146f, 0x1p-146f), pack2(0x1p-140f, 0x1p-140f));
+  const uint64_t rel = pack2(0x1.01p-22f, 0x1.01p-22f);
+  const uint64_t er = fma2(abs_sum(p, q), rel, tiny), ei = fma2(abs_sum(v, w), rel, tiny);
+  float r0, r1, i0, i1;
+  unpack2(sub2(re, er), r0, r1);
+  unpack2(sub2(im, ei), i0, i1);
+  out[0] = pack_pair<T>(r0, i0);
+  out[1] = pack_pair<T>(r1, i1);
+  unpack2(add2(re, er), r0, r1);
+  unpack2(add2(im, ei), i0, i1);
+  unsettled[0] = out[0] ^ pack_pair<T>(r0, i0);
+  unsettled[1] = out[1] ^ pack_pair<T>(r1, i1);
+  unpack2(er, r0, r1);
+  unpack2(ei, i0, i1);
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(worst) : "f"(worst), "f"(r0), "f"(i0));
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(worst) : "f"(worst), "f"(r1), "f"(i1));
+}
+// The fp32 rotation of two pairs, products packed; every product and sum is rounded by itself.
+template <typename T>
+__device__ __forceinline__ void rotate_pairs_f32(uint64_t x0, uint64_t x1, uint64_t c, uint64_t s, uint32_t* out) {
+  float p0, p1, q0, q1, v0, v1, w0, w1;
+  unpack2(mul2(x0, c), p0, p1);
+  unpack2(mul2(x1, s), q0, q1);
+  unpack2(mul2(x0, s), v0, v1);
+  unpack2(mul2(x1, c), w0, w1);
+  out[0] = pack_pair<T>(__fsub_rn(p0, q0), __fadd_rn(w0, v0));
+  out[1] = pack_pair<T>(__fsub_rn(p1, q1), __fadd_rn(w1, v1));
 }
 
 template <int MODE>
@@ -172,14 +205,17 @@ __device__ __forceinline__ void rotate8(Pack8<T>* x, const PairAxes& pa, const R
       }
 #pragma unroll
     for (int u = 0; u < NR; ++u) {
-      uint32_t out[4], unsettled[4];
-      float worst = 0.f;
+      uint32_t out[4];
+      [[maybe_unused]] uint32_t unsettled[4];
+      [[maybe_unused]] float worst = 0.f;
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const float c = p & 1 ? cs[u][p >> 1].z : cs[u][p >> 1].x, s = p & 1 ? cs[u][p >> 1].w : cs[u][p >> 1].y;
-        const float x0 = F16Traits<T>::to_float(x[u].e[2 * p]), x1 = F16Traits<T>::to_float(x[u].e[2 * p + 1]);
-        if constexpr (MODE == PARO_ROPE_REAL_F32) out[p] = rotate_pair_f32<T>(x0, x1, c, s);
-        else unsettled[p] = rotate_pair_checked<T>(x0, x1, c, s, out[p], worst);
+      for (int h = 0; h < 2; ++h) {
+        const T* e = x[u].e + 4 * h;
+        const uint64_t x0 = pack2(F16Traits<T>::to_float(e[0]), F16Traits<T>::to_float(e[2]));
+        const uint64_t x1 = pack2(F16Traits<T>::to_float(e[1]), F16Traits<T>::to_float(e[3]));
+        const uint64_t c = pack2(cs[u][h].x, cs[u][h].z), s = pack2(cs[u][h].y, cs[u][h].w);
+        if constexpr (MODE == PARO_ROPE_REAL_F32) rotate_pairs_f32<T>(x0, x1, c, s, out + 2 * h);
+        else rotate_pairs_checked<T>(x0, x1, c, s, out + 2 * h, unsettled + 2 * h, worst);
       }
       if (o0[u] < 0) continue;
       if constexpr (MODE == PARO_ROPE_COMPLEX_F64) {

@@ -11,7 +11,7 @@ namespace paro {
 // Block = 256 threads = 64 (D = 128) or 128 rows; a thread owns one 16-byte slice of PASSES consecutive rows.
 // blockIdx.x: group of rows, blockIdx.y: b*H + h.
 template <typename T, int D, int MODE, int NM>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 rope_permute_kernel(const T* __restrict__ in, T* __restrict__ out, int H, int N,
                     int64_t sb, int64_t sh, int64_t sn, int n_text, int F, int Hh, int W,
                     const int32_t* __restrict__ order_ids, int inverse, RopeArgs rope, NormArgs norm) {
