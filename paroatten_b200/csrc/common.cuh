@@ -90,6 +90,30 @@ template <typename T> struct Inf16;   // bits of the 16-bit type's Inf: larger m
 template <> struct Inf16<__half> { static constexpr uint32_t BITS = 0x7C00u; };
 template <> struct Inf16<__nv_bfloat16> { static constexpr uint32_t BITS = 0x7F80u; };
 
+// The two values of a word of 16-bit floats as doubles that are the values times 2^-896: sign, exponent field and fraction moved
+// to their places (denormals included; an Inf or NaN becomes a number and has to be looked for).  A few integer operations
+// where a conversion occupies a pipe of 16 per clock and SM.
+constexpr double WIDE_SCALE = 0x1p896;
+template <typename T> __device__ __forceinline__ void widen_word(uint32_t w, double& lo, double& hi);
+template <> __device__ __forceinline__ void widen_word<__nv_bfloat16>(uint32_t w, double& lo, double& hi) {
+  lo = __hiloint2double((int)((uint32_t)((int)(w << 16) >> 3) & 0x8FFFE000u), 0);
+  hi = __hiloint2double((int)((uint32_t)((int)w >> 3) & 0x8FFFE000u), 0);
+}
+template <> __device__ __forceinline__ void widen_word<__half>(uint32_t w, double& lo, double& hi) {
+  const __half2 h = *reinterpret_cast<const __half2*>(&w);
+  lo = __hiloint2double((int)((uint32_t)((int)__float_as_uint(__low2float(h)) >> 3) & 0x8FFFFFFFu), 0);
+  hi = __hiloint2double((int)((uint32_t)((int)__float_as_uint(__high2float(h)) >> 3) & 0x8FFFFFFFu), 0);
+}
+template <typename T> struct Two16;
+template <> struct Two16<__half> { using type = __half2; };
+template <> struct Two16<__nv_bfloat16> { using type = __nv_bfloat162; };
+// Read-only load that stays where it is written (a loop does not keep what it is widened to in registers).
+__device__ __forceinline__ uint4 ld_pinned16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // Passes of a layer over V and over K's rotated copy (quant.cu), issued by paro_layer.
 size_t layer_kv_scratch_bytes(int B, int H, int N, int D);
 int layer_kv_passes(const paro_layer_args& a, const void* kp, void* km, int8_t* k8, float* ks, uint16_t* v16, float* vs,

@@ -19,50 +19,105 @@ struct NormArgs {
   float eps;
 };
 
-// Normalises the 8 channels c8..c8+7 of one token row held by this thread.  The row is spread over
-// TPR consecutive lanes (TPR = D/8); every lane of the warp must call this (full-mask shuffles).
-template <typename T, int NM, int TPR>
-__device__ __forceinline__ void normalize8(Pack8<T>& x, int c8, int D, int b, int h, int N, int tok,
-                                           const NormArgs& a) {
+// Normalises the 8 channels c8..c8+7 of NR token rows held by this thread (tok[u]: the token of row u).  A row is spread
+// over TPR consecutive lanes (TPR = D/8); every lane of the warp must call this (full-mask shuffles).
+// LayerNorm: the root and the quotient of a row are computed by one of its lanes, another row's by another, and handed
+// round: as separately rounded IEEE operations they cost as much as the rest of a row's arithmetic.  The sums take the values
+// times 2^-896 (widen_word; an Inf or NaN makes the row's mean a NaN, as the sums of it would), in two passes over all
+// rows, so that the rows' shuffles overlap; the values are widened twice, which costs fewer instructions than keeping the
+// doubles costs registers.
+template <typename T, int NM, int TPR, int NR>
+__device__ __forceinline__ void normalize_rows(Pack8<T>* x, int c8, int D, int b, int h, int N, const int* tok, const NormArgs& a) {
   if constexpr (NM == PARO_NORM_LAYER_HEAD) {
-    float f[8];
-    double s = 0.0;
+    static_assert((NR & (NR - 1)) == 0 && NR <= TPR, "a lane of the row per row");
+    constexpr double INV_D = 1.0 / (8 * TPR);   // (a power of two: the product is the quotient)
+    float mean[NR], var[NR];
+    double sum[NR];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      f[j] = F16Traits<T>::to_float(x.e[j]);
-      s += (double)f[j];
+    for (int u = 0; u < NR; ++u) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&x[u].v);
+      double s = 0.0;
+      uint32_t top = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        double d0, d1;
+        widen_word<T>(w[j], d0, d1);
+        s += d0;
+        s += d1;
+        top = __vmaxu2(top, w[j] & 0x7fff7fffu);
+      }
+      s *= WIDE_SCALE;
+      if (max(top & 0xFFFFu, top >> 16) >= Inf16<T>::BITS) s = __hiloint2double(0x7ff80000, 0);
+      sum[u] = s;
     }
 #pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const double inv_d = 1.0 / (8 * TPR);   // (a power of two: the product is the quotient)
-    const float mean = __double2float_rn(s * inv_d);
-    double q = 0.0;
+    for (int o = TPR / 2; o > 0; o >>= 1)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double d = (double)f[j] - (double)mean;
-      q += d * d;
+      for (int u = 0; u < NR; ++u) sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], o);
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+      mean[u] = __double2float_rn(sum[u] * INV_D);
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&x[u].v);
+      const double m = (double)mean[u];
+      double q = 0.0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        double d0, d1;
+        widen_word<T>(w[j], d0, d1);
+        d0 = fma(d0, WIDE_SCALE, -m);   // (the product is exact)
+        q = fma(d0, d0, q);
+        d1 = fma(d1, WIDE_SCALE, -m);
+        q = fma(d1, d1, q);
+      }
+      sum[u] = q;
     }
 #pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    const float var = __double2float_rn(q * inv_d);
-    const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, a.eps)));
+    for (int o = TPR / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < NR; ++u) sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], o);
+#pragma unroll
+    for (int u = 0; u < NR; ++u) var[u] = __double2float_rn(sum[u] * INV_D);
+    const int lane = threadIdx.x & 31;
+    float mine = var[0];
+#pragma unroll
+    for (int u = 1; u < NR; ++u)
+      if (lane % NR == u) mine = var[u];
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mine, a.eps)));
     Pack8<T> w, bb;
     w.v = *reinterpret_cast<const uint4*>(static_cast<const T*>(a.weight) + c8);
+    bb.v = make_uint4(0, 0, 0, 0);
     if (a.bias) bb.v = *reinterpret_cast<const uint4*>(static_cast<const T*>(a.bias) + c8);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float y = __fmul_rn(__fmul_rn(__fsub_rn(f[j], mean), rstd), F16Traits<T>::to_float(w.e[j]));
-      if (a.bias) y = __fadd_rn(y, F16Traits<T>::to_float(bb.e[j]));
-      x.e[j] = F16Traits<T>::from_float(y);
+    for (int u = 0; u < NR; ++u) {
+      const float rstd = __shfl_sync(0xffffffffu, r, lane / TPR * TPR + u);
+      const uint64_t mean2 = pack2(mean[u], mean[u]), rstd2 = pack2(rstd, rstd);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t f = pack2(F16Traits<T>::to_float(x[u].e[2 * j]), F16Traits<T>::to_float(x[u].e[2 * j + 1]));
+        const uint64_t w2 = pack2(F16Traits<T>::to_float(w.e[2 * j]), F16Traits<T>::to_float(w.e[2 * j + 1]));
+        float y0, y1;
+        unpack2(mul2(mul2(sub2(f, mean2), rstd2), w2), y0, y1);
+        if (a.bias) {
+          y0 = __fadd_rn(y0, F16Traits<T>::to_float(bb.e[2 * j]));
+          y1 = __fadd_rn(y1, F16Traits<T>::to_float(bb.e[2 * j + 1]));
+        }
+        x[u].e[2 * j] = F16Traits<T>::from_float(y0);
+        x[u].e[2 * j + 1] = F16Traits<T>::from_float(y1);
+      }
     }
   } else if constexpr (NM == PARO_NORM_RMS_ALL) {
-    const float inv = a.inv_rms[(size_t)b * N + tok];
     Pack8<T> w;
-    w.v = *reinterpret_cast<const uint4*>(static_cast<const T*>(a.weight) + (size_t)h * D + c8);
+    w.v = ld_pinned16(static_cast<const T*>(a.weight) + (size_t)h * D + c8);
+    float inv[NR];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const T y1 = F16Traits<T>::from_float(__fmul_rn(F16Traits<T>::to_float(x.e[j]), inv));
-      x.e[j] = F16Traits<T>::from_float(__fmul_rn(F16Traits<T>::to_float(y1), F16Traits<T>::to_float(w.e[j])));
+    for (int u = 0; u < NR; ++u) inv[u] = a.inv_rms[(size_t)b * N + tok[u]];
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const T y1 = F16Traits<T>::from_float(__fmul_rn(F16Traits<T>::to_float(x[u].e[j]), inv[u]));
+        x[u].e[j] = F16Traits<T>::from_float(__fmul_rn(F16Traits<T>::to_float(y1), F16Traits<T>::to_float(w.e[j])));
+      }
     }
   }
 }

@@ -110,11 +110,23 @@ channel_stats_kernel(const StatsSrc src0, const StatsSrc src1, int H, int N, int
     gc.fill(rows, STATS_CHUNK, t0, N, D);
     __syncthreads();
   }
+  // The sums are taken of the values times 2^-896 (see widen_word): exact scaling, no conversions.  Maxima and minima of
+  // two channels at a time in the 16-bit type.  `top`: the largest magnitudes, as integers; a thread that meets an Inf or
+  // NaN goes over its rows again below.
+  using T2 = typename Two16<T>::type;
   double sum[8];
-  float mx[8], mn[8];
+  T2 mx[4], mn[4];
+  uint32_t top = 0;
+  const uint32_t inf2 = Inf16<T>::BITS * 0x10001u, minus_inf2 = inf2 | 0x80008000u;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) { sum[j] = 0.0; mx[j] = -INFINITY; mn[j] = INFINITY; }
-  // four rows are in flight per thread; they are accumulated in the order of a plain loop
+  for (int j = 0; j < 8; ++j) sum[j] = 0.0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    mx[j] = *reinterpret_cast<const T2*>(&minus_inf2);
+    mn[j] = *reinterpret_cast<const T2*>(&inf2);
+  }
+  // four rows are in flight per thread; they are accumulated in the order of a plain loop.  (Eight do not help: 54 us for K
+  // and V of 5 x 75600 x 128 either way.)
   for (int t = t0 + r; t < t1; t += 4 * ROWS) {
     Pack8<T> v[4];
 #pragma unroll
@@ -130,21 +142,41 @@ channel_stats_kernel(const StatsSrc src0, const StatsSrc src1, int H, int N, int
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (t + u * ROWS >= t1) break;
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&v[u].v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float f = F16Traits<T>::to_float(v[u].e[j]);
-        sum[j] += (double)f;
+      for (int j = 0; j < 4; ++j) {
+        double lo, hi;
+        widen_word<T>(w[j], lo, hi);
+        sum[2 * j] += lo;
+        sum[2 * j + 1] += hi;
+        top = __vmaxu2(top, w[j] & 0x7fff7fffu);
         if (EXTREMES) {
-          mx[j] = fmaxf(mx[j], f);
-          mn[j] = fminf(mn[j], f);
+          const T2 x = *reinterpret_cast<const T2*>(w + j);
+          mx[j] = __hmax2(mx[j], x);
+          mn[j] = __hmin2(mn[j], x);
         }
       }
     }
   }
 #pragma unroll
+  for (int j = 0; j < 8; ++j) sum[j] *= WIDE_SCALE;
+  if (max(top & 0xFFFFu, top >> 16) >= Inf16<T>::BITS) {
+    for (int j = 0; j < 8; ++j) sum[j] = 0.0;
+    for (int t = t0 + r; t < t1; t += ROWS) {
+      Pack8<T> v;
+      v.v = *reinterpret_cast<const uint4*>(base + (size_t)(GM == GM_PLAIN ? t : rows.src[t - t0]) * sn + c8);
+      if constexpr (GM == GM_ROPE_F32 || GM == GM_ROPE_F64) gc.template rotate<1>(&v, pa, rows, t - t0, 0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum[j] += (double)F16Traits<T>::to_float(v.e[j]);
+    }
+  }
+#pragma unroll
   for (int j = 0; j < 8; ++j) {
     s_sum[r][c8 + j] = sum[j];
-    if (EXTREMES) { s_mx[r][c8 + j] = mx[j]; s_mn[r][c8 + j] = mn[j]; }
+    if (EXTREMES) {
+      s_mx[r][c8 + j] = F16Traits<T>::to_float(j & 1 ? mx[j >> 1].y : mx[j >> 1].x);
+      s_mn[r][c8 + j] = F16Traits<T>::to_float(j & 1 ? mn[j >> 1].y : mn[j >> 1].x);
+    }
   }
   __syncthreads();
   if (threadIdx.x < D) {
@@ -302,10 +334,17 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
       if (first + blk * 64 + r0 + i * RPL < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn);
     }
     if constexpr (NM != PARO_NORM_NONE) {
+// all lanes: the row statistics are reduced with full-warp shuffles
+      constexpr int NORM_ROWS = LOADS < 4 ? LOADS : 4;
 #pragma unroll
-      for (int i = 0; i < LOADS; ++i) {   // all lanes: the row statistics are reduced with full-warp shuffles
-        const int src = source(blk, i);
-        normalize8<T, NM, TPR>(row[i], c8, D, b, h, N, first + blk * 64 + r0 + i * RPL < N ? src : 0, norm);
+      for (int i = 0; i < LOADS; i += NORM_ROWS) {
+        int tok[NORM_ROWS];
+#pragma unroll
+        for (int u = 0; u < NORM_ROWS; ++u) {
+          const int src = source(blk, i + u);
+          tok[u] = first + blk * 64 + r0 + (i + u) * RPL < N ? src : 0;
+        }
+        normalize_rows<T, NM, TPR, NORM_ROWS>(row + i, c8, D, b, h, N, tok, norm);
       }
     }
     if constexpr (TABLE) {

@@ -10,6 +10,7 @@ namespace paro {
 
 // Block = 256 threads = 64 (D = 128) or 128 rows; a thread owns one 16-byte slice of PASSES consecutive rows.
 // blockIdx.x: group of rows, blockIdx.y: b*H + h.
+constexpr int PERM_NORM_ROWS = 2;   // rows normalised together
 template <typename T, int D, int MODE, int NM>
 __global__ void __launch_bounds__(256, 4)
 rope_permute_kernel(const T* __restrict__ in, T* __restrict__ out, int H, int N,
@@ -39,9 +40,11 @@ rope_permute_kernel(const T* __restrict__ in, T* __restrict__ out, int H, int N,
   [[maybe_unused]] const PairAxes pa(c8, rope);
   // every lane takes part in the normalisation's shuffles, also those whose row is past the end
   if constexpr (NM != PARO_NORM_NONE) {
+int tok[PASSES];
 #pragma unroll
-    for (int i = 0; i < PASSES; ++i)
-      normalize8<T, NM, TPR>(val[i], c8, D, b, h, N, tok0 + r0 + i < N ? rows.src[r0 + i] : 0, norm);
+    for (int i = 0; i < PASSES; ++i) tok[i] = tok0 + r0 + i < N ? rows.src[r0 + i] : 0;
+#pragma unroll
+    for (int i = 0; i < PASSES; i += PERM_NORM_ROWS) normalize_rows<T, NM, TPR, PERM_NORM_ROWS>(val + i, c8, D, b, h, N, tok + i, norm);
   }
   if constexpr (MODE != PARO_ROPE_NONE) {
     constexpr int NR = MODE == PARO_ROPE_REAL_F32 ? ROTATE_ROWS_F32 : ROTATE_ROWS_F64;
