@@ -5,11 +5,10 @@
 
 namespace paro {
 
-__global__ void perm_index_kernel(const int32_t* __restrict__ order_ids, int F, int Hh, int W,
+__global__ void perm_index_kernel(const int32_t* __restrict__ order_ids, const GridDims dims, int n_img,
                                   int32_t* __restrict__ idx) {
   const int h = blockIdx.y;
-  const int n_img = F * Hh * W;
-  const PermDecoder dec(order_ids[h], F, Hh, W);
+  const PermDecoder dec(order_ids[h], dims);
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n_img; j += gridDim.x * blockDim.x) {
     int f, y, x;
     idx[(size_t)h * n_img + j] = dec.source(j, f, y, x);
@@ -147,7 +146,7 @@ extern "C" int paro_build_perm_index(const int32_t* order_ids, int H, int F, int
   PARO_REQUIRE((int64_t)F * Hh * W < (1ll << 31), PARO_ESHAPE, "paro_build_perm_index: grid too large");
   const int n_img = F * Hh * W;
   dim3 grid((unsigned)min(1024, (n_img + 255) / 256), (unsigned)H);
-  perm_index_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(order_ids, F, Hh, W, idx);
+  perm_index_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(order_ids, grid_dims(F, Hh, W), n_img, idx);
   return check_launch("perm_index_kernel");
 }
 

@@ -19,7 +19,8 @@ namespace paro {
 // consume RoPE + per-head reordering on the fly instead of a materialised bf16 copy.
 struct Gather {
   int enabled;        // 0: plain input, tok -> tok, no RoPE
-  int n_text, F, Hh, W;
+  int n_text;
+  GridDims dims;
   const int32_t* order_ids;   // [H] or nullptr (natural order)
   RopeArgs rope;
 };
@@ -40,7 +41,7 @@ struct GatherCtx {
   const Gather& g;
   PermDecoder dec;
   __device__ GatherCtx(const Gather& g_, int h)
-      : g(g_), dec(GM != GM_PLAIN && g_.order_ids ? g_.order_ids[h] : 0, g_.F, g_.Hh, g_.W) {}
+      : g(g_), dec(GM != GM_PLAIN && g_.order_ids ? g_.order_ids[h] : 0, g_.dims) {}
   // source token of row `tok`
   __device__ __forceinline__ int source(int tok) const {
     int f, y, x;
@@ -50,7 +51,7 @@ struct GatherCtx {
   }
   // Entry r of the table: row tok0 + r of the sequence (rows past the end: not rotated).
   template <int ROWS> __device__ __forceinline__ void fill(RowTable<ROWS>& t, int rows, int tok0, int N, int D) const {
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) fill_row(t, r, tok0 + r, N, D >> 2, dec, g.n_text, g.F, g.Hh);
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) fill_row(t, r, tok0 + r, N, D >> 2, dec, g.n_text, g.dims);
   }
   // rows r, r + step, ... of the table
   template <int NR, typename T, int ROWS>
@@ -451,44 +452,50 @@ quant_int8_kernel(const T* __restrict__ x, const T* __restrict__ km, int8_t* __r
 // 8*(row/2) + 2*matrix + row%2 of a 32-token group.  A thread then stores 16 bytes and four lanes together
 // 64, whole sectors.  16-byte chunks are XOR-swizzled by (token & 1) | (token/8 & 3) * 2, which takes the
 // eight rows of every matrix to different banks.
+// A CTA takes `blocks` consecutive blocks: the source tokens of all of them are worked out once, a row per thread, and the
+// channels' means and scales are read once (one block each, its rows decoded by its warps with integer divisions: 45 us for
+// 5 x 75600 x 128, 119 for 2 x 48 x 17776 x 64, 89 % of the issue slots; now 40 and 92).
+constexpr int V_BLOCKS = 4;
 template <typename T, int D, int GM>
 __global__ void __launch_bounds__(256)
 quant_v_fp8_kernel(const T* __restrict__ v, int H, int N, int npad, int64_t sb, int64_t sh, int64_t sn,
                    const float* __restrict__ inv_tab, const float* __restrict__ mean_tab,
-                   uint8_t* __restrict__ v8, __nv_bfloat16* __restrict__ v16, const Gather gather) {
+                   uint8_t* __restrict__ v8, __nv_bfloat16* __restrict__ v16, int blocks, const Gather gather) {
   constexpr int TPR = D / 8;                // 16-byte chunks (= threads) per row
   constexpr int ROWS = 256 / TPR;
   constexpr int LOADS = 64 / ROWS;
-  __shared__ __align__(16) uint4 tile[64 * TPR];
+  __shared__ __align__(16) uint4 tiles[2][64 * TPR];   // (two: one barrier per block)
+  __shared__ int s_src[GM == GM_PLAIN ? 1 : 64 * V_BLOCKS];
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
-  const int t0 = blockIdx.x * 64;
+  const int first_tok = blockIdx.x * blocks * 64, n_blocks = min(blocks, (N - first_tok + 63) / 64);
   const T* base = v + b * sb + h * sh;
   auto slot = [](int token, int chunk) { return token * TPR + (chunk ^ ((token & 1) | ((token >> 3) & 3) << 1)); };
-  {
+  const int c = threadIdx.x % TPR, r0 = threadIdx.x / TPR;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if constexpr (GM != GM_PLAIN) {
     const GatherCtx<GM> gc(gather, h);
-    const int c = threadIdx.x % TPR, r0 = threadIdx.x / TPR;
-    constexpr int RPW = 32 / TPR;           // rows a warp covers with one load
-    const int lane = threadIdx.x & 31;
+    const int t = first_tok + threadIdx.x;
+    static_assert(64 * V_BLOCKS == 256, "a row per thread");
+    s_src[threadIdx.x] = t < N ? gc.source(t) : 0;
+  }
+  uint64_t mean2[4], inv2[4];               // inv = scale_max / amax, from the finalize pass
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    mean2[j] = *reinterpret_cast<const uint64_t*>(mean_tab + (size_t)bh * D + c * 8 + 2 * j);
+    inv2[j] = *reinterpret_cast<const uint64_t*>(inv_tab + (size_t)bh * D + c * 8 + 2 * j);
+  }
+  if constexpr (GM != GM_PLAIN) __syncthreads();
+#pragma unroll 1
+  for (int blk = 0; blk < n_blocks; ++blk) {
+    const int t0 = first_tok + blk * 64;
+    uint4* const tile = tiles[blk & 1];
     Pack8<T> row[LOADS];
-    // each of the warp's eight rows is decoded once, by lane (load, row of the load), and handed to its threads
-    int d_src = 0;
-    if constexpr (GM != GM_PLAIN) {
-      const int t = t0 + (threadIdx.x >> 5) * RPW + lane % RPW + (lane / RPW) % LOADS * ROWS;
-      if (t < N) d_src = gc.source(t);
-    }
 #pragma unroll
     for (int i = 0; i < LOADS; ++i) {
-      const int tok = t0 + r0 + i * ROWS;
-      int src = tok;
-      if constexpr (GM != GM_PLAIN) src = __shfl_sync(0xffffffffu, d_src, i * RPW + lane / TPR);
+      const int r = r0 + i * ROWS;
+      const int src = GM == GM_PLAIN ? t0 + r : s_src[blk * 64 + r];
       row[i].v = make_uint4(0, 0, 0, 0);
-      if (tok < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn + c * 8);
-    }
-    float mean[8], inv[8];                  // inv = scale_max / amax, from the finalize pass
-#pragma unroll
-    for (int j = 0; j < 8; j += 4) {
-      *reinterpret_cast<float4*>(mean + j) = *reinterpret_cast<const float4*>(mean_tab + (size_t)bh * D + c * 8 + j);
-      *reinterpret_cast<float4*>(inv + j) = *reinterpret_cast<const float4*>(inv_tab + (size_t)bh * D + c * 8 + j);
+      if (t0 + r < N) row[i].v = *reinterpret_cast<const uint4*>(base + (size_t)src * sn + c * 8);
     }
 #pragma unroll
     for (int i = 0; i < LOADS; ++i) {
@@ -497,9 +504,10 @@ quant_v_fp8_kernel(const T* __restrict__ v, int H, int N, int npad, int64_t sb, 
       if (t0 + r < N) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float y0 = __fmul_rn(__fsub_rn(F16Traits<T>::to_float(row[i].e[2 * j]), mean[2 * j]), inv[2 * j]);
-          const float y1 = __fmul_rn(__fsub_rn(F16Traits<T>::to_float(row[i].e[2 * j + 1]), mean[2 * j + 1]), inv[2 * j + 1]);
-          const __nv_fp8x2_storage_t p = __nv_cvt_float2_to_fp8x2(make_float2(y0, y1), __NV_SATFINITE, __NV_E4M3);
+          const uint64_t f = pack2(F16Traits<T>::to_float(row[i].e[2 * j]), F16Traits<T>::to_float(row[i].e[2 * j + 1]));
+          float2 y;
+          unpack2(mul2(sub2(f, mean2[j]), inv2[j]), y.x, y.y);
+          const __nv_fp8x2_storage_t p = __nv_cvt_float2_to_fp8x2(y, __NV_SATFINITE, __NV_E4M3);
           // e4m3 -> fp16 -> bf16: both steps exact (3 mantissa bits, exponents inside either range)
           const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(p, __NV_E4M3);
           const __nv_bfloat162 b2 = __floats2bfloat162_rn(__half2float(__half(__half_raw{h2.x})), __half2float(__half(__half_raw{h2.y})));
@@ -508,27 +516,26 @@ quant_v_fp8_kernel(const T* __restrict__ v, int H, int N, int npad, int64_t sb, 
       }
       tile[slot(r, c)] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
 #pragma unroll
-  for (int u = warp; u < 2 * TPR; u += 8) {   // unit = 8 channels x 32 tokens
-    const int chunk = u >> 1, tg = (u & 1) * 32;
-    const int tok = tg + 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);   // the row this lane points ldmatrix at
-    const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(tile + slot(tok, chunk)));
-    uint32_t w[4];
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
-    const int d = chunk * 8 + (lane >> 2), first = t0 + tg + (lane & 3) * 8;
-    const size_t o = ((size_t)bh * D + d) * npad + first;
-    if (v16) *reinterpret_cast<uint4*>(v16 + o) = make_uint4(w[0], w[1], w[2], w[3]);
-    if (v8) {   // the bf16 values are e4m3 values: the conversion back is exact
-      uint32_t q[4];
+    for (int u = warp; u < 2 * TPR; u += 8) {   // unit = 8 channels x 32 tokens
+      const int chunk = u >> 1, tg = (u & 1) * 32;
+      const int tok = tg + 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);   // the row this lane points ldmatrix at
+      const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(tile + slot(tok, chunk)));
+      uint32_t w[4];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+      const int d = chunk * 8 + (lane >> 2), first = t0 + tg + (lane & 3) * 8;
+      const size_t o = ((size_t)bh * D + d) * npad + first;
+      if (v16) *reinterpret_cast<uint4*>(v16 + o) = make_uint4(w[0], w[1], w[2], w[3]);
+      if (v8) {   // the bf16 values are e4m3 values: the conversion back is exact
+        uint32_t q[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        q[j] = __nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u)),
-                                        __NV_SATFINITE, __NV_E4M3);
-      *reinterpret_cast<uint2*>(v8 + o) = make_uint2(q[0] | q[1] << 16, q[2] | q[3] << 16);
+        for (int j = 0; j < 4; ++j)
+          q[j] = __nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u)),
+                                          __NV_SATFINITE, __NV_E4M3);
+        *reinterpret_cast<uint2*>(v8 + o) = make_uint2(q[0] | q[1] << 16, q[2] | q[3] << 16);
+      }
     }
   }
 }
@@ -663,16 +670,19 @@ template <typename T>
 void launch_v_fp8(const void* v, int B, int H, int N, int D, int64_t sb, int64_t sh, int64_t sn, const float* inv_tab,
                   const float* mean_tab, uint8_t* v8, uint16_t* v16, cudaStream_t s, const Gather& g) {
   const int npad = (N + 63) / 64 * 64;
-  dim3 grid(npad / 64, B * H);
+  const int nb = npad / 64;
+  const int64_t total = (int64_t)nb * B * H;
+  const int blocks = total >= 148 * 24 ? V_BLOCKS : total >= 148 * 12 ? 2 : 1;   // (as long as every SM gets several CTAs)
+  dim3 grid((nb + blocks - 1) / blocks, B * H);
   dispatch_gather(g, [&](auto gm) {
     // the V pass never rotates: reordering only
     constexpr int GM = decltype(gm)::value == GM_PLAIN ? GM_PLAIN : GM_REORDER;
     if (D == 128)
       quant_v_fp8_kernel<T, 128, GM><<<grid, 256, 0, s>>>((const T*)v, H, N, npad, sb, sh, sn, inv_tab, mean_tab, v8,
-                                                          (__nv_bfloat16*)v16, g);
+                                                          (__nv_bfloat16*)v16, blocks, g);
     else
       quant_v_fp8_kernel<T, 64, GM><<<grid, 256, 0, s>>>((const T*)v, H, N, npad, sb, sh, sn, inv_tab, mean_tab, v8,
-                                                         (__nv_bfloat16*)v16, g);
+                                                         (__nv_bfloat16*)v16, blocks, g);
   });
 }
 
@@ -781,7 +791,8 @@ int make_gather(Gather* g, const char* who, int N, int D, int n_text, int F, int
                "%s: n_text + F*H*W = %lld != N = %d", who, (long long)n_text + (long long)F * Hh * W, N);
   if (int rc = check_rope(who, rope_mode, cos_tab, sin_tab, pairs_f, pairs_h, D)) return rc;
   g->enabled = 1;
-  g->n_text = n_text; g->F = F; g->Hh = Hh; g->W = W;
+  g->n_text = n_text;
+  g->dims = grid_dims(F, Hh, W);
   g->order_ids = order_ids;
   g->rope = make_rope(rope_mode, cos_tab, sin_tab, pairs_f, pairs_h);
   return PARO_OK;

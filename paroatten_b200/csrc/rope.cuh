@@ -66,13 +66,13 @@ template <int ROWS> struct RowTable {
 
 template <int ROWS>
 __device__ __forceinline__ void fill_row(RowTable<ROWS>& t, int r, int tok, int N, int quarter, const PermDecoder& dec,
-                                         int n_text, int F, int Hh) {
+                                         int n_text, const GridDims& g) {
   int src = tok, f = -1, y = 0, x = 0;
   if (tok >= n_text && tok < N) src = n_text + dec.source(tok - n_text, f, y, x);
   t.src[r] = src;
   t.off[0][r] = f < 0 ? -1 : f * quarter;
-  t.off[1][r] = f < 0 ? -1 : (F + y) * quarter;
-  t.off[2][r] = f < 0 ? -1 : (F + Hh + x) * quarter;
+  t.off[1][r] = f < 0 ? -1 : (g.f.d + y) * quarter;
+  t.off[2][r] = f < 0 ? -1 : (g.f.d + g.y.d + x) * quarter;
 }
 
 // What a thread that owns channels c8..c8+7 needs to find its four pairs' angles: the axis that drives each.
