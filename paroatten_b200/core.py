@@ -8,7 +8,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib
-from .plan import (CompactPlan, PermutePlan, PlanStore, SparsePlan, apply_empty_heads, compact_plan, perm_index)
+from .plan import (CompactPlan, PermutePlan, PlanStore, SparsePlan, apply_empty_heads, begin_plan, compact_plan, perm_index)
 from .quant import _hnd, channel_mean, per_channel_fp8, per_warp_int8, per_block_int8
 from .rope import RopeTables, _NO_ROPE, _norm_params
 
@@ -252,10 +252,6 @@ def _pad_head_dim(*ts):
     return tuple(F.pad(t, (0, target - d)) for t in ts), d
 
 
-def _as_plan(sparse: Union[torch.Tensor, CompactPlan]) -> CompactPlan:
-    return sparse if isinstance(sparse, CompactPlan) else compact_plan(sparse)
-
-
 @torch.compiler.disable
 def paroattn_qk_int8_pv_fp16_cuda(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
                                   sparse: Union[torch.Tensor, CompactPlan], tensor_layout: str = "HND",
@@ -286,6 +282,9 @@ def paroattn_qk_int8_pv_fp16_cuda(q: torch.Tensor, k: torch.Tensor, v: torch.Ten
     if sm_scale is None:
         sm_scale = head_dim_og ** -0.5
     with torch.cuda.device(q.device):
+        # a mask's compaction begins before the quantisers are issued and ends behind them: the GPU works on these while the
+        # host waits for the lists' lengths
+        finish_plan = None if isinstance(sparse, CompactPlan) else begin_plan(sparse)
         km = channel_mean(k, tensor_layout) if smooth_k else None
         if qk_quant_gran == "per_warp":
             q8, qs, k8, ks = per_warp_int8(q, k, km, BLKQ=64, WARPQ=32, BLKK=64, tensor_layout=tensor_layout)
@@ -298,7 +297,8 @@ def paroattn_qk_int8_pv_fp16_cuda(q: torch.Tensor, k: torch.Tensor, v: torch.Ten
         _, vs, vm, v16 = per_channel_fp8(v, tensor_layout, smooth_v=smooth_v, return_16=True)
         if tensor_layout == "NHD":
             q8, k8 = q8.transpose(1, 2), k8.transpose(1, 2)  # back to the HND buffers
-        res = sparse_attn_quantized(q8, qs, k8, ks, v16, vs, vm, _as_plan(sparse), scale, out_dtype=dtype,
+        plan = finish_plan() if finish_plan else sparse
+        res = sparse_attn_quantized(q8, qs, k8, ks, v16, vs, vm, plan, scale, out_dtype=dtype,
                                     q_group=group, return_lse=return_lse, out_layout=tensor_layout, mode=attn_mode)
     o, lse = res if return_lse else (res, None)
     o = o[..., :head_dim_og]

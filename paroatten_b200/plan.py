@@ -135,6 +135,13 @@ def compact_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: s
     k-blocks they share (pair_rows_by_overlap), kept for the slices (heads) where that needs fewer tiles than adjacency.
     The choice is made slice by slice, so that a head's plan -- and with it the order in which its rows
     accumulate -- does not depend on which other heads are compacted with it."""
+    return begin_plan(mask, validate, pairing)()
+
+
+def begin_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: str = "adjacent"):
+    """compact_plan in two parts: launches everything up to the lists' lengths and returns a function that waits for these,
+    makes the lists and returns the plan.  A caller with other work for the stream issues it in between, so that the GPU does
+    not stand still while the host reads three numbers and allocates (on the calling thread's current stream, both times)."""
     if pairing not in ("adjacent", "overlap"):
         raise ValueError(f"unknown pairing {pairing!r}")
     _lib.require_cuda(mask)
@@ -160,24 +167,35 @@ def compact_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: s
         s = _lib.stream_ptr()
         _lib.check(L.paro_plan_offsets(m.data_ptr(), slices, nbq, nbk, overlap, row_ptr.data_ptr(), pair_ptr.data_ptr(),
                                        _lib.ptr(pair_q), totals.data_ptr(), scratch.data_ptr(), scratch.numel(), s))
-        kept, tiles, paired, expired = totals.tolist()      # the lists' lengths: the one synchronisation of the call
+        # the lists' lengths, read by the host in `finish`: the one synchronisation of the call
+        lengths = torch.empty(4, dtype=torch.int32, pin_memory=True)
+        lengths.copy_(totals, non_blocking=True)
+        arrived = torch.cuda.Event()
+        arrived.record()
+        sched_cnt = torch.empty(slices * npairs, 2, dtype=torch.int32, device=dev)
+
+    def finish() -> CompactPlan:
+        arrived.synchronize()
+        kept, tiles, paired, expired = lengths.tolist()
         if expired:
             raise _lib.ParoError(_lib.PARO_ETIMEOUT, "a wait of the q-block pairing expired")
-        cols = torch.empty(max(kept, 1), dtype=torch.int32, device=dev)
-        pair_ent = torch.empty(max(tiles, 1), dtype=torch.int32, device=dev)
-        sched = torch.empty(max(tiles, 1), dtype=torch.int32, device=dev)
-        sched_cnt = torch.empty(slices * npairs, 2, dtype=torch.int32, device=dev)
-        cnt_kernel = torch.empty_like(sched_cnt) if paired else None
-        _lib.check(L.paro_plan_lists(slices, nbq, nbk, overlap, row_ptr.data_ptr(), pair_ptr.data_ptr(), _lib.ptr(pair_q),
-                                     cols.data_ptr(), pair_ent.data_ptr(), sched.data_ptr(), sched_cnt.data_ptr(),
-                                     _lib.ptr(cnt_kernel), scratch.data_ptr(), scratch.numel(), s))
-    plan = CompactPlan(slices, nbq, nbk, row_ptr, cols[:kept], pair_ptr, pair_ent[:tiles], kept, tiles,
-                       sched[:tiles], sched_cnt)
-    if validate:
-        validate_plan(plan)
-    if paired:
-        plan.pair_q, plan.sched_cnt_kernel = pair_q, cnt_kernel
-    return plan
+        with torch.cuda.device(dev):
+            cols = torch.empty(max(kept, 1), dtype=torch.int32, device=dev)
+            pair_ent = torch.empty(max(tiles, 1), dtype=torch.int32, device=dev)
+            sched = torch.empty(max(tiles, 1), dtype=torch.int32, device=dev)
+            cnt_kernel = torch.empty_like(sched_cnt) if paired else None
+            _lib.check(L.paro_plan_lists(slices, nbq, nbk, overlap, row_ptr.data_ptr(), pair_ptr.data_ptr(), _lib.ptr(pair_q),
+                                         cols.data_ptr(), pair_ent.data_ptr(), sched.data_ptr(), sched_cnt.data_ptr(),
+                                         _lib.ptr(cnt_kernel), scratch.data_ptr(), scratch.numel(), s))
+        plan = CompactPlan(slices, nbq, nbk, row_ptr, cols[:kept], pair_ptr, pair_ent[:tiles], kept, tiles,
+                           sched[:tiles], sched_cnt)
+        if validate:
+            validate_plan(plan)
+        if paired:
+            plan.pair_q, plan.sched_cnt_kernel = pair_q, cnt_kernel
+        return plan
+
+    return finish
 
 
 class SparsePlan:

@@ -1,0 +1,105 @@
+"""The pre-attention passes at the sizes where their launches change form, and on Inf, NaN and signed extremes; the mask's
+packing at any address.  Everything here is exact."""
+import pytest
+import torch
+
+import paroatten_b200 as pb
+from oracle import paro_oracle as po
+
+pytestmark = pytest.mark.gpu
+GRIDS = {2560: (4, 20, 32), 4864: (19, 16, 16), 4805: (5, 31, 31), 40: (1, 1, 40), 91: (7, 1, 13)}
+
+
+def rand(*shape, dtype=torch.bfloat16, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(dtype).cuda()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N, D, family, norm", [(2560, 128, "wan", "none"), (4864, 64, "cogvideox", "layer"), (4805, 128, "wan", "rms"),
+                                               (4805, 64, "cogvideox", "none"), (40, 64, "none", "layer"), (91, 128, "wan", "none")])
+def test_many_heads_at_once_equal_one_head_at_a_time(N, D, family, norm, dtype):
+    """Several blocks of rows per CTA from some size on, one below it: the same bits (48 heads against one).  RMS norm takes its
+    statistic over the heads, so that pass is compared with the separate ones instead."""
+    H, grid = 48, GRIDS[N]
+    x, v = rand(1, H, N, D, dtype=dtype), rand(1, H, N, D, dtype=dtype, seed=1)
+    orders = (torch.arange(H) % 6).to(torch.int32).cuda()
+    rope = pb.rope_tables(grid, D, family) if family != "none" else None
+    nm = None if norm != "layer" else pb.QKNorm("layer", rand(D, dtype=dtype, seed=2), rand(D, dtype=dtype, seed=3), 1e-6)
+    if norm == "rms":
+        nm = pb.QKNorm("rms", rand(H * D, dtype=dtype, seed=2), None, 1e-6)
+    whole = [pb.rope_permute(x, orders, grid, 0, rope, norm=nm), *pb.prep_qk_int8(x, orders, grid, 0, rope, group=32, norm=nm)[:2]]
+    if nm is None:
+        whole += pb.prep_qk_int8(x, orders, grid, 0, rope, group=64, smooth=True)
+    whole += [t for t in pb.prep_v_fp8(v, orders, grid, 0) if t is not None]
+    if norm == "rms":     # rotation + reorder of the normalised copy, then the plain quantiser
+        q8, qs = pb.quant._quant_int8(whole[0], "HND", 32)
+        assert torch.equal(whole[1], q8) and torch.equal(whole[2], qs)
+    for h in (0, 1, 2, 5, H - 1):
+        xs, vs, o = x[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous(), orders[h:h + 1].contiguous()
+        part = [] if norm == "rms" else [pb.rope_permute(xs, o, grid, 0, rope, norm=nm),
+                                         *pb.prep_qk_int8(xs, o, grid, 0, rope, group=32, norm=nm)[:2]]
+        if nm is None:
+            part += pb.prep_qk_int8(xs, o, grid, 0, rope, group=64, smooth=True)
+        part += [t for t in pb.prep_v_fp8(vs, o, grid, 0) if t is not None]
+        for a, b in zip(whole[len(whole) - len(part):], part):
+            assert torch.equal(a[:, h:h + 1], b)
+
+
+def int8_rule(x, group, mean=None):
+    """The quantiser's rule in plain torch: amax ignores NaN and is at least 1e-7; NaN becomes 0."""
+    f = x.float() - (mean.float().unsqueeze(2) if mean is not None else 0)
+    B, H, N, D = f.shape
+    n = -(-N // 64) * 64
+    g = torch.nn.functional.pad(f, (0, 0, 0, n - N)).view(B, H, n // group, group * D)
+    amax = g.abs().nan_to_num(nan=0.0, posinf=float("inf")).amax(-1).clamp(min=1e-7)
+    inv = torch.div(torch.full_like(amax, 127.0), amax)     # (127.0 / amax would be a rounded reciprocal times 127)
+    q = (g * inv.unsqueeze(-1)).nan_to_num(nan=0.0, posinf=127.0, neginf=-128.0).round().clamp(-128, 127).to(torch.int8)
+    return q.view(B, H, n, D)[:, :, :N], torch.div(amax, torch.full_like(amax, 127.0))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf"), 0.0])
+def test_special_values(bad, D, dtype):
+    N, H = 200, 2
+    x = rand(1, H, N, D, dtype=dtype).cpu()
+    x[0, 0, 3, 5] = bad
+    x[0, 1, 130, D - 1] = bad
+    x[0, 1, 190] = torch.finfo(dtype).max
+    x[0, 0, 64:128] = 0
+    x[0, 0, 70, 1] = -torch.finfo(dtype).tiny / 4
+    for group in (32, 64):
+        q, s = pb.quant._quant_int8(x.cuda(), "HND", group)
+        want_q, want_s = int8_rule(x, group)
+        assert torch.equal(q.cpu(), want_q) and torch.equal(s.cpu().view_as(want_s), want_s)
+    km = rand(1, H, D, dtype=dtype, seed=4).cpu()
+    q, s = pb.quant._quant_int8(x.cuda(), "HND", 64, km=km.cuda())
+    want_q, want_s = int8_rule(x, 64, km)
+    assert torch.equal(q.cpu(), want_q) and torch.equal(s.cpu().view_as(want_s), want_s)
+    # sums: only the channels with the value feel it
+    mean = pb.channel_mean(x.cuda(), out_dtype=torch.float32).cpu()
+    want = (x.double().sum(2) / N).float().view_as(mean)
+    assert torch.equal(mean.isnan(), want.isnan()) and torch.equal(mean.nan_to_num(), want.nan_to_num())
+    # LayerNorm: a row that holds an Inf or NaN is NaN as a whole, the others do not feel it
+    grid = (2, 10, 10)
+    w, b = rand(D, dtype=dtype, seed=5), rand(D, dtype=dtype, seed=6)
+    got = pb.rope_permute(x.cuda(), None, grid, 0, None, norm=pb.QKNorm("layer", w, b, 1e-6)).cpu()
+    finite = x.isfinite().all(-1)
+    assert got[~finite].isnan().all()
+    clean = x.clone()
+    clean[~finite] = 1
+    same = pb.rope_permute(clean.cuda(), None, grid, 0, None, norm=pb.QKNorm("layer", w, b, 1e-6)).cpu()
+    assert torch.equal(got[finite], same[finite])
+
+
+@pytest.mark.parametrize("nbq, nbk", [(4, 4), (9, 33), (17, 127), (40, 129), (12, 1530), (8, 1600)])
+@pytest.mark.parametrize("offset", [0, 1, 7, 15])
+def test_masks_at_any_address(nbq, nbk, offset):
+    g = torch.Generator().manual_seed(nbk)
+    mask = torch.rand(2, nbq, nbk, generator=g) < 0.3
+    buf = torch.full((offset + mask.numel(),), 255, dtype=torch.uint8, device="cuda")
+    view = buf[offset:].view(2, nbq, nbk)
+    view.copy_(mask.to(torch.uint8) * (1 + torch.randint(0, 255, mask.shape, generator=g).to(torch.uint8)))
+    plan = pb.compact_plan(view)
+    ptr, cols = po.compact_plan(mask)
+    assert torch.equal(plan.row_ptr.cpu(), ptr) and torch.equal(plan.cols.cpu(), cols)
