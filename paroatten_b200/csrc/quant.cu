@@ -608,8 +608,8 @@ void launch_int8_norm(const void* x, const void* km, int8_t* out, float* scale, 
   dispatch_gather(g, [&](auto gm) {
     constexpr int GM = decltype(gm)::value;
     // Several blocks per CTA where that leaves every SM a few CTAs; below that one each, for the latency.  Three or four
-    // CTAs fit an SM: four blocks each from 21 blocks per SM on, two from five blocks per SM on (1, 2, 4 blocks, us, Q in bf16
-    // with the fp64 rotation: 12 x 32760 x 128 92, 82, 78; 20 x 7800 x 128 39, 35, 39; 24 x 2926 x 64 14.5, 12.5, 12.5;
+    // CTAs fit an SM: four blocks each from 21 blocks per SM on, two from five blocks per SM on (1, 2, 4 blocks, us, in scalar
+    // arithmetic, Q in bf16 with the fp64 rotation: 12 x 32760 x 128 92, 82, 78; 20 x 7800 x 128 39, 35, 39; 24 x 2926 x 64 14.5, 12.5, 12.5;
     // 2 x 12 x 1560 x 128 14.5, 14.5, 18.6, with LayerNorm 19, 21, 29).
     const int64_t total = (int64_t)nb * B * H;
     const int blocks = !Int8Cfg<GM, D>::TABLE ? 1 : total >= 148 * 21 ? INT8_BLOCKS : total >= 148 * 5 ? 2 : 1;

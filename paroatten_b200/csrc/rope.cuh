@@ -107,7 +107,7 @@ __device__ __forceinline__ uint32_t rotate_pair_f32(float x0, float x1, float c,
 // 16-bit value the fp64 result between them does too.  On N(0,1) inputs one pair of values in 2^10.6 is uncertain for
 // bf16 and in 2^7.9 for fp16; so are zeros and everything whose e is not finite: an Inf or NaN operand, or a product past
 // the range of fp32 (r-e and r+e may then be the same NaN, where fp64 has a value).  Those show in `worst`, the largest
-// e so far or NaN.  Of 2 x 12 x 32760 x 128, bf16 and fp16: INT8 Q 142 and 148 us, rotation + reorder 107 and 113; with one
+// e so far or NaN.  In scalar arithmetic, of 2 x 12 x 32760 x 128, bf16 and fp16: INT8 Q 142 and 148 us, rotation + reorder 107 and 113; with one
 // e from (|x0|+|x1|) * (|c|+|s|), four times as many unsettled pairs and all four of a thread settled together 149 and
 // 172, 115 and 133; with fp64 alone 167 and 164, 138 and 144.
 //

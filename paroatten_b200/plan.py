@@ -135,13 +135,15 @@ def compact_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: s
     k-blocks they share (pair_rows_by_overlap), kept for the slices (heads) where that needs fewer tiles than adjacency.
     The choice is made slice by slice, so that a head's plan -- and with it the order in which its rows
     accumulate -- does not depend on which other heads are compacted with it."""
-    return begin_plan(mask, validate, pairing)()
+    return begin_plan(mask, validate, pairing, ahead=False)()
 
 
-def begin_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: str = "adjacent"):
+def begin_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: str = "adjacent", ahead: bool = True):
     """compact_plan in two parts: launches everything up to the lists' lengths and returns a function that waits for these,
     makes the lists and returns the plan.  A caller with other work for the stream issues it in between, so that the GPU does
-    not stand still while the host reads three numbers and allocates (on the calling thread's current stream, both times)."""
+    not stand still while the host reads three numbers and allocates (on the calling thread's current stream, both times).
+    ahead: bring the lengths to the host as soon as they are known, through pinned memory; otherwise they are read when the
+    function is called, behind whatever was issued in between."""
     if pairing not in ("adjacent", "overlap"):
         raise ValueError(f"unknown pairing {pairing!r}")
     _lib.require_cuda(mask)
@@ -168,15 +170,17 @@ def begin_plan(mask: torch.Tensor, validate: Optional[bool] = None, pairing: str
         _lib.check(L.paro_plan_offsets(m.data_ptr(), slices, nbq, nbk, overlap, row_ptr.data_ptr(), pair_ptr.data_ptr(),
                                        _lib.ptr(pair_q), totals.data_ptr(), scratch.data_ptr(), scratch.numel(), s))
         # the lists' lengths, read by the host in `finish`: the one synchronisation of the call
-        lengths = torch.empty(4, dtype=torch.int32, pin_memory=True)
-        lengths.copy_(totals, non_blocking=True)
-        arrived = torch.cuda.Event()
-        arrived.record()
+        if ahead:
+            lengths = torch.empty(4, dtype=torch.int32, pin_memory=True)
+            lengths.copy_(totals, non_blocking=True)
+            arrived = torch.cuda.Event()
+            arrived.record()
         sched_cnt = torch.empty(slices * npairs, 2, dtype=torch.int32, device=dev)
 
     def finish() -> CompactPlan:
-        arrived.synchronize()
-        kept, tiles, paired, expired = lengths.tolist()
+        if ahead:
+            arrived.synchronize()
+        kept, tiles, paired, expired = (lengths if ahead else totals).tolist()
         if expired:
             raise _lib.ParoError(_lib.PARO_ETIMEOUT, "a wait of the q-block pairing expired")
         with torch.cuda.device(dev):
